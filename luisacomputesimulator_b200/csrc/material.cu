@@ -15,112 +15,167 @@ using namespace lcs;
 
 namespace {
 
-__device__ __forceinline__ void st3(float4* p, v3 a) { *p = make_float4(a.x, a.y, a.z, 0.0f); }
-// 3x3 block (column-major [3 c + r]) to a float3x3 record (three 16-byte columns); transposed if t
-__device__ __forceinline__ void st33(float4* p, const float* K, bool t)
+// The evaluators write 224 to 832 bytes per element, so they are bound by those stores.  One thread storing its own
+// element spreads every store instruction of a warp over 32 half-written sectors (bending of an 88,800-vertex cloth,
+// 221 MB: 212 us, 1.0 TB/s; the three evaluators and the energy: 368 us, now 88 us).  Here a warp's 32 elements are evaluated one per lane into shared memory (an odd
+// number of words per element: no bank conflicts) and the warp then writes their output as one run of consecutive
+// 16-byte words, each lane forming the word it stores.
+constexpr int kEvalThreads = 128, kEvalWarps = kEvalThreads / 32;
+
+__global__ void __launch_bounds__(kEvalThreads) k_eval_springs(uint32_t n, const float4* __restrict__ x,
+                                                               const uint2* __restrict__ edges,
+                                                               const float* __restrict__ rest_len,
+                                                               const float* __restrict__ stiff, float4* grad, float4* hess)
 {
+    __shared__ float sh[kEvalWarps][32][13];  // gradient, Hessian block (column-major)
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float(*sw)[13] = sh[warp];
+    for (uint32_t e0 = 32u * (blockIdx.x * kEvalWarps + warp); e0 < n; e0 += 32u * kEvalWarps * gridDim.x) {
+        const uint32_t e = e0 + lane, m = min(32u, n - e0);
+        if (e < n) {
+            const uint2 ed = edges[e];
+            const v3 p0 = ld3(x, ed.x), p1 = ld3(x, ed.y);
+            const v3 d = p0 - p1;
+            const float l = fmx(sqrtf(dot3(d, d)), 1.19209290E-7f);
+            const float k = stiff[e], L = rest_len[e];
+            const float C = l - L, il = 1.0f / l, il2 = il * il;
+            sw[lane][0] = k * d.x * il * C;
+            sw[lane][1] = k * d.y * il * C;
+            sw[lane][2] = k * d.z * il * C;
+            const float a = k * il2, c = k * fmx(1.0f - L * il, 0.0f);
+            const float dd[3] = {d.x, d.y, d.z};
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-        p[c] = t ? make_float4(K[c], K[3 + c], K[6 + c], 0.0f) : make_float4(K[3 * c], K[3 * c + 1], K[3 * c + 2], 0.0f);
+            for (int cc = 0; cc < 3; ++cc)
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    sw[lane][3 + 3 * cc + r] = a * dd[r] * dd[cc] + c * ((r == cc ? 1.0f : 0.0f) - il2 * dd[r] * dd[cc]);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < 2u * m; i += 32u) {  // g, -g
+            const float* g = sw[i >> 1];
+            const float sgn = (i & 1u) ? -1.0f : 1.0f;
+            __stcs(&grad[2 * (size_t)e0 + i], make_float4(sgn * g[0], sgn * g[1], sgn * g[2], 0.0f));
+        }
+        for (uint32_t i = lane; i < 12u * m; i += 32u) {  // blocks (0,0) (1,1) (0,1) (1,0): H, H, -H, -H
+            const uint32_t el = i / 12u, k = i - 12u * el, c = k % 3u;
+            const float* H = sw[el] + 3 + 3 * c;
+            const float sgn = k >= 6u ? -1.0f : 1.0f;
+            __stcs(&hess[12 * (size_t)e0 + i], make_float4(sgn * H[0], sgn * H[1], sgn * H[2], 0.0f));
+        }
+        __syncwarp();
+    }
 }
 
-__global__ void k_eval_springs(uint32_t n, const float4* __restrict__ x, const uint2* __restrict__ edges,
-                               const float* __restrict__ rest_len, const float* __restrict__ stiff, float4* grad,
-                               float4* hess)
+__global__ void __launch_bounds__(kEvalThreads) k_eval_stretch_faces(uint32_t n, const float4* __restrict__ x,
+                                                                     const uint4* __restrict__ faces,
+                                                                     const float4* __restrict__ dm,
+                                                                     const float* __restrict__ area,
+                                                                     const float2* __restrict__ mu_lambda, float4* grad,
+                                                                     float4* hess)
 {
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const uint2 ed = edges[e];
-        const v3 p0 = ld3(x, ed.x), p1 = ld3(x, ed.y);
-        const v3 d = p0 - p1;
-        const float l = fmx(sqrtf(dot3(d, d)), 1.19209290E-7f);
-        const float k = stiff[e], L = rest_len[e];
-        const float C = l - L, il = 1.0f / l, il2 = il * il;
-        const v3 g = mk3(k * d.x * il * C, k * d.y * il * C, k * d.z * il * C);
-        st3(&grad[2 * (size_t)e], g);
-        st3(&grad[2 * (size_t)e + 1], neg3(g));
-        const float a = k * il2, c = k * fmx(1.0f - L * il, 0.0f);
-        const float dd[3] = {d.x, d.y, d.z};
-        float H[9], N[9];
+    __shared__ float sh[kEvalWarps][32][63];  // 3 gradients, 6 blocks (column-major)
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float(*sw)[63] = sh[warp];
+    for (uint32_t f0 = 32u * (blockIdx.x * kEvalWarps + warp); f0 < n; f0 += 32u * kEvalWarps * gridDim.x) {
+        const uint32_t f = f0 + lane, m = min(32u, n - f0);
+        if (f < n) {
+            const uint4 fc = faces[f];
+            const float2 ml = mu_lambda[f];
+            Bw98Out o;
+            bw98_face(ld3(x, fc.x), ld3(x, fc.y), ld3(x, fc.z), dm[f], ml.x, ml.y, area[f], o);
 #pragma unroll
-        for (int cc = 0; cc < 3; ++cc)
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                H[3 * cc + r] = a * dd[r] * dd[cc] + c * ((r == cc ? 1.0f : 0.0f) - il2 * dd[r] * dd[cc]);
-                N[3 * cc + r] = -H[3 * cc + r];
+            for (int a = 0; a < 3; ++a) {
+                sw[lane][3 * a] = o.g[a].x;
+                sw[lane][3 * a + 1] = o.g[a].y;
+                sw[lane][3 * a + 2] = o.g[a].z;
             }
-        float4* o = hess + 12 * (size_t)e;  // 4 blocks: (0,0) (1,1) (0,1) (1,0)
-        st33(o, H, false);
-        st33(o + 3, H, false);
-        st33(o + 6, N, false);
-        st33(o + 9, N, false);
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+#pragma unroll
+                for (int j = 0; j < 9; ++j) sw[lane][9 + 9 * k + j] = o.K[k][j];
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < 3u * m; i += 32u) {
+            const uint32_t el = i / 3u;
+            const float* g = sw[el] + 3u * (i - 3u * el);
+            __stcs(&grad[3 * (size_t)f0 + i], make_float4(g[0], g[1], g[2], 0.0f));
+        }
+        // blocks (0,0) (1,1) (2,2), then (0,1) (0,2) (1,0) (1,2) (2,0) (2,1) (row vertex, column vertex): the stored
+        // blocks 0 1 2 3 4 3' 5 4' 5' (' transposed)
+        for (uint32_t i = lane; i < 27u * m; i += 32u) {
+            const uint32_t el = i / 27u, k = i - 27u * el, blk = k / 3u, c = k - 3u * blk;
+            const uint32_t src = (0x545343210ull >> (4u * blk)) & 15u;
+            const bool tr = (0x1A0u >> blk) & 1u;
+            const float* K = sw[el] + 9 + 9 * src + (tr ? c : 3u * c);
+            const uint32_t st = tr ? 3u : 1u;
+            __stcs(&hess[27 * (size_t)f0 + i], make_float4(K[0], K[st], K[2 * st], 0.0f));
+        }
+        __syncwarp();
     }
 }
 
-__global__ void k_eval_stretch_faces(uint32_t n, const float4* __restrict__ x, const uint4* __restrict__ faces,
-                                     const float4* __restrict__ dm, const float* __restrict__ area,
-                                     const float2* __restrict__ mu_lambda, float4* grad, float4* hess)
+__global__ void __launch_bounds__(kEvalThreads) k_eval_bending(uint32_t n, const float4* __restrict__ x,
+                                                               const uint4* __restrict__ st,
+                                                               const float* __restrict__ rest_angle,
+                                                               const float* __restrict__ hbar,
+                                                               const float* __restrict__ stiffness, float scaling,
+                                                               float4* grad, float4* hess)
 {
-    for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
-        const uint4 fc = faces[f];
-        const float2 ml = mu_lambda[f];
-        Bw98Out o;
-        bw98_face(ld3(x, fc.x), ld3(x, fc.y), ld3(x, fc.z), dm[f], ml.x, ml.y, area[f], o);
+    __shared__ float sh[kEvalWarps][32][15];  // dtheta/dx of the four vertices, stiffness, stiffness (theta - rest)
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float(*sw)[15] = sh[warp];
+    // 48 Hessian words per element: a run of 96 words (two elements) is three words per lane, so the lane's three
+    // places (element of the two, vertices i and j, column) are the same in every run
+    uint32_t pe[3], pi[3], pj[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) st3(&grad[3 * (size_t)f + a], o.g[a]);
-        // blocks: (0,0) (1,1) (2,2), then (0,1) (0,2) (1,0) (1,2) (2,0) (2,1) (row vertex, column vertex)
-        float4* h = hess + 27 * (size_t)f;
-        st33(h + 0, o.K[0], false);
-        st33(h + 3, o.K[1], false);
-        st33(h + 6, o.K[2], false);
-        st33(h + 9, o.K[3], false);
-        st33(h + 12, o.K[4], false);
-        st33(h + 15, o.K[3], true);
-        st33(h + 18, o.K[5], false);
-        st33(h + 21, o.K[4], true);
-        st33(h + 24, o.K[5], true);
+    for (uint32_t q = 0; q < 3; ++q) {
+        const uint32_t w = 32u * q + lane, k = w % 48u, blk = k / 3u, c = k - 3u * blk;
+        pe[q] = w / 48u;
+        // blocks (i, i), then (i, j), i != j, row-major
+        const uint32_t o = blk - 4u, i = blk < 4u ? blk : o / 3u, jj = blk < 4u ? blk : o - 3u * i;
+        const uint32_t j = blk < 4u ? blk : jj + (jj >= i ? 1u : 0u);
+        pi[q] = 3u * i;
+        pj[q] = 3u * j + c;
     }
-}
-
-__global__ void k_eval_bending(uint32_t n, const float4* __restrict__ x, const uint4* __restrict__ st,
-                               const float* __restrict__ rest_angle, const float* __restrict__ hbar,
-                               const float* __restrict__ stiffness, float scaling, float4* grad, float4* hess)
-{
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const uint4 e = st[s];
-        v3 g[4];
-        const float theta = dihedral_angle_grad(ld3(x, e.x), ld3(x, e.y), ld3(x, e.z), ld3(x, e.w), g);
-        const float stiff = stiffness[s] * scaling * hbar[s];
-        const float sd = stiff * (theta - rest_angle[s]);
+    for (uint32_t s0 = 32u * (blockIdx.x * kEvalWarps + warp); s0 < n; s0 += 32u * kEvalWarps * gridDim.x) {
+        const uint32_t s = s0 + lane, m = min(32u, n - s0);
+        if (s < n) {
+            const uint4 e = st[s];
+            v3 g[4];
+            const float theta = dihedral_angle_grad(ld3(x, e.x), ld3(x, e.y), ld3(x, e.z), ld3(x, e.w), g);
+            const float stiff = stiffness[s] * scaling * hbar[s];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) st3(&grad[4 * (size_t)s + i], sd * g[i]);
-        // blocks stiff g_i g_j^T: (i, i) for i = 0..3, then (i, j), i != j, row-major
-        float4* h = hess + 48 * (size_t)s;
-        int k = 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float gi[3] = {g[i].x, g[i].y, g[i].z}, gj[3] = {g[j].x, g[j].y, g[j].z};
-                float K[9];
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int r = 0; r < 3; ++r) K[3 * c + r] = stiff * (gi[r] * gj[c]);
-                st33(h + 3 * (i == j ? i : k), K, false);
-                if (i != j) ++k;
+            for (int i = 0; i < 4; ++i) {
+                sw[lane][3 * i] = g[i].x;
+                sw[lane][3 * i + 1] = g[i].y;
+                sw[lane][3 * i + 2] = g[i].z;
             }
-    }
-}
-
-__device__ __forceinline__ void warp_add_f64(double* dst, double v)
-{
+            sw[lane][12] = stiff;
+            sw[lane][13] = stiff * (theta - rest_angle[s]);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < 4u * m; i += 32u) {
+            const float *o = sw[i >> 2], *g = o + 3u * (i & 3u);
+            __stcs(&grad[4 * (size_t)s0 + i], make_float4(o[13] * g[0], o[13] * g[1], o[13] * g[2], 0.0f));
+        }
+        float4* h = hess + 48 * (size_t)s0 + lane;
+        for (uint32_t e = 0; e < m; e += 2u, h += 96) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    if (lane_id() == 0 && v != 0.0) atomicAdd(dst, v);
+            for (int q = 0; q < 3; ++q) {
+                if (e + pe[q] >= m) continue;  // the last element of an odd count
+                const float *o = sw[e + pe[q]], *gi = o + pi[q];
+                const float k = o[12], gj = o[pj[q]];
+                __stcs(h + 32 * q, make_float4(k * (gi[0] * gj), k * (gi[1] * gj), k * (gi[2] * gj), 0.0f));
+            }
+        }
+        __syncwarp();
+    }
 }
 
 // energy terms: [0] inertia (fn_calc_energy_inertia), [1] springs, [2] stretch faces, [3] bending
-__global__ void k_material_energy(lcs_cloth_elements m, const float4* __restrict__ x, const float4* __restrict__ xt,
+// One atomic per block and term: with one per warp, the 33,000 additions to each of four addresses took most of the
+// time (46 us on 88,800 vertices).
+__global__ void __launch_bounds__(256) k_material_energy(lcs_cloth_elements m, const float4* __restrict__ x, const float4* __restrict__ xt,
                                   float dt, float dirichlet, double* out)
 {
     const uint32_t n = max(max(m.n_verts, m.n_springs), max(m.n_stretch_faces, m.n_bending));
@@ -162,8 +217,20 @@ __global__ void k_material_energy(lcs_cloth_elements m, const float4* __restrict
             e[3] += (double)(0.5f * m.bending_stiffness[i] * m.bending_scaling * m.bending_hbar[i] * d * d);
         }
     }
+    __shared__ double red[4][8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) warp_add_f64(out + k, e[k]);
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e[k] += __shfl_xor_sync(0xFFFFFFFFu, e[k], o);
+        if (lane_id() == 0) red[k][threadIdx.x >> 5] = e[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
+        if (v != 0.0) atomicAdd(out + threadIdx.x, v);
+    }
 }
 
 int launch_check(const char* what)
@@ -180,7 +247,7 @@ extern "C" int lcs_eval_springs(const float* x, const uint32_t* edges, const flo
     if (n == 0) return LCS_OK;
     if (!x || !edges || !rest_len || !stiffness || !gradients || !hessians)
         return lcs_fail(LCS_ERR_INVALID, "lcs_eval_springs: null argument");
-    k_eval_springs<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(
+    k_eval_springs<<<grid_for(n, kEvalThreads, 16), kEvalThreads, 0, (cudaStream_t)stream>>>(
         n, reinterpret_cast<const float4*>(x), reinterpret_cast<const uint2*>(edges), rest_len, stiffness,
         reinterpret_cast<float4*>(gradients), reinterpret_cast<float4*>(hessians));
     return launch_check("lcs_eval_springs: launch failed");
@@ -193,7 +260,7 @@ extern "C" int lcs_eval_stretch_faces(const float* x, const uint32_t* faces, con
     if (n == 0) return LCS_OK;
     if (!x || !faces || !dm_inv || !rest_area || !mu_lambda || !gradients || !hessians)
         return lcs_fail(LCS_ERR_INVALID, "lcs_eval_stretch_faces: null argument");
-    k_eval_stretch_faces<<<grid_for(n, 128), 128, 0, (cudaStream_t)stream>>>(
+    k_eval_stretch_faces<<<grid_for(n, kEvalThreads, 7), kEvalThreads, 0, (cudaStream_t)stream>>>(
         n, reinterpret_cast<const float4*>(x), reinterpret_cast<const uint4*>(faces),
         reinterpret_cast<const float4*>(dm_inv), rest_area, reinterpret_cast<const float2*>(mu_lambda),
         reinterpret_cast<float4*>(gradients), reinterpret_cast<float4*>(hessians));
@@ -207,7 +274,7 @@ extern "C" int lcs_eval_bending(const float* x, const uint32_t* stencils, const 
     if (n == 0) return LCS_OK;
     if (!x || !stencils || !rest_angle || !rest_hbar || !stiffness || !gradients || !hessians)
         return lcs_fail(LCS_ERR_INVALID, "lcs_eval_bending: null argument");
-    k_eval_bending<<<grid_for(n, 128), 128, 0, (cudaStream_t)stream>>>(
+    k_eval_bending<<<grid_for(n, kEvalThreads, 16), kEvalThreads, 0, (cudaStream_t)stream>>>(
         n, reinterpret_cast<const float4*>(x), reinterpret_cast<const uint4*>(stencils), rest_angle, rest_hbar,
         stiffness, scaling, reinterpret_cast<float4*>(gradients), reinterpret_cast<float4*>(hessians));
     return launch_check("lcs_eval_bending: launch failed");
@@ -225,7 +292,7 @@ extern "C" int lcs_material_energy(const lcs_cloth_elements* m, const float* x, 
     LCS_CUDA_TRY(cudaMemsetAsync(energy, 0, 4 * sizeof(double), s));
     const uint32_t n = std::max(std::max(m->n_verts, m->n_springs), std::max(m->n_stretch_faces, m->n_bending));
     if (n == 0) return LCS_OK;
-    k_material_energy<<<grid_for(n, 256), 256, 0, s>>>(*m, reinterpret_cast<const float4*>(x),
+    k_material_energy<<<grid_for(n, 256, 4), 256, 0, s>>>(*m, reinterpret_cast<const float4*>(x),
                                                       reinterpret_cast<const float4*>(x_tilde), dt,
                                                       stiffness_dirichlet, energy);
     return launch_check("lcs_material_energy: launch failed");
