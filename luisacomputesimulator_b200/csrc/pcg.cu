@@ -24,6 +24,7 @@
 
 #include "lcs_common.cuh"
 #include "lcs_internal.h"
+#include "row_stage.cuh"
 
 using namespace lcs;
 
@@ -1728,18 +1729,21 @@ __global__ void __launch_bounds__(BT, 1) k_pcg_res(ResArgs ra)
 // Many independent systems (one per scene, rows [roff[s], roff[s+1])) solved in one launch: one
 // thread-block cluster per scene, synchronised by the hardware cluster barrier, with the scene's
 // own alpha, beta and stop decision (the recurrences and stop rules of k_pcg_fused).  The rows of a
-// scene are cut into chunks of 256; chunk k belongs to CTA k mod C of the cluster, thread t to row
-// 256k + t (the SpMV uses 4 lanes per row).  Every dot product is summed per chunk in a fixed tree
-// and then over the chunks in a fixed order, so a scene's result does not depend on the cluster
-// size C nor on the other scenes of the launch.  Vectors live in global memory (L2-resident per
-// scene); cross-CTA reads use ld.cg.
-constexpr int kBatchThreads = 256;
-constexpr int kBatchLanes = 4;
+// scene are cut into chunks of 256; chunk k belongs to CTA k mod C of the cluster, and a warp owns
+// 32-row slices of the CTA's chunks through all phases, so that only p crosses the CTA.  Every dot
+// product is summed per slice and per chunk in a fixed tree and then over the chunks in a fixed
+// order, so a scene's result does not depend on the cluster size C, on the CTA size nor on the other
+// scenes of the launch.  Vectors live in global memory (L2-resident per scene); the cluster barrier's
+// acquire makes the other CTAs' p visible to ordinary (L1-cached) loads.
+constexpr int kChunk = 256;
+constexpr uint32_t kChunkSlices = kChunk / 32;
+constexpr uint32_t kRoundSlices = 512;  // slices whose sums a CTA holds before it reduces them to chunk sums
 
 struct BatchArgs {
-    const uint32_t* scenes;  // cluster index -> scene id (null: the identity)
+    const uint32_t* scenes;  // cluster index -> scene id (null: by falling size, see k_pcg_batch)
     const uint32_t* roff;    // S + 1
     const uint32_t* active;  // S (0: skip the scene, x = 0) or null
+    uint32_t n_rows;         // rows of the matrices
     const float4* diag;
     Bsr A, B;
     const float4* b;
@@ -1755,6 +1759,7 @@ struct BatchArgs {
 
 __device__ __forceinline__ void cluster_sync_all()
 {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -1772,100 +1777,150 @@ __device__ __forceinline__ uint32_t cluster_ctas()
     return n;
 }
 
-// fixed-tree sum of one value per thread (256 threads) -> thread 0
-__device__ __forceinline__ double chunk_sum(double v, double* s_w)
+__device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    if (lane_id() == 0) s_w[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int w = 0; w < kBatchThreads / 32; ++w) t += s_w[w];
-    __syncthreads();
-    return t;
+    return v;
 }
 
-// sum over a scene's chunks in a fixed order, the same in every CTA of the cluster
-__device__ __forceinline__ void scene_sum(const double* cp, uint32_t nchunks, int k, int count, double* out,
-                                          double* s_out)
+// sum of `count` values over a scene's chunks in a fixed order, the same in every warp of the cluster
+__device__ __forceinline__ void scene_sum(const double* cp, uint32_t nchunks, int k, int count, double* out)
 {
-    if (threadIdx.x < 32) {
-        double v[2] = {0.0, 0.0};
-        for (uint32_t c = threadIdx.x; c < nchunks; c += 32)
-            for (int j = 0; j < count; ++j) v[j] += __ldcg(&cp[4 * c + k + j]);
-        for (int j = 0; j < count; ++j) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xFFFFFFFFu, v[j], o);
-        }
-        if (threadIdx.x == 0)
-            for (int j = 0; j < count; ++j) s_out[j] = v[j];
-    }
-    __syncthreads();
-    for (int j = 0; j < count; ++j) out[j] = s_out[j];
-    __syncthreads();
+    double v[2] = {0.0, 0.0};
+    for (uint32_t c = lane_id(); c < nchunks; c += 32)
+        for (int j = 0; j < count; ++j) v[j] += __ldcg(&cp[4 * (size_t)c + k + j]);
+    for (int j = 0; j < count; ++j) out[j] = warp_sum(v[j]);
 }
 
-__global__ void __launch_bounds__(kBatchThreads) k_pcg_batch(BatchArgs a)
+// W warps per CTA.  The matrix streams through shared memory (row_stage.cuh).  48 scenes of 2,000 to 16,000 rows,
+// cluster 4 (340,000 rows, 13 blocks each, 50 to 100 iterations): 18.9 ms with the blocks read straight from global
+// memory by 256 threads per CTA, 5.25 ms so; what bounds it now is the L2 traffic of the SMs that hold the largest
+// scenes (4,000 rows a CTA, 0.8 KB a row and iteration).
+template <int W, bool Staged>
+__global__ void __launch_bounds__(32 * W, !Staged ? 4 : W > 8 ? 1 : 2) k_pcg_batch(BatchArgs a)
 {
-    __shared__ double s_w[kBatchThreads / 32];
-    __shared__ double s_out[2];
-    __shared__ double s_pq[kBatchThreads];
+    extern __shared__ __align__(128) unsigned char s_stage[];
+    __shared__ double s_part[2][kRoundSlices];
+    __shared__ __align__(8) uint64_t s_bar[2 * W];
+    __shared__ uint32_t s_scene;
     const uint32_t C = cluster_ctas(), rank = cluster_rank();
-    const uint32_t s = a.scenes ? a.scenes[blockIdx.x / C] : blockIdx.x / C;
-    const uint32_t r0 = a.roff[s], r1 = a.roff[s + 1], nrows = r1 - r0;
-    const uint32_t nchunks = (nrows + kBatchThreads - 1) / kBatchThreads;
-    double* cp = a.cpart + 4 * (size_t)((r0 >> 8) + s);
-    const uint32_t t = threadIdx.x;
-    const bool on = !a.active || a.active[s] != 0u;  // uniform over the cluster
-    for (uint32_t k = rank; k < nchunks; k += C) {
-        const uint32_t i = r0 + k * kBatchThreads + t;
-        if (i >= r1) continue;
-        a.x[i] = make_float4(0, 0, 0, 0);
-        if (!on) continue;
-        a.r[i] = a.b[i];
-        a.p[i] = make_float4(0, 0, 0, 0);
-        const float4 c0 = a.diag[3 * i], c1 = a.diag[3 * i + 1], c2 = a.diag[3 * i + 2];
-        const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, kk = c2.z;
-        const float A = e * kk - f * h, B = f * g - d * kk, Cc = d * h - e * g;
-        const float id = 1.0f / (aa * A + bb * B + c * Cc);
-        a.minv[3 * i + 0] = make_float4(A * id, B * id, Cc * id, 0.0f);
-        a.minv[3 * i + 1] = make_float4((c * h - bb * kk) * id, (aa * kk - c * g) * id, (bb * g - aa * h) * id, 0.0f);
-        a.minv[3 * i + 2] = make_float4((bb * f - c * e) * id, (c * d - aa * f) * id, (aa * e - bb * d) * id, 0.0f);
+    const uint32_t t = threadIdx.x, w = t >> 5, lane = lane_id();
+    uint32_t s = blockIdx.x / C;
+    if (a.scenes) {
+        s = a.scenes[s];
+    } else if (gridDim.x / C <= kChunk) {
+        // the largest scenes first: the cluster's place in the order of falling size (ties by index)
+        const uint32_t S = gridDim.x / C;
+        for (uint32_t c = t; c < S; c += 32 * W) {
+            const uint32_t len = a.roff[c + 1] - a.roff[c];
+            uint32_t place = 0;
+            for (uint32_t o = 0; o < S; ++o) {
+                const uint32_t lo = a.roff[o + 1] - a.roff[o];
+                place += lo > len || (lo == len && o < c) ? 1u : 0u;
+            }
+            if (place == s) s_scene = c;
+        }
+        __syncthreads();
+        s = s_scene;
     }
+    const uint32_t r0 = a.roff[s], r1 = a.roff[s + 1], nrows = r1 - r0;
+    const uint32_t nchunks = (nrows + kChunk - 1) / kChunk;
+    const uint32_t nlocal = rank < nchunks ? (nchunks - rank + C - 1) / C : 0u;  // this CTA's chunks
+    const uint32_t nslices = nlocal * kChunkSlices;
+    double* cp = a.cpart + 4 * (size_t)((r0 >> 8) + s);
+    const bool on = !a.active || a.active[s] != 0u;  // uniform over the cluster
+    auto base_of = [&](uint32_t ls) {
+        return r0 + (rank + C * (ls / kChunkSlices)) * kChunk + 32 * (ls % kChunkSlices);
+    };
+    // the CTA's slice sums in s_part -> chunk sums in cp, for the slices [ls0, ls0 + kRoundSlices)
+    auto chunk_sums = [&](uint32_t ls0, int k, int count) {
+        __syncthreads();
+        const uint32_t nc = (min(nslices, ls0 + kRoundSlices) - ls0) / kChunkSlices;
+        for (uint32_t e = t; e < nc * count; e += 32 * W) {
+            const uint32_t c = e % nc, j = e / nc;
+            double v = 0.0;
+#pragma unroll
+            for (uint32_t q = 0; q < kChunkSlices; ++q) v += s_part[j][c * kChunkSlices + q];
+            cp[4 * (size_t)(rank + C * (ls0 / kChunkSlices + c)) + k + j] = v;
+        }
+        if (ls0 + kRoundSlices < nslices) __syncthreads();
+    };
     if (!on) {
+        for (uint32_t ls = w; ls < nslices; ls += W) {
+            const uint32_t i = base_of(ls) + lane;
+            if (i < r1) a.x[i] = make_float4(0, 0, 0, 0);
+        }
         if (rank == 0 && t == 0) a.stats[s] = lcs_pcg_stats{0, 0.0f, 0.0f, LCS_OK};
         return;
     }
-    float rz_old = 0.0f, norm_r0 = 0.0f, norm_r = 0.0f, rz = 0.0f;
+    stage::Warp st;
+    st.init(s_stage + w * stage::kWarpBytes, Staged ? s_bar + 2 * w : nullptr, stage::Csr{a.A.rp, a.A.col, a.A.val},
+            stage::Csr{a.B.rp, a.B.col, a.B.val}, a.n_rows);
+    const float4* p_all = a.p;
+    auto ld_p = [&](uint32_t col) -> float4 { return p_all[col]; };
+
+    float rz_old = 0.0f, norm_r0 = 0.0f, norm_r = 0.0f, rz = 0.0f, alpha = 0.0f;
     int iter = 0, status = 0;
-    for (iter = 0; iter < a.max_iter; ++iter) {
-        // z = Minv r ; r.r ; r.z per chunk
-        for (uint32_t k = rank; k < nchunks; k += C) {
-            const uint32_t i = r0 + k * kBatchThreads + t;
-            double drr = 0.0, drz = 0.0;
-            if (i < r1) {
-                const float4 rv = a.r[i];
-                const float3 zv = mv12(a.minv + 3 * (size_t)i, rv);
-                a.z[i] = make_float4(zv.x, zv.y, zv.z, 0.0f);
-                if (a.fp64) {
-                    drr = (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z;
-                    drz = (double)rv.x * zv.x + (double)rv.y * zv.y + (double)rv.z * zv.z;
-                } else {
-                    drr = __fmaf_rn(rv.z, rv.z, __fmaf_rn(rv.y, rv.y, rv.x * rv.x));
-                    drz = __fmaf_rn(rv.z, zv.z, __fmaf_rn(rv.y, zv.y, rv.x * zv.x));
+    for (;; ++iter) {
+        // x += alpha p, r -= alpha q of the step before; z = Minv r; r.r and r.z per chunk
+        const bool last = iter >= a.max_iter;
+        for (uint32_t ls0 = 0; ls0 < nslices; ls0 += kRoundSlices) {
+            for (uint32_t ls = ls0 + w; ls < min(nslices, ls0 + kRoundSlices); ls += W) {
+                const uint32_t i = base_of(ls) + lane;
+                double drr = 0.0, drz = 0.0;
+                if (i < r1) {
+                    float4 rv, m0, m1, m2;
+                    if (iter == 0) {
+                        rv = a.b[i];
+                        a.x[i] = make_float4(0, 0, 0, 0);
+                        a.p[i] = make_float4(0, 0, 0, 0);
+                        const float4 c0 = a.diag[3 * (size_t)i], c1 = a.diag[3 * (size_t)i + 1], c2 = a.diag[3 * (size_t)i + 2];
+                        const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, kk = c2.z;
+                        const float A = e * kk - f * h, Bc = f * g - d * kk, Cc = d * h - e * g;
+                        const float id = 1.0f / (aa * A + bb * Bc + c * Cc);
+                        m0 = make_float4(A * id, Bc * id, Cc * id, 0.0f);
+                        m1 = make_float4((c * h - bb * kk) * id, (aa * kk - c * g) * id, (bb * g - aa * h) * id, 0.0f);
+                        m2 = make_float4((bb * f - c * e) * id, (c * d - aa * f) * id, (aa * e - bb * d) * id, 0.0f);
+                        a.minv[3 * (size_t)i] = m0;
+                        a.minv[3 * (size_t)i + 1] = m1;
+                        a.minv[3 * (size_t)i + 2] = m2;
+                        a.r[i] = rv;
+                    } else {
+                        const float4 pv = a.p[i], qv = a.q[i], xv = a.x[i], ro = a.r[i];
+                        m0 = a.minv[3 * (size_t)i];
+                        m1 = a.minv[3 * (size_t)i + 1];
+                        m2 = a.minv[3 * (size_t)i + 2];
+                        a.x[i] = make_float4(xv.x + alpha * pv.x, xv.y + alpha * pv.y, xv.z + alpha * pv.z, 0.0f);
+                        rv = make_float4(ro.x - alpha * qv.x, ro.y - alpha * qv.y, ro.z - alpha * qv.z, 0.0f);
+                        a.r[i] = rv;
+                    }
+                    float3 zv;
+                    zv.x = __fmaf_rn(m2.x, rv.z, __fmaf_rn(m1.x, rv.y, m0.x * rv.x));
+                    zv.y = __fmaf_rn(m2.y, rv.z, __fmaf_rn(m1.y, rv.y, m0.y * rv.x));
+                    zv.z = __fmaf_rn(m2.z, rv.z, __fmaf_rn(m1.z, rv.y, m0.z * rv.x));
+                    a.z[i] = make_float4(zv.x, zv.y, zv.z, 0.0f);
+                    if (a.fp64) {
+                        drr = (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z;
+                        drz = (double)rv.x * zv.x + (double)rv.y * zv.y + (double)rv.z * zv.z;
+                    } else {
+                        drr = __fmaf_rn(rv.z, rv.z, __fmaf_rn(rv.y, rv.y, rv.x * rv.x));
+                        drz = __fmaf_rn(rv.z, zv.z, __fmaf_rn(rv.y, zv.y, rv.x * zv.x));
+                    }
+                }
+                drr = warp_sum(drr);
+                drz = warp_sum(drz);
+                if (lane == 0) {
+                    s_part[0][ls - ls0] = drr;
+                    s_part[1][ls - ls0] = drz;
                 }
             }
-            const double srr = chunk_sum(drr, s_w), srz = chunk_sum(drz, s_w);
-            if (t == 0) {
-                cp[4 * k + 0] = srr;
-                cp[4 * k + 1] = srz;
-            }
+            chunk_sums(ls0, 0, 2);
         }
+        if (last) break;  // uniform over the grid
         cluster_sync_all();
         double red[2];
-        scene_sum(cp, nchunks, 0, 2, red, s_out);
+        scene_sum(cp, nchunks, 0, 2, red);
         const float rr = (float)red[0];
         rz = (float)red[1];
         const float beta = safe_div(rz, rz_old);
@@ -1877,57 +1932,53 @@ __global__ void __launch_bounds__(kBatchThreads) k_pcg_batch(BatchArgs a)
             if (rz < a.abs_rz_tol) break;
             if (a.rel_tol > 0.0f && norm_r <= a.rel_tol * norm_r0) break;
         }
-        for (uint32_t k = rank; k < nchunks; k += C) {
-            const uint32_t i = r0 + k * kBatchThreads + t;
+        stage::Slice cur, next;
+        cur.load(st, w < nslices ? base_of(w) : r1, r1);
+        for (uint32_t ls = w; ls < nslices; ls += W) {
+            const uint32_t i = base_of(ls) + lane;
             if (i < r1) {
                 const float4 zv = a.z[i], pv = a.p[i];
                 a.p[i] = make_float4(zv.x + beta * pv.x, zv.y + beta * pv.y, zv.z + beta * pv.z, 0.0f);
             }
         }
+        if (Staged) cur.prefetch(st, cur.first());  // the matrix does not wait for p
         cluster_sync_all();
-        // q = A p (4 lanes per row) ; p.q per chunk
-        for (uint32_t k = rank; k < nchunks; k += C) {
-            const uint32_t base = r0 + k * kBatchThreads;
-            const uint32_t lig = t % kBatchLanes;
-            for (uint32_t rr_ = t / kBatchLanes; rr_ < (uint32_t)kBatchThreads; rr_ += kBatchThreads / kBatchLanes) {
-                const uint32_t row = base + rr_ < r1 ? base + rr_ : r1 - 1;  // whole groups stay converged
-                const float3 qv = row_product<kBatchLanes>(row, lig, a.diag, a.A, a.B, a.p);
-                if (lig == 0) {
-                    double d = 0.0;
-                    if (base + rr_ < r1) {
-                        a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
-                        const float4 pv = __ldcg(&a.p[row]);
-                        d = a.fp64 ? (double)pv.x * qv.x + (double)pv.y * qv.y + (double)pv.z * qv.z
-                                   : (double)__fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
-                    }
-                    s_pq[rr_] = d;
+        // q = A p ; p.q per chunk
+        for (uint32_t ls0 = 0; ls0 < nslices; ls0 += kRoundSlices) {
+            for (uint32_t ls = ls0 + w; ls < min(nslices, ls0 + kRoundSlices); ls += W) {
+                const uint32_t i = base_of(ls) + lane;
+                next.load(st, ls + W < nslices ? base_of(ls + W) : r1, r1);
+                const float3 off = stage::slice_product<Staged>(st, cur, next, ld_p);
+                cur = next;
+                double d = 0.0;
+                if (i < r1) {
+                    const float4 pv = p_all[i];
+                    const float3 dv = mv12(a.diag + 3 * (size_t)i, pv);
+                    const float3 qv = make_float3(dv.x + off.x, dv.y + off.y, dv.z + off.z);
+                    a.q[i] = make_float4(qv.x, qv.y, qv.z, 0.0f);
+                    d = a.fp64 ? (double)pv.x * qv.x + (double)pv.y * qv.y + (double)pv.z * qv.z
+                               : (double)__fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
                 }
+                d = warp_sum(d);
+                if (lane == 0) s_part[0][ls - ls0] = d;
             }
-            __syncthreads();
-            const double spq = chunk_sum(s_pq[t], s_w);
-            if (t == 0) cp[4 * k + 2] = spq;
+            chunk_sums(ls0, 2, 1);
         }
         cluster_sync_all();
         double pq;
-        scene_sum(cp, nchunks, 2, 1, &pq, s_out);
-        const float alpha = safe_div(rz, (float)pq);
-        for (uint32_t k = rank; k < nchunks; k += C) {
-            const uint32_t i = r0 + k * kBatchThreads + t;
-            if (i < r1) {
-                const float4 pv = a.p[i], qv = __ldcg(&a.q[i]), xv = a.x[i], rv = a.r[i];
-                a.x[i] = make_float4(xv.x + alpha * pv.x, xv.y + alpha * pv.y, xv.z + alpha * pv.z, 0.0f);
-                a.r[i] = make_float4(rv.x - alpha * qv.x, rv.y - alpha * qv.y, rv.z - alpha * qv.z, 0.0f);
-            }
-        }
+        scene_sum(cp, nchunks, 2, 1, &pq);
+        alpha = safe_div(rz, (float)pq);
     }
     if (rank == 0 && t == 0) {
-        lcs_pcg_stats st;
-        st.iterations = iter;
-        st.rel_residual = norm_r0 > 0.0f ? norm_r / norm_r0 : 0.0f;
-        st.dot_rz = rz_old;
-        st.status = status;
-        a.stats[s] = st;
+        lcs_pcg_stats out;
+        out.iterations = iter;
+        out.rel_residual = norm_r0 > 0.0f ? norm_r / norm_r0 : 0.0f;
+        out.dot_rz = rz_old;
+        out.status = status;
+        a.stats[s] = out;
     }
+    cluster_sync_all();  // a copy that never came in any CTA outlives rank 0's verdict
+    if (st.failed && lane == 0) a.stats[s].status = LCS_ERR_TIMEOUT;
 }
 
 }  // namespace
@@ -2679,17 +2730,30 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
     a.fp64 = (o.flags & LCS_PCG_FP64_DOTS) ? 1 : 0;
     a.stats = stats_per_scene;
     a.scenes = nullptr;
-    auto launch = [&](int C, uint32_t clusters, const uint32_t* scene_list, cudaStream_t st) -> cudaError_t {
-        if (C == 16) {
-            const cudaError_t e = cudaFuncSetAttribute(k_pcg_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return e;
-        }
+    a.n_rows = P->n;
+    auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list, cudaStream_t st) -> cudaError_t {
+        // By the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a single slice, for which
+        // the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600 rows: 2.7 ms so, 3.7 ms
+        // staged).  Two or more are staged, by 16 warps (one CTA per SM) if the grid fits the GPU once or a CTA has
+        // work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to 4,000: 1.7 and 2.3), else
+        // by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).  Clusters of 16 stay at 8 warps,
+        // so that the SMs of one GPC always hold them.
+        const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
+        const bool staged = cta_chunks >= 2;
+        const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= 148);
+        const void* kernel = wide ? (const void*)k_pcg_batch<16, true>
+                                  : staged ? (const void*)k_pcg_batch<8, true> : (const void*)k_pcg_batch<8, false>;
+        const uint32_t warps = wide ? 16 : 8, smem = staged ? warps * stage::kWarpBytes : 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (e == cudaSuccess && C == 16) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
         BatchArgs b = a;
         b.scenes = scene_list;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(clusters * (uint32_t)C);
-        cfg.blockDim = dim3(kBatchThreads);
-        cfg.dynamicSmemBytes = 0;
+        cfg.blockDim = dim3(32 * warps);
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2698,11 +2762,15 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_pcg_batch, b);
+        void* args[] = {&b};
+        return cudaLaunchKernelExC(&cfg, kernel, args);
     };
     cudaStream_t s0 = (cudaStream_t)stream;
     if (cluster != 0) {
-        LCS_CUDA_TRY(launch(cluster, n_scenes, nullptr, s0));
+        uint32_t max_rows = 0;
+        for (uint32_t sc = 0; sc < n_scenes; ++sc)
+            max_rows = std::max(max_rows, host_row_offsets[sc + 1] - host_row_offsets[sc]);
+        LCS_CUDA_TRY(launch(cluster, n_scenes, max_rows, nullptr, s0));
         lcs_count_launch();
         return LCS_OK;
     }
@@ -2753,7 +2821,9 @@ static int solve_batch_auto(lcs_pcg* P, uint32_t n_scenes, const uint32_t* host_
     }
     std::vector<uint32_t> flat;
     size_t start[6] = {0};
-    for (int k = 0; k < 5; ++k) {
+    auto rows_of = [&](uint32_t sc) { return host_row_offsets[sc + 1] - host_row_offsets[sc]; };
+    for (int k = 0; k < 5; ++k) {  // the largest scenes of a class start first
+        std::stable_sort(lists[k].begin(), lists[k].end(), [&](uint32_t p, uint32_t q) { return rows_of(p) > rows_of(q); });
         start[k] = flat.size();
         flat.insert(flat.end(), lists[k].begin(), lists[k].end());
     }
@@ -2783,7 +2853,7 @@ static int solve_batch_auto(lcs_pcg* P, uint32_t n_scenes, const uint32_t* host_
         const uint32_t m = (uint32_t)(start[k + 1] - start[k]);
         if (m == 0) continue;
         LCS_CUDA_TRY(cudaStreamWaitEvent(P->class_stream[k], P->class_fork, 0));
-        LCS_CUDA_TRY(launch(1 << k, m, P->class_scenes + start[k], P->class_stream[k]));
+        LCS_CUDA_TRY(launch(1 << k, m, rows_of(flat[start[k]]), P->class_scenes + start[k], P->class_stream[k]));
         lcs_count_launch();
         LCS_CUDA_TRY(cudaEventRecord(P->class_join[k], P->class_stream[k]));
         LCS_CUDA_TRY(cudaStreamWaitEvent(s0, P->class_join[k], 0));
