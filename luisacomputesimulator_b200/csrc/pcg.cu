@@ -7,10 +7,11 @@
 //  * plain  -- the reference's dispatch structure: one kernel per operation (apply
 //              preconditioner, its second pass, update p, SpMV, p.q, its second pass, step)
 //              and a host read-back of r.z every `check_every` iterations;
-//  * fused  -- one persistent cooperative launch for the whole solve: rows are owned by
-//              threads, the three grid-wide reductions per iteration go through bounded
-//              software grid barriers, and every block reduces the per-block partials in the
-//              same fixed order, so all blocks agree on alpha / beta / convergence.
+//  * fused  -- one persistent cooperative launch for the whole solve: the grid-wide reductions
+//              of an iteration go through bounded software grid barriers, and every block reduces
+//              the per-block partials in the same fixed order, so all blocks agree on alpha / beta
+//              / convergence.  Small systems stay in registers (k_pcg_small), larger ones stream
+//              through L2 (k_pcg_fused).
 // Reductions are FP32 (the reference) or FP64 (precision form, LCS_PCG_FP64_DOTS).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -60,16 +61,35 @@ __device__ __forceinline__ float3 mv12(const float4* __restrict__ m, float4 x)
     return y;
 }
 
-// G lanes per row; returns the full row product on every lane of the group
-template <int G>
+// a load that L2 drops before others
+__device__ __forceinline__ float ld_stream(const float* p, uint64_t policy)
+{
+    float v;
+    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+    return v;
+}
+
+// G lanes per row; returns the full row product on every lane of the group.  Stream: A's values are read as data that
+// L2 need not keep.
+template <int G, bool Stream = false>
 __device__ __forceinline__ float3 row_product(uint32_t row, uint32_t lig, const float4* __restrict__ diag,
                                               const Bsr A, const Bsr B, const float4* x)
 {
     float3 acc = make_float3(0.f, 0.f, 0.f);
+    uint64_t policy = 0;
+    if (Stream) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     if (A.rp) {
         const uint32_t e = __ldg(&A.rp[row + 1]);
         for (uint32_t k = __ldg(&A.rp[row]) + lig; k < e; k += G) {
-            const float3 t = mv9(A.val + 9 * (size_t)k, __ldcg(&x[__ldg(&A.col[k])]));
+            float3 t;
+            if (Stream) {
+                float s[9];
+#pragma unroll
+                for (int c = 0; c < 9; ++c) s[c] = ld_stream(A.val + 9 * (size_t)k + c, policy);
+                t = mv9(s, __ldcg(&x[__ldg(&A.col[k])]));
+            } else {
+                t = mv9(A.val + 9 * (size_t)k, __ldcg(&x[__ldg(&A.col[k])]));
+            }
             acc.x += t.x; acc.y += t.y; acc.z += t.z;
         }
     }
@@ -295,59 +315,99 @@ __device__ __forceinline__ void reduce_partials(const FusedArgs& a, int k, int c
     __syncthreads();
 }
 
+__device__ __forceinline__ double warp_sum(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// The inverse of a diagonal block as three columns.
+__device__ __forceinline__ void invert_diag(const float4 c0, const float4 c1, const float4 c2, float4& m0, float4& m1, float4& m2)
+{
+    const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, k = c2.z;
+    const float A = e * k - f * h, B = f * g - d * k, C = d * h - e * g;
+    const float id = 1.0f / (aa * A + bb * B + c * C);
+    m0 = make_float4(A * id, B * id, C * id, 0.0f);
+    m1 = make_float4((c * h - bb * k) * id, (aa * k - c * g) * id, (bb * g - aa * h) * id, 0.0f);
+    m2 = make_float4((bb * f - c * e) * id, (c * d - aa * f) * id, (aa * e - bb * d) * id, 0.0f);
+}
+
+__device__ __forceinline__ float3 mul3(const float4 m0, const float4 m1, const float4 m2, const float4 v)
+{
+    return make_float3(__fmaf_rn(m2.x, v.z, __fmaf_rn(m1.x, v.y, m0.x * v.x)),
+                       __fmaf_rn(m2.y, v.z, __fmaf_rn(m1.y, v.y, m0.y * v.x)),
+                       __fmaf_rn(m2.z, v.z, __fmaf_rn(m1.z, v.y, m0.z * v.x)));
+}
+
+// The persistent solve of systems beyond k_pcg_small.  Bound by HBM and L2 traffic, about 0.8 KB a row and iteration.
+// The matrix is larger than L2 here and is read once an iteration, so its loads ask L2 to evict them first: the vectors
+// and diagonal blocks then stay.  The step's x and r updates and the next preconditioner are one pass.
+// 401,322 rows (13 blocks each, FP64 dots): 6.44 ms with neither, 5.97 ms so; copies of the blocks to shared memory
+// (row_stage.cuh), which pay in k_pcg_batch's smaller blocks, took 8.4 ms against 1,024 threads that read directly.
 template <int G>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
 {
+    constexpr uint32_t W = kFusedThreads / 32;
     __shared__ int s_fail;
-    __shared__ double s_red[kFusedThreads / 32][3];
+    __shared__ double s_red[W][3];
     if (threadIdx.x == 0) s_fail = 0;
-    const uint32_t n = a.n;
+    const uint32_t n = a.n, w = threadIdx.x >> 5, lane = lane_id();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    // the block's partial sums: one double per warp, added in warp order
+    auto publish = [&](double v, int k) {
+        v = warp_sum(v);
+        if (lane == 0) s_red[w][k] = v;
+    };
+    auto block_part = [&](int k, int count) {
+        __syncthreads();
+        if (threadIdx.x < (uint32_t)count) {
+            double v = 0.0;
+            for (uint32_t q = 0; q < W; ++q) v += s_red[q][k + threadIdx.x];
+            a.part[3 * blockIdx.x + k + threadIdx.x] = v;
+        }
+    };
 
-    // x = 0, r = b, p = 0, Minv = inverse(D)
-    for (uint32_t i = tid; i < n; i += nthreads) {
-        a.r[i] = a.b[i];
-        a.p[i] = make_float4(0, 0, 0, 0);
-        a.x[i] = make_float4(0, 0, 0, 0);
-        const float4 c0 = a.diag[3 * i], c1 = a.diag[3 * i + 1], c2 = a.diag[3 * i + 2];
-        const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, k = c2.z;
-        const float A = e * k - f * h, B = f * g - d * k, C = d * h - e * g;
-        const float id = 1.0f / (aa * A + bb * B + c * C);
-        a.minv[3 * i + 0] = make_float4(A * id, B * id, C * id, 0.0f);
-        a.minv[3 * i + 1] = make_float4((c * h - bb * k) * id, (aa * k - c * g) * id, (bb * g - aa * h) * id, 0.0f);
-        a.minv[3 * i + 2] = make_float4((bb * f - c * e) * id, (c * d - aa * f) * id, (aa * e - bb * d) * id, 0.0f);
-    }
-
-    float rz_old = 0.0f, norm_r0 = 0.0f, norm_r = 0.0f, rz = 0.0f;
+    float rz_old = 0.0f, norm_r0 = 0.0f, norm_r = 0.0f, rz = 0.0f, alpha = 0.0f;
     int iter = 0, status = 0;
-    for (iter = 0; iter < a.max_iter; ++iter) {
-        // z = Minv r ; r.r ; r.z
+    for (;; ++iter) {
+        // x += alpha p, r -= alpha q of the step before; z = Minv r; r.r; r.z
         double rr_d = 0.0, rz_d = 0.0;
         float rr_f = 0.0f, rz_f = 0.0f;
-        for (uint32_t i = tid; i < n; i += nthreads) {
-            const float4 rv = a.r[i];
-            const float3 zv = mv12(a.minv + 3 * (size_t)i, rv);
+        for (size_t i = tid; i < n; i += nthreads) {
+            float4 rv, m0, m1, m2;
+            if (iter == 0) {
+                rv = a.b[i];
+                a.p[i] = make_float4(0, 0, 0, 0);
+                a.x[i] = make_float4(0, 0, 0, 0);
+                invert_diag(a.diag[3 * i], a.diag[3 * i + 1], a.diag[3 * i + 2], m0, m1, m2);
+                a.minv[3 * i] = m0;
+                a.minv[3 * i + 1] = m1;
+                a.minv[3 * i + 2] = m2;
+            } else {
+                const float4 pv = a.p[i], qv = __ldcg(&a.q[i]), xv = a.x[i], ro = a.r[i];
+                m0 = a.minv[3 * i];
+                m1 = a.minv[3 * i + 1];
+                m2 = a.minv[3 * i + 2];
+                a.x[i] = make_float4(xv.x + alpha * pv.x, xv.y + alpha * pv.y, xv.z + alpha * pv.z, 0.0f);
+                rv = make_float4(ro.x - alpha * qv.x, ro.y - alpha * qv.y, ro.z - alpha * qv.z, 0.0f);
+            }
+            a.r[i] = rv;
+            const float3 zv = mul3(m0, m1, m2, rv);
             a.z[i] = make_float4(zv.x, zv.y, zv.z, 0.0f);
             const float drr = __fmaf_rn(rv.z, rv.z, __fmaf_rn(rv.y, rv.y, rv.x * rv.x));
             const float drz = __fmaf_rn(rv.z, zv.z, __fmaf_rn(rv.y, zv.y, rv.x * zv.x));
             rr_d += drr; rz_d += drz; rr_f += drr; rz_f += drz;
         }
-        {
-            double v0 = a.fp64 ? rr_d : (double)rr_f, v1 = a.fp64 ? rz_d : (double)rz_f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, o);
-                v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, o);
-            }
-            if (lane_id() == 0) { s_red[threadIdx.x >> 5][0] = v0; s_red[threadIdx.x >> 5][1] = v1; }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t0 = 0, t1 = 0;
-                for (int w = 0; w < kFusedThreads / 32; ++w) { t0 += s_red[w][0]; t1 += s_red[w][1]; }
-                a.part[3 * blockIdx.x + 0] = t0;
-                a.part[3 * blockIdx.x + 1] = t1;
-            }
-        }
+        if (iter >= a.max_iter) break;
+        publish(a.fp64 ? rr_d : (double)rr_f, 0);
+        publish(a.fp64 ? rz_d : (double)rz_f, 1);
+        block_part(0, 2);
         if (!grid_barrier(a, &s_fail)) return;
         double red[2];
         reduce_partials(a, 0, 2, red);
@@ -363,7 +423,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
             if (a.rel_tol > 0.0f && norm_r <= a.rel_tol * norm_r0) break;
         }
         // p = z + beta p
-        for (uint32_t i = tid; i < n; i += nthreads) {
+        for (size_t i = tid; i < n; i += nthreads) {
             const float4 zv = a.z[i], pv = a.p[i];
             a.p[i] = make_float4(zv.x + beta * pv.x, zv.y + beta * pv.y, zv.z + beta * pv.z, 0.0f);
         }
@@ -371,43 +431,205 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
         // q = A p ; p.q
         double pq_d = 0.0;
         float pq_f = 0.0f;
-        {
-            const uint32_t lig = tid % G, ngroups = nthreads / G;
-            const uint32_t rows_round = (n + ngroups - 1) / ngroups * ngroups;
-            for (uint32_t row = tid / G; row < rows_round; row += ngroups) {
-                const uint32_t rr_ = row < n ? row : n - 1;
-                const float3 qv = row_product<G>(rr_, lig, a.diag, a.A, a.B, a.p);
-                if (row < n && lig == 0) {
-                    a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
-                    const float4 pv = __ldcg(&a.p[row]);
-                    const float d = __fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
-                    pq_d += d;
-                    pq_f += d;
-                }
-            }
-            double v = a.fp64 ? pq_d : (double)pq_f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-            if (lane_id() == 0) s_red[threadIdx.x >> 5][2] = v;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t = 0;
-                for (int w = 0; w < kFusedThreads / 32; ++w) t += s_red[w][2];
-                a.part[3 * blockIdx.x + 2] = t;
+        const uint32_t lig = tid % G, ngroups = nthreads / G;
+        const uint32_t rows_round = (n + ngroups - 1) / ngroups * ngroups;
+        for (uint32_t row = tid / G; row < rows_round; row += ngroups) {
+            const uint32_t r = row < n ? row : n - 1;  // whole groups stay converged for the shuffles
+            const float3 qv = row_product<G, true>(r, lig, a.diag, a.A, a.B, a.p);
+            if (row < n && lig == 0) {
+                a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
+                const float4 pv = __ldcg(&a.p[row]);
+                const float d = __fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
+                pq_d += d;
+                pq_f += d;
             }
         }
+        publish(a.fp64 ? pq_d : (double)pq_f, 2);
+        block_part(2, 1);
         if (!grid_barrier(a, &s_fail)) return;
         double pq;
         reduce_partials(a, 2, 1, &pq);
-        const float alpha = safe_div(rz, (float)pq);
-        // x += alpha p ; r -= alpha q
-        for (uint32_t i = tid; i < n; i += nthreads) {
-            const float4 pv = a.p[i], qv = __ldcg(&a.q[i]), xv = a.x[i], rv = a.r[i];
-            a.x[i] = make_float4(xv.x + alpha * pv.x, xv.y + alpha * pv.y, xv.z + alpha * pv.z, 0.0f);
-            a.r[i] = make_float4(rv.x - alpha * qv.x, rv.y - alpha * qv.y, rv.z - alpha * qv.z, 0.0f);
-        }
+        alpha = safe_div(rz, (float)pq);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.stats->iterations = iter;
+        a.stats->rel_residual = norm_r0 > 0.0f ? norm_r / norm_r0 : 0.0f;
+        a.stats->dot_rz = rz_old;
+        if (a.stats->status == LCS_OK) a.stats->status = status;
+    }
+}
+
+// The persistent solve of systems whose rows all have their four lanes at once (BT / 4 rows per block, one block per
+// SM).  Latency bounds it, so everything but the vectors that cross blocks stays in registers: the row's vectors and
+// diagonal blocks (the same on its four lanes) and up to four blocks of A per lane.  z crosses, and p is formed where
+// it is read, z + beta p_old, with two alternating buffers of p_old; that leaves two grid-wide exchanges per iteration,
+// and each exchange is one trip: a block's partial sums carry the exchange's number in their low four bits (see
+// res_allgather3) and are its arrival at the barrier too (release / acquire).
+// 100 iterations: 400 rows 1.19 ms as k_pcg_fused, 0.37 ms so; 4,096 rows 1.35 and 0.64; 10,000 rows 1.24 and 0.69.
+__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+constexpr int kSmallMaxBlocks = 256;
+constexpr int kSmallBlocksPerLane = 4;
+
+template <int BT>
+__global__ void __launch_bounds__(BT, 1) k_pcg_small(FusedArgs a)
+{
+    __shared__ double s_warp[2][BT / 32];
+    __shared__ double s_part[2][kSmallMaxBlocks];
+    __shared__ int s_fail;
+    const uint32_t t = threadIdx.x, lane = lane_id(), lig = t & 3u, n = a.n;
+    const uint32_t row = blockIdx.x * (BT / 4) + t / 4;
+    const bool own = row < n, lead = own && lig == 0;
+    const size_t i = own ? row : n - 1;
+    if (t == 0) s_fail = 0;
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(a.part);
+    unsigned step = 0;  // exchanges done
+    auto exchange = [&](double v0, double v1, int count, double* out) -> bool {
+        const unsigned long long tag = step % 15u;
+        unsigned long long* buf = slots + 2 * (size_t)(step & 1u) * gridDim.x;
+        ++step;
+        v0 = warp_sum(v0);
+        if (count > 1) v1 = warp_sum(v1);
+        if (lane == 0) {
+            s_warp[0][t >> 5] = v0;
+            s_warp[1][t >> 5] = v1;
+        }
+        __syncthreads();
+        if (t == 0) {
+            double b0 = 0.0, b1 = 0.0;
+#pragma unroll
+            for (int w = 0; w < BT / 32; ++w) {
+                b0 += s_warp[0][w];
+                b1 += s_warp[1][w];
+            }
+            if (count > 1)
+                st_relaxed_u64(&buf[2 * blockIdx.x + 1], ((unsigned long long)__double_as_longlong(b1) & ~0xFull) | tag);
+            st_release_u64(&buf[2 * blockIdx.x], ((unsigned long long)__double_as_longlong(b0) & ~0xFull) | tag);
+        }
+        for (uint32_t k = t; k < (uint32_t)count * gridDim.x; k += BT) {
+            const uint32_t j = k / gridDim.x, b = k % gridDim.x;
+            unsigned long long bits;
+            unsigned it = 0;
+            while (((bits = ld_acquire_u64(&buf[2 * b + j])) & 0xFull) != tag) {
+                if (++it > kBarrierSpinLimit) {
+                    s_fail = 1;
+                    a.stats->status = LCS_ERR_TIMEOUT;
+                    break;
+                }
+            }
+            s_part[j][b] = __longlong_as_double((long long)(bits & ~0xFull));
+        }
+        __syncthreads();
+        if (s_fail) return false;
+        double o[2] = {0.0, 0.0};
+        for (uint32_t b = lane; b < gridDim.x; b += 32) {
+            o[0] += s_part[0][b];
+            if (count > 1) o[1] += s_part[1][b];
+        }
+        out[0] = warp_sum(o[0]);
+        if (count > 1) out[1] = warp_sum(o[1]);
+        return true;
+    };
+
+    // the row's blocks of A: the lane's first four in registers, the rest read again each time
+    float blk[kSmallBlocksPerLane][9];
+    uint32_t bcol[kSmallBlocksPerLane];
+    uint32_t a_next = 0, a_end = 0, b_lo = 0, b_hi = 0;
+    int held = 0;
+    if (own && a.A.rp) {
+        a_end = __ldg(&a.A.rp[row + 1]);
+        a_next = __ldg(&a.A.rp[row]) + lig;
+    }
+    if (own && a.B.rp) {
+        b_lo = __ldg(&a.B.rp[row]) + lig;
+        b_hi = __ldg(&a.B.rp[row + 1]);
+    }
+#pragma unroll
+    for (int u = 0; u < kSmallBlocksPerLane; ++u) {
+        bcol[u] = 0;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) blk[u][e] = 0.0f;
+        if (a_next < a_end) {
+            bcol[u] = __ldg(&a.A.col[a_next]);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) blk[u][e] = __ldg(&a.A.val[9 * (size_t)a_next + e]);
+            a_next += 4;
+            held = u + 1;
+        }
+    }
+    const float4 d0 = a.diag[3 * i], d1 = a.diag[3 * i + 1], d2 = a.diag[3 * i + 2];
+    float4 m0, m1, m2;
+    invert_diag(d0, d1, d2, m0, m1, m2);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 rv = own ? a.b[i] : zero, xv = zero, pv = zero;
+    float3 qv = make_float3(0.f, 0.f, 0.f);
+    __syncthreads();
+
+    float rz_old = 0.0f, norm_r0 = 0.0f, norm_r = 0.0f, rz = 0.0f, alpha = 0.0f;
+    int iter = 0, status = 0;
+    for (;; ++iter) {
+        if (iter > 0) {
+            xv = make_float4(xv.x + alpha * pv.x, xv.y + alpha * pv.y, xv.z + alpha * pv.z, 0.0f);
+            rv = make_float4(rv.x - alpha * qv.x, rv.y - alpha * qv.y, rv.z - alpha * qv.z, 0.0f);
+        }
+        if (iter >= a.max_iter) break;
+        const float3 zv = mul3(m0, m1, m2, rv);
+        if (lead) __stcg(&a.z[i], make_float4(zv.x, zv.y, zv.z, 0.0f));
+        const float drr = __fmaf_rn(rv.z, rv.z, __fmaf_rn(rv.y, rv.y, rv.x * rv.x));
+        const float drz = __fmaf_rn(rv.z, zv.z, __fmaf_rn(rv.y, zv.y, rv.x * zv.x));
+        double red[2];
+        if (!exchange(lead ? (double)drr : 0.0, lead ? (double)drz : 0.0, 2, red)) return;
+        const float rr = (float)red[0];
+        rz = (float)red[1];
+        const float beta = safe_div(rz, rz_old);
+        rz_old = rz;
+        norm_r = sqrtf(rr);
+        if (iter == 0) norm_r0 = norm_r;
+        if (iter % a.check_every == 0) {
+            if (isnan(rz) || isinf(rz)) { status = LCS_ERR_NAN; break; }
+            if (rz < a.abs_rz_tol) break;
+            if (a.rel_tol > 0.0f && norm_r <= a.rel_tol * norm_r0) break;
+        }
+        const float4* p_old = iter & 1 ? a.q : a.p;
+        float4* p_new = iter & 1 ? a.p : a.q;
+        auto ld_p = [&](uint32_t c) -> float4 {
+            const float4 zc = __ldcg(&a.z[c]);
+            const float4 pc = iter > 0 ? __ldcg(&p_old[c]) : zero;
+            return make_float4(zc.x + beta * pc.x, zc.y + beta * pc.y, zc.z + beta * pc.z, 0.0f);
+        };
+        pv = make_float4(zv.x + beta * pv.x, zv.y + beta * pv.y, zv.z + beta * pv.z, 0.0f);
+        if (lead) __stcg(&p_new[i], pv);
+        float3 acc = make_float3(0.f, 0.f, 0.f);
+        {
+            float4 v[kSmallBlocksPerLane];
+#pragma unroll
+            for (int u = 0; u < kSmallBlocksPerLane; ++u)
+                if (u < held) v[u] = ld_p(bcol[u]);
+#pragma unroll
+            for (int u = 0; u < kSmallBlocksPerLane; ++u)
+                if (u < held) stage::add_block(blk[u], v[u], acc);
+        }
+        stage::direct_blocks<4>(stage::Csr{a.A.rp, a.A.col, a.A.val}, a_next, a_end, ld_p, acc);
+        stage::direct_blocks<4>(stage::Csr{a.B.rp, a.B.col, a.B.val}, b_lo, b_hi, ld_p, acc);
+        __syncwarp();
+        stage::group_sum<4>(acc);
+        const float3 dv = mul3(d0, d1, d2, pv);
+        qv = make_float3(dv.x + acc.x, dv.y + acc.y, dv.z + acc.z);
+        const float d = __fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
+        double pq[2];
+        if (!exchange(lead ? (double)d : 0.0, 0.0, 1, pq)) return;
+        alpha = safe_div(rz, (float)pq[0]);
+    }
+    if (lead) a.x[i] = xv;
+    if (blockIdx.x == 0 && t == 0) {
         a.stats->iterations = iter;
         a.stats->rel_residual = norm_r0 > 0.0f ? norm_r / norm_r0 : 0.0f;
         a.stats->dot_rz = rz_old;
@@ -1325,10 +1547,6 @@ __device__ __forceinline__ bool res_publish_wait(unsigned* flags, unsigned tag, 
 // (the same sums in every block).  Slots alternate between two buffers by iteration parity: a block can
 // only rewrite a buffer after every block has read it, since its next partial needs the next iteration's
 // sums, which need every block's next partial, which each block writes only after reading this one.
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v)
-{
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p)
 {
     unsigned long long v;
@@ -1777,13 +1995,6 @@ __device__ __forceinline__ uint32_t cluster_ctas()
     return n;
 }
 
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-
 // sum of `count` values over a scene's chunks in a fixed order, the same in every warp of the cluster
 __device__ __forceinline__ void scene_sum(const double* cp, uint32_t nchunks, int k, int count, double* out)
 {
@@ -2070,6 +2281,14 @@ extern "C" int lcs_debug_pcg_wait(int32_t which, int32_t missing_block, uint32_t
     return h.status;
 }
 
+// 1 if the device holds a block of the persistent solve on each SM, else 0
+static int fused_per_sm()
+{
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused<kRowLanes>, kFusedThreads, 0) != cudaSuccess) return 0;
+    return per_sm > 0 ? 1 : 0;
+}
+
 extern "C" int lcs_pcg_create(uint32_t n, lcs_pcg** out)
 {
     if (!out || n == 0) return lcs_fail(LCS_ERR_INVALID, "lcs_pcg_create: bad argument");
@@ -2079,8 +2298,7 @@ extern "C" int lcs_pcg_create(uint32_t n, lcs_pcg** out)
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused<kRowLanes>, kFusedThreads, 0);
-    if (per_sm > 1) per_sm = 1;
+    per_sm = fused_per_sm();
     p->fused_grid = sms * (per_sm > 0 ? per_sm : 1);
     // fused: 3 doubles per block; row-resident: 4 per block, twice (alternate iterations) for up to kRowMaxBlocks
     const int parts = 8 * kRowMaxBlocks / 3 + 1 + (p->fused_grid > kPlainBlocks ? p->fused_grid : kPlainBlocks);
@@ -2480,6 +2698,28 @@ int lcs_pcg_solve_sell(lcs_pcg* P, const float* diag, const uint32_t* slice_ptr,
                       (cudaStream_t)stream, c_ptr, c_col, c_val, c_ok);
 }
 
+// The persistent solve on at most `grid` co-resident blocks (one per SM); a.part holds 4 doubles per block.  Rows that
+// fit four lanes each in one block of 256 or 512 threads per SM take k_pcg_small.
+static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
+{
+    // the partial sums' tags (small), the barrier arrival counter and the stats have to be set; the rest is written
+    // before it is read
+    LCS_CUDA_TRY(cudaMemsetAsync(a.stats, 0, sizeof(lcs_pcg_stats), s));
+    void* args[] = {&a};
+    const uint64_t cap = (uint64_t)std::min(grid, kSmallMaxBlocks);
+    if (a.n <= 128 * cap) {
+        const uint32_t bt = a.n <= 64 * cap ? 256 : 512, blocks = (a.n + bt / 4 - 1) / (bt / 4);
+        LCS_CUDA_TRY(cudaMemsetAsync(a.part, 0xFF, 4 * sizeof(double) * blocks, s));
+        LCS_CUDA_TRY(cudaLaunchCooperativeKernel(bt == 256 ? (const void*)k_pcg_small<256> : (const void*)k_pcg_small<512>,
+                                                 dim3(blocks), dim3(bt), args, 0, s));
+    } else {
+        LCS_CUDA_TRY(cudaMemsetAsync(a.bar_count, 0, sizeof(unsigned), s));
+        LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(grid), dim3(kFusedThreads), args, 0, s));
+    }
+    lcs_count_launch();
+    return LCS_OK;
+}
+
 extern "C" int lcs_pcg_solve(lcs_pcg* P, const float* diag, const lcs_bsr* A, const lcs_bsr* B, const float* b,
                              float* x, const lcs_pcg_opts* opts, lcs_pcg_stats* stats, lcs_stream stream)
 {
@@ -2531,12 +2771,8 @@ extern "C" int lcs_pcg_solve(lcs_pcg* P, const float* diag, const lcs_bsr* A, co
     a.check_every = o.check_every;
     a.fp64 = (o.flags & LCS_PCG_FP64_DOTS) ? 1 : 0;
     a.stats = P->d_stats;
-    LCS_CUDA_TRY(cudaMemsetAsync(P->d_stats, 0, sizeof(lcs_pcg_stats), s));
-    LCS_CUDA_TRY(cudaMemsetAsync(P->bar, 0, sizeof(unsigned), s));
-    void* args[] = {&a};
-    LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(P->fused_grid), dim3(kFusedThreads), args,
-                                             0, s));
-    lcs_count_launch();
+    int rc = launch_persistent(a, P->fused_grid, s);
+    if (rc != LCS_OK) return rc;
     if (stats && !(o.flags & LCS_PCG_NO_STATS)) {
         LCS_CUDA_TRY(cudaMemcpyAsync(stats, P->d_stats, sizeof(lcs_pcg_stats), cudaMemcpyDeviceToHost, s));
         LCS_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2631,7 +2867,7 @@ extern "C" int lcs_pcg_solve_noalloc(uint32_t n, const float* diag, const lcs_bs
             }
             int sms = 0, per_sm = 0;
             LCS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            LCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused<kRowLanes>, kFusedThreads, 0));
+            per_sm = fused_per_sm();
             int grid = sms * (per_sm > 0 ? 1 : 0);
             if (grid <= 0 || grid > (int)kNoAllocMaxBlocks)
                 return lcs_fail(LCS_ERR_CUDA, "lcs_pcg_solve_noalloc: no co-resident launch shape");
@@ -2663,14 +2899,8 @@ extern "C" int lcs_pcg_solve_noalloc(uint32_t n, const float* diag, const lcs_bs
     a.check_every = o.check_every;
     a.fp64 = (o.flags & LCS_PCG_FP64_DOTS) ? 1 : 0;
     a.stats = reinterpret_cast<lcs_pcg_stats*>(base + kNaOffStats);
-    // the barrier arrival counter and the stats must start at zero; the rest is written
-    // before it is read
-    LCS_CUDA_TRY(cudaMemsetAsync(a.bar_count, 0, sizeof(unsigned), s));
-    LCS_CUDA_TRY(cudaMemsetAsync(a.stats, 0, sizeof(lcs_pcg_stats), s));
-    void* args[] = {&a};
-    LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(nd.grid), dim3(kFusedThreads),
-                                             args, 0, s));
-    lcs_count_launch();
+    const int rc = launch_persistent(a, nd.grid, s);
+    if (rc != LCS_OK) return rc;
     if (stats && !(o.flags & LCS_PCG_NO_STATS)) {
         LCS_CUDA_TRY(cudaMemcpyAsync(stats, a.stats, sizeof(lcs_pcg_stats), cudaMemcpyDeviceToHost, s));
         LCS_CUDA_TRY(cudaStreamSynchronize(s));
