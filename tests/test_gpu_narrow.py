@@ -177,3 +177,27 @@ def test_ccd_fp64_form_matches_fp64_oracle(name):
         _, t32 = (O.ccd_ee if is_ee else O.ccd_vf)(p, x0, x1, el, sc.body, sc.offset)
         m = ref < 1.25
         assert np.all(np.abs(t32[m] - ref[m]) <= 1e-6 * ref[m])
+
+
+@pytest.mark.parametrize("n", [700, 32768, 32769])       # a warp per row, and per four rows
+@pytest.mark.parametrize("shared", [1, 10, 11, 170, 171, 200])  # row 0 holds 3 entries per pair: 512 is the staged limit
+def test_assembly_row_order_at_the_edges(n, shared):
+    _, _, _, got, _ = _dcd("cloth_sphere")
+    pairs = np.resize(got, shared + 8)
+    bits = pairs["idx"] & np.uint32(0x80000000)
+    k = np.arange(len(pairs), dtype=np.uint32)
+    own = np.stack([np.zeros_like(k), 1 + 3 * (k % 200), 2 + 3 * (k % 200), 3 + 3 * (k % 200)], 1)
+    own[shared:, 0] = n - 1  # and the last row a few
+    pairs["idx"] = own.astype(np.uint32) | bits
+    pairs = np.random.default_rng(shared).permutation(pairs)
+    det = NarrowPhasesDetector(n, n)
+    assert len(pairs) <= det.cap_pairs
+    raw = torch.from_numpy(np.ascontiguousarray(pairs).view(np.uint8).copy()).cuda()
+    det.narrow_phase_list.view(torch.uint8).reshape(-1)[:raw.numel()] = raw
+    det.counts[2] = len(pairs)
+    det.device_assemble_contact_triplet()
+    rp, col, val = O.contact_offdiag_bsr(pairs, n)
+    g_rp, g_col, g_val = det.assembler.export(n, 12 * len(pairs))
+    np.testing.assert_array_equal(host(g_rp, np.uint32), rp)
+    np.testing.assert_array_equal(host(g_col, np.uint32), col)
+    np.testing.assert_array_equal(host(g_val), val)
