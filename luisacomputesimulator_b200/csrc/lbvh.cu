@@ -21,6 +21,10 @@
 
 using namespace lcs;
 
+// query calls on one tree that may be in flight at once with different arguments
+constexpr uint32_t kSymSlots = 1024;
+constexpr uint32_t kMaxTops = 4096;  // listed tops of the parts of a tree where a walk may end early
+
 struct lcs_bvh {
     int kind = 0;
     uint32_t n = 0, ni = 0, nb = 0;  // leaves, inner nodes, 256-element blocks
@@ -56,7 +60,11 @@ struct lcs_bvh {
     float4* seg_box = nullptr;       // 2 per 32 union-order positions (whole refit chunks): {min | 0}{max | 0}
     float4* chunk_box = nullptr;     // 2 per refit chunk: its union
     uint32_t* healthy = nullptr;     // 1
-    uint32_t* maxdepth = nullptr;    // 1: depth of the deepest inner node (root: 0), capped at 256
+    uint32_t* turns = nullptr;       // 2 + kMaxTops: see k_depth_parity
+    uint32_t* top_lefts = nullptr;   // 32 * kMaxTops: slots of the 31 inner left siblings above each listed top
+    uint32_t* early = nullptr;       // kSymSlots: number of the query call that may end early, a slot per call in turn
+    uint32_t* sym_info = nullptr;    // kSymSlots x 4: k_sym_check's findings, a slot per query call in turn
+    mutable uint32_t calls = 0;
     bool built = false;              // a construct has written the topology, slots and refit tables
 };
 
@@ -166,11 +174,11 @@ static_assert((1u << kRefitLevels) == kRefitSegs, "one sparse-table level per do
 // its left child's range in swap_diff (see k_eorder)
 __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* __restrict__ sgo, uint32_t n,
                               uint32_t* __restrict__ parent, uint2* __restrict__ children,
-                              uint32_t* __restrict__ slot, float4* __restrict__ wide, uint32_t* __restrict__ maxdepth,
+                              uint32_t* __restrict__ slot, float4* __restrict__ wide, uint32_t* __restrict__ max_pending,
                               uint2* __restrict__ range, uint32_t* __restrict__ swap_diff)
 {
     const int ni = (int)n - 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *maxdepth = 0u;  // raised by k_depth_parity, launched after this
+    if (blockIdx.x == 0 && threadIdx.x == 0) max_pending[0] = max_pending[1] = 0u;  // raised by k_depth_parity, launched after this
     for (int nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
         int i = 0, j = ni;
         if (nid != 0) {
@@ -235,21 +243,47 @@ __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* _
 // overlap test passes.  A traversal then takes one dependent
 // 128-B fetch where the binary walk took two 64-B ones.  k_depth_parity marks the even-depth inner nodes
 // after each build (a climb to the root per node, at most 256 levels).
-__global__ void k_depth_parity(const uint32_t* __restrict__ parent, uint32_t ni, uint8_t* __restrict__ even,
-                               uint32_t* __restrict__ maxdepth)
+// It also counts, for each inner node, the nodes that a walk of the reference can at most have pending when it pops it:
+// one for every ancestor whose second child the path takes and whose first child is an inner node.  turns: [0] the
+// largest count, [1] how many nodes reach kRefPending by their own turn (every node with as many descends from one of
+// them), [2...] the slots of the first kMaxTops of those, whose 31 inner left siblings top_lefts lists.
+constexpr uint32_t kRefStack = 32;
+constexpr uint32_t kRefPending = kRefStack - 1;
+
+__global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* __restrict__ children, uint32_t ni,
+                               uint8_t* __restrict__ even, uint32_t* __restrict__ turns,
+                               uint32_t* __restrict__ top_lefts)
 {
-    uint32_t deepest = 0;
+    uint32_t most = 0;
     for (uint32_t nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
-        uint32_t p = nid, d = 0;
+        uint32_t p = nid, d = 0, pending = 0;
+        bool own = false;
         while (p != 0u && p < ni && d < 256u) {
-            p = parent[p];
+            const uint32_t s = slot[p];
+            p = s >> 1;
+            if ((s & 1u) && p < ni && children[p].x < ni) {
+                ++pending;
+                own = own || d == 0u;
+            }
             ++d;
         }
         even[nid] = (d & 1u) == 0u ? 1 : 0;
-        deepest = d > deepest ? d : deepest;
+        most = pending > most ? pending : most;
+        if (own && pending == kRefPending) {
+            const uint32_t k = atomicAdd(&turns[1], 1u);
+            if (k < kMaxTops) {
+                turns[2 + k] = slot[nid];
+                uint32_t i = 0;
+                for (p = nid; p != 0u && i < kRefPending;) {
+                    const uint32_t s = slot[p];
+                    p = s >> 1;
+                    if ((s & 1u) && children[p].x < ni) top_lefts[32 * k + i++] = s & ~1u;
+                }
+            }
+        }
     }
-    deepest = __reduce_max_sync(0xFFFFFFFFu, deepest);
-    if (lane_id() == 0 && deepest) atomicMax(maxdepth, deepest);
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    if (lane_id() == 0 && most) atomicMax(&turns[0], most);
 }
 
 // the 4-wide record of inner node b from the binary records (leaf_only: a one-leaf tree, whose two slots
@@ -632,14 +666,122 @@ __global__ void k_refit_span_records(const uint32_t* __restrict__ spans, const u
 // and fn_query_from_edges_v2 (EE = true, lbvh.cpp:810-846)
 constexpr int kStack4 = 64;  // entries of the 4-wide traversal stack
 
-// The reference's stack holds at most one pending node per level above the node it pops (children are
-// pushed left, right and the right one is popped next), so it can only fill -- and end a query early --
-// in a tree with an inner node at depth >= 32.  k_depth_parity records the deepest inner node after each
-// build; the 4-wide walks below serve the trees where that early exit cannot happen (their own 64-entry
-// stack then holds at most 3 nodes per 4-wide level: 48), and k_query_ref restates the reference's walk,
-// early exit included, on the others.  Each launch reads the depth and returns at once when the tree is
-// the other kind, so the choice costs no host synchronisation.
-constexpr uint32_t kRefStack = 32;
+// The reference's stack (32 entries; children are pushed left, right and the right one is popped next) holds one
+// pending node for each right turn of the path past an inner left child that overlaps the query, so it can only fill --
+// and end a query early -- below one of the tops that k_depth_parity lists.  Every call first asks (k_may_end) whether
+// any of its queries could meet a full stack there; if none can, the 4-wide walks below serve it (their own 64-entry
+// stack holds at most two nodes per turn), else k_query_ref restates the reference's walk, early exit included.  Each
+// launch reads the answer and returns at once if it is the other's call, so the choice costs no host
+// synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
+// with a few paths of 31 turns near one corner, but no query keeps more than a handful of nodes pending.
+struct Early {
+    const uint32_t* turns;
+    const uint32_t* flag;  // the call's slot: its number if it may end early
+    uint32_t call;
+    __device__ __forceinline__ bool operator()() const { return __ldg(&turns[0]) >= kRefPending && *flag == call; }
+};
+
+// the box of query q: an edge (EE) or a vertex, swept, widened by per-vertex thickness + d_hat, or by one radius for
+// every query (the once-per-pair EE form's callers: thickness 0 and one d_hat)
+template <bool EE>
+__device__ __forceinline__ void query_box(const float4* x0, const float4* x1, const uint2* edges, const float* dhat,
+                                          const float* thickness, float uniform_r, uint32_t q, float* box)
+{
+    v3 mn, mx;
+    uint32_t v0;
+    if (EE) {
+        const uint2 ed = __ldg(&edges[q]);
+        const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
+        mn = min3(min3(s0, s1), min3(e0, e1));
+        mx = max3(max3(s0, s1), max3(e0, e1));
+        v0 = ed.x;
+    } else {
+        const v3 a = ld3(x0, q), b = ld3(x1, q);
+        mn = min3(a, b);
+        mx = max3(a, b);
+        v0 = q;
+    }
+    const float dh = dhat ? __ldg(&dhat[v0]) : uniform_r;
+    const float r = dhat ? __ldg(&thickness[v0]) + dh : uniform_r;
+    box[0] = mn.x - r; box[1] = mn.y - r; box[2] = mn.z - r;
+    box[3] = mx.x + r; box[4] = mx.y + r; box[5] = mx.z + r;
+    if (!EE && dh < 0.0f) {  // a vertex with a negative d_hat (affine-body DOF slot) queries nothing
+        box[0] = box[1] = box[2] = __int_as_float(0x7f800000);
+        box[3] = box[4] = box[5] = __int_as_float(0xff800000);
+    }
+}
+
+// Marks the call if one of its queries overlaps a listed top with so many overlapping inner left siblings above it that,
+// were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's walk
+// reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and a near
+// top's left siblings, one per lane, against the union of its 32 queries' boxes; only where that is not enough does each
+// query climb.
+template <bool EE>
+__global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide, const uint32_t* __restrict__ slot,
+                                                 const uint32_t* __restrict__ turns, const uint32_t* __restrict__ top_lefts,
+                                                 const float4* __restrict__ x0,
+                                                 const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                 uint32_t n_queries, const float* __restrict__ dhat,
+                                                 const float* __restrict__ thickness, float uniform_r,
+                                                 const uint32_t* __restrict__ order, uint32_t call, uint32_t* __restrict__ flag)
+{
+    const uint32_t most = turns[0], tops = turns[1];
+    if (most < kRefPending) return;
+    if (tops > kMaxTops) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *flag = call;
+        return;
+    }
+    const uint32_t lane = lane_id(), n_round = (n_queries + 31u) & ~31u;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_round; t += gridDim.x * blockDim.x) {
+        float box[6], all[6];
+        box[0] = box[1] = box[2] = __int_as_float(0x7f800000);
+        box[3] = box[4] = box[5] = __int_as_float(0xff800000);
+        if (t < n_queries) query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, order ? __ldg(&order[t]) : t, box);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            all[c] = box[c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float v = __shfl_xor_sync(0xFFFFFFFFu, all[c], o);
+                all[c] = c < 3 ? fminf(all[c], v) : fmaxf(all[c], v);
+            }
+        }
+        for (uint32_t k0 = 0; k0 < tops; k0 += 32) {
+            uint32_t top = 0;
+            bool near = false;
+            if (k0 + lane < tops) {
+                top = turns[2 + k0 + lane];
+                float4 mn, mx;
+                ld_slot(wide + 2 * (size_t)top, mn, mx);
+                near = overlap(mn, mx, all);
+            }
+            for (uint32_t m = __ballot_sync(0xFFFFFFFFu, near); m; m &= m - 1) {
+                uint32_t s = __shfl_sync(0xFFFFFFFFu, top, __ffs(m) - 1), pending = 0;
+                float4 mn, mx;
+                bool left = false;
+                if (lane < kRefPending) {
+                    ld_slot(wide + 2 * (size_t)top_lefts[32 * (size_t)(k0 + __ffs(m) - 1) + lane], mn, mx);
+                    left = overlap(mn, mx, all);
+                }
+                const uint32_t bound = __popc(__ballot_sync(0xFFFFFFFFu, left));
+                if (bound + (most - kRefPending) + 2 < kRefStack) continue;
+                ld_slot(wide + 2 * (size_t)s, mn, mx);
+                if (!overlap(mn, mx, box)) continue;
+                for (int d = 0; d < 256; ++d) {
+                    const uint32_t p = s >> 1;
+                    if (s & 1u) {
+                        ld_slot(wide + 4 * (size_t)p, mn, mx);
+                        if (!(__float_as_uint(mn.w) & 0x80000000u) && overlap(mn, mx, box)) ++pending;
+                    }
+                    if (p == 0u) break;
+                    s = slot[p];
+                }
+                if (pending + (most - kRefPending) + 2 >= kRefStack) *flag = call;
+            }
+            __syncwarp();
+        }
+    }
+}
 
 template <bool EE>
 __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4, uint32_t n_leaves,
@@ -648,38 +790,17 @@ __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4,
                                                const float* __restrict__ dhat, const float* __restrict__ thickness,
                                                uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count,
                                                const uint32_t* __restrict__ order, uint32_t* capped,
-                                               const uint32_t* __restrict__ maxdepth)
+                                               const Early early,
+                                               const uint32_t* __restrict__ sym_info)
 {
-    if (__ldg(maxdepth) >= kRefStack) return;
+    if (early()) return;
+    if (EE && sym_info && sym_info[0] == 0u) return;  // k_query_ee_sym<true> serves the call
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_queries; t += gridDim.x * blockDim.x) {
         // queries in the order of `order` (the tree's Morton order when the queries are its own
         // leaves): neighbouring threads then walk nearly the same nodes
         const uint32_t q = order ? __ldg(&order[t]) : t;
         float box[6];
-        {
-            v3 mn, mx;
-            uint32_t v0;
-            if (EE) {
-                uint2 ed = __ldg(&edges[q]);
-                v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
-                mn = min3(min3(s0, s1), min3(e0, e1));
-                mx = max3(max3(s0, s1), max3(e0, e1));
-                v0 = ed.x;
-            } else {
-                v3 a = ld3(x0, q), b = ld3(x1, q);
-                mn = min3(a, b);
-                mx = max3(a, b);
-                v0 = q;
-            }
-            const float dh = __ldg(&dhat[v0]);
-            const float r = __ldg(&thickness[v0]) + dh;
-            box[0] = mn.x - r; box[1] = mn.y - r; box[2] = mn.z - r;
-            box[3] = mx.x + r; box[4] = mx.y + r; box[5] = mx.z + r;
-            if (!EE && dh < 0.0f) {  // a vertex with a negative d_hat (affine-body DOF slot) queries nothing
-                box[0] = box[1] = box[2] = __int_as_float(0x7f800000);
-                box[3] = box[4] = box[5] = __int_as_float(0xff800000);
-            }
-        }
+        query_box<EE>(x0, x1, edges, dhat, thickness, 0.0f, q, box);
         uint32_t stack[kStack4];
         int sp = 0;
         uint32_t loop = 0;
@@ -717,8 +838,8 @@ __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4,
     }
 }
 
-// query_template2 as the reference runs it (lbvh.cpp:293-360) on the binary records, for trees with an
-// inner node at depth >= 32 (see kRefStack): a stack of 32 inner nodes starting at the root, the two
+// query_template2 as the reference runs it (lbvh.cpp:293-360) on the binary records, for calls in
+// which the stack may fill (see Early): a stack of 32 inner nodes starting at the root, the two
 // children tested in order (left, then right) and the right one popped first; an inner child that meets a
 // full stack ends the whole query (the pairs found so far stay), and so does the 100001st popped node.
 // Both early exits are reported through `capped`.  EE keeps the reference's eid < adj filter.
@@ -728,37 +849,12 @@ __global__ void __launch_bounds__(128) k_query_ref(const float4* __restrict__ wi
                                                    uint32_t n_queries, const float* __restrict__ dhat,
                                                    const float* __restrict__ thickness, float uniform_r,
                                                    uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count,
-                                                   uint32_t* capped, const uint32_t* __restrict__ maxdepth)
+                                                   uint32_t* capped, const Early early)
 {
-    if (__ldg(maxdepth) < kRefStack) return;
+    if (!early()) return;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n_queries; q += gridDim.x * blockDim.x) {
         float box[6];
-        {
-            v3 mn, mx;
-            uint32_t v0;
-            if (EE) {
-                const uint2 ed = __ldg(&edges[q]);
-                const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
-                mn = min3(min3(s0, s1), min3(e0, e1));
-                mx = max3(max3(s0, s1), max3(e0, e1));
-                v0 = ed.x;
-            } else {
-                const v3 a = ld3(x0, q), b = ld3(x1, q);
-                mn = min3(a, b);
-                mx = max3(a, b);
-                v0 = q;
-            }
-            // per-vertex thickness + d_hat, or one radius for every query (the once-per-pair EE form's
-            // callers: thickness 0 and one d_hat)
-            const float dh = dhat ? __ldg(&dhat[v0]) : uniform_r;
-            const float r = dhat ? __ldg(&thickness[v0]) + dh : uniform_r;
-            box[0] = mn.x - r; box[1] = mn.y - r; box[2] = mn.z - r;
-            box[3] = mx.x + r; box[4] = mx.y + r; box[5] = mx.z + r;
-            if (!EE && dh < 0.0f) {  // a vertex with a negative d_hat (affine-body DOF slot) queries nothing
-                box[0] = box[1] = box[2] = __int_as_float(0x7f800000);
-                box[3] = box[4] = box[5] = __int_as_float(0xff800000);
-            }
-        }
+        query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
         uint32_t stack[kRefStack];
         int sp = 0;
         uint32_t loop = 0;
@@ -794,37 +890,216 @@ __global__ void __launch_bounds__(128) k_query_ref(const float4* __restrict__ wi
     }
 }
 
+constexpr uint32_t kPacketPairs = 256;  // pairs a warp collects before it appends them to the list
+// Leaves from which the warp walk is taken: 6,658 vertices (19,900 edges) 52 us a query by the lane walk, 67 by the
+// warp walk; 88,800 vertices (265,800 edges) 447 and 343.
+constexpr uint32_t kPacketLeaves = 65536;
+constexpr int kPacketStack = 128;       // two nodes per turn on paths of at most 62 levels, and a record's four
+
+// floats as unsigned integers of the same order
+__device__ __forceinline__ uint32_t ordered(float f)
+{
+    const uint32_t u = __float_as_uint(f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(uint32_t u)
+{
+    return __uint_as_float(u & 0x80000000u ? u & 0x7FFFFFFFu : ~u);
+}
+
+// Whether a general EE query may take the once-per-pair walk: its edges, positions and thicknesses are, bit for bit,
+// those of the tree's leaf boxes.  info (zeroed before): [0] leaves that differ or whose radius is not finite, [1] the
+// largest d_hat, [2] the largest thickness + d_hat (as `ordered`).
+__global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wide, const uint32_t* __restrict__ sgo,
+                                                   const uint32_t* __restrict__ slot, uint32_t n,
+                                                   const float4* __restrict__ x0, const float4* __restrict__ x1,
+                                                   const uint2* __restrict__ edges, const float* __restrict__ dhat,
+                                                   const float* __restrict__ thickness, uint32_t* __restrict__ info)
+{
+    uint32_t bad = 0, dm = 0, rm = 0;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const uint32_t q = sgo[t], s = slot[n - 1 + t];
+        v3 mn, mx;
+        leaf_box(LCS_TREE_EDGE, q, thickness, x0, x1, reinterpret_cast<const uint32_t*>(edges), mn, mx);
+        float4 a, b;
+        ld_slot(wide + 4 * (size_t)(s >> 1) + 2 * (s & 1u), a, b);
+        const uint32_t v0 = __ldg(&edges[q].x);
+        const float d = __ldg(&dhat[v0]), r = __ldg(&thickness[v0]) + d;
+        if (!(mn.x == a.x && mn.y == a.y && mn.z == a.z && mx.x == b.x && mx.y == b.y && mx.z == b.z) || !isfinite(d) ||
+            !isfinite(r))
+            bad = 1;
+        dm = max(dm, ordered(d));
+        rm = max(rm, ordered(r));
+    }
+    bad = __reduce_max_sync(0xFFFFFFFFu, bad);
+    dm = __reduce_max_sync(0xFFFFFFFFu, dm);
+    rm = __reduce_max_sync(0xFFFFFFFFu, rm);
+    if (lane_id() == 0) {
+        if (bad) atomicOr(&info[0], 1u);
+        atomicMax(&info[1], dm);
+        atomicMax(&info[2], rm);
+    }
+}
+
 // EE candidates with every pair found once: the set query_template2 / fn_query_from_edges_v2 produce
-// ({(a, b): a < b, query box of a overlaps leaf box of b}) when every edge's first vertex has thickness 0
-// and the same d_hat r.  The query of the leaf at sorted position i visits only slots whose largest
-// sorted position (`last`) exceeds i, so each pair of leaves is met from the lower position alone, with a
-// culling box a few ulps wider than the query box; at a leaf the reference's own test decides, in the
-// reference's direction: for q < e the query box of q against the leaf box of e, for e < q the query box
-// of e (e's leaf box widened by r, exact since its thickness is 0) against the leaf box of q (q's own box).
-// Pairs are written (smaller id, larger id) as the reference writes them.  Leaves of other queries are
-// pruned by position, not by id, so a traversal visits about half the nodes of k_query<true>.
+// ({(a, b): a < b, query box of a overlaps leaf box of b}).  The query of the leaf at sorted position i visits only
+// slots whose largest sorted position (`last`) exceeds i, so each pair of leaves is met from the lower position alone,
+// with a culling box a few ulps wider than the query box needs; at a leaf the reference's own test decides, in the
+// reference's direction: for q < e the query box of q against the leaf box of e, for e < q the query box of e against
+// the leaf box of q.  Pairs are written (smaller id, larger id) as the reference writes them.  Leaves of other queries
+// are pruned by position, not by id, so a traversal visits about half the nodes of k_query<true>.
+// PerEdge = false: every edge's first vertex has thickness 0 and the same d_hat r, so that e's query box is its leaf box
+// widened by r and q's leaf box is q's own.  PerEdge = true: per-vertex thickness and d_hat on the tree's own leaves
+// (k_sym_check); e's query box is formed from its vertices, and the culling box holds the largest d_hat.
+// A warp walks the union of its 32 queries' paths -- they are neighbours in the tree's own order -- with one stack of
+// {node, the lanes it overlaps} in shared memory: a record is then one broadcast line for the warp instead of up to 32
+// scattered ones, no lane waits for another's longer walk, and the pairs leave in runs.  Each lane still counts its own
+// steps.
+// Static and swept queries of two sheets of 448 x 448 vertices with a thickness: 12.9 ms as k_query_ref, 8.6 ms so; of
+// 212 x 212 vertices of thickness 0: 2.3 and 1.3 ms.
+template <bool PerEdge>
 __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__ wide4, const uint32_t* __restrict__ sgo,
                                                       uint32_t n_leaves, const float4* __restrict__ x0,
                                                       const float4* __restrict__ x1, const uint2* __restrict__ edges,
-                                                      float r, uint2* __restrict__ pairs, uint32_t capacity,
-                                                      uint32_t* d_count, uint32_t* capped,
-                                                      const uint32_t* __restrict__ maxdepth)
+                                                      float uniform_r, const float* __restrict__ dhat,
+                                                      const float* __restrict__ thickness,
+                                                      const uint32_t* __restrict__ sym_info, uint2* __restrict__ pairs,
+                                                      uint32_t capacity, uint32_t* d_count, uint32_t* capped,
+                                                      const Early early)
 {
-    if (__ldg(maxdepth) >= kRefStack) return;  // a deep tree: k_query_ref<true> (the full EE walk) instead
+    __shared__ uint2 s_stack[4][kPacketStack];
+    __shared__ uint2 s_pairs[4][kPacketPairs];
+    if (early()) return;  // k_query_ref<true> (the full EE walk) instead
+    if (PerEdge && sym_info[0] != 0u) return;       // k_query<true> instead
+    const float d_max = PerEdge ? from_ordered(sym_info[1]) : 0.0f;
+    const float r_max = PerEdge ? fabsf(from_ordered(sym_info[2])) : 0.0f;
+    const uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
+    uint2* stack = s_stack[threadIdx.x >> 5];
+    uint2* buf = s_pairs[threadIdx.x >> 5];
+    const uint32_t n_round = (n_leaves + 31u) & ~31u;  // whole warps stay in the walk
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_round; t += gridDim.x * blockDim.x) {
+        const bool on = t < n_leaves;
+        const uint32_t q = __ldg(&sgo[on ? t : n_leaves - 1]);
+        const uint2 ed = __ldg(&edges[q]);
+        const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
+        const v3 mn = min3(min3(s0, s1), min3(e0, e1)), mx = max3(max3(s0, s1), max3(e0, e1));
+        const float th = PerEdge ? __ldg(&thickness[ed.x]) : 0.0f;
+        const float r = PerEdge ? th + __ldg(&dhat[ed.x]) : uniform_r;
+        const float4 own_mn = make_float4(PerEdge ? mn.x - th : mn.x, PerEdge ? mn.y - th : mn.y, PerEdge ? mn.z - th : mn.z, 0.f);
+        const float4 own_mx = make_float4(PerEdge ? mx.x + th : mx.x, PerEdge ? mx.y + th : mx.y, PerEdge ? mx.z + th : mx.z, 0.f);
+        const float box[6] = {mn.x - r, mn.y - r, mn.z - r, mx.x + r, mx.y + r, mx.z + r};
+        float cull[6];
+        {
+            const float rc = PerEdge ? fmaxf(r, th + d_max) : r;
+            const float rm = PerEdge ? fabsf(rc) + r_max + fabsf(th) + fabsf(d_max) : r;
+            const float mgx = (fabsf(mn.x) + fabsf(mx.x) + rm) * 9.5367431640625e-07f;  // 2^-20
+            const float mgy = (fabsf(mn.y) + fabsf(mx.y) + rm) * 9.5367431640625e-07f;
+            const float mgz = (fabsf(mn.z) + fabsf(mx.z) + rm) * 9.5367431640625e-07f;
+            cull[0] = mn.x - rc - mgx; cull[1] = mn.y - rc - mgy; cull[2] = mn.z - rc - mgz;
+            cull[3] = mx.x + rc + mgx; cull[4] = mx.y + rc + mgy; cull[5] = mx.z + rc + mgz;
+        }
+        uint32_t steps = 0, held = 0;
+        bool dead = false;
+        auto flush = [&]() {
+            __syncwarp();
+            uint32_t base = 0;
+            if (lane == 0 && held) base = atomicAdd(d_count, held);
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            for (uint32_t k = lane; k < held; k += 32)
+                if (base + k < capacity) pairs[base + k] = buf[k];
+            held = 0;
+            __syncwarp();
+        };
+        int sp = 1;
+        {
+            const uint32_t all = __ballot_sync(0xFFFFFFFFu, on);
+            if (lane == 0) stack[0] = make_uint2(0u, all);
+        }
+        while (sp > 0) {
+            __syncwarp();
+            const uint2 top = stack[--sp];
+            __syncwarp();  // read by every lane before lane 0 pushes over it
+            const bool act = ((top.y >> lane) & 1u) && !dead;
+            const float4* node_rec = wide4 + 8 * (size_t)top.x;
+            float4 rec[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ld_slot(node_rec + 2 * j, rec[2 * j], rec[2 * j + 1]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 cmn = rec[2 * k], cmx = rec[2 * k + 1];
+                const bool ov = act && !dead && __float_as_uint(cmx.w) > t && overlap(cmn, cmx, cull);
+                const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, ov);
+                if (lanes == 0) continue;
+                const uint32_t code = __float_as_uint(cmn.w);
+                if (code & 0x80000000u) {
+                    const uint32_t e = code & 0x7FFFFFFFu;
+                    v3 en = mk3(cmn.x, cmn.y, cmn.z), ex = mk3(cmx.x, cmx.y, cmx.z);
+                    float re = r;
+                    if (PerEdge) {  // e's own query box, the same for every lane
+                        const uint2 ee = __ldg(&edges[e]);
+                        const v3 a0 = ld3(x0, ee.x), a1 = ld3(x0, ee.y), b0 = ld3(x1, ee.x), b1 = ld3(x1, ee.y);
+                        en = min3(min3(a0, a1), min3(b0, b1));
+                        ex = max3(max3(a0, a1), max3(b0, b1));
+                        re = __ldg(&thickness[ee.x]) + __ldg(&dhat[ee.x]);
+                    }
+                    const float qe[6] = {en.x - re, en.y - re, en.z - re, ex.x + re, ex.y + re, ex.z + re};
+                    const bool hit = ov && (q < e ? overlap(cmn, cmx, box) : overlap(own_mn, own_mx, qe));
+                    const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+                    if (hit) buf[held + __popc(hits & lt)] = q < e ? make_uint2(q, e) : make_uint2(e, q);
+                    held += __popc(hits);
+                } else if (sp < kPacketStack) {
+                    if (lane == 0) stack[sp] = make_uint2(code, lanes);
+                    ++sp;
+                } else if (ov) {
+                    dead = true;
+                    if (capped) atomicOr(capped, 1u);
+                }
+            }
+            if (act && !dead && ++steps > 100000u) {
+                dead = true;
+                if (capped) atomicOr(capped, 1u);
+            }
+            if (held > kPacketPairs - 128) flush();  // a record adds at most 4 pairs per lane
+        }
+        flush();
+    }
+}
+
+// The same walk, one query per thread, for trees that leave most of the GPU's warps idle: a warp's union of paths is
+// longer than its longest path, which is what the time is there.
+template <bool PerEdge>
+__global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restrict__ wide4, const uint32_t* __restrict__ sgo,
+                                                      uint32_t n_leaves, const float4* __restrict__ x0,
+                                                      const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                      float uniform_r, const float* __restrict__ dhat,
+                                                      const float* __restrict__ thickness,
+                                                      const uint32_t* __restrict__ sym_info, uint2* __restrict__ pairs,
+                                                      uint32_t capacity, uint32_t* d_count, uint32_t* capped,
+                                                      const Early early)
+{
+    if (early()) return;  // k_query_ref<true> (the full EE walk) instead
+    if (PerEdge && sym_info[0] != 0u) return;       // k_query<true> instead
+    const float d_max = PerEdge ? from_ordered(sym_info[1]) : 0.0f;
+    const float r_max = PerEdge ? fabsf(from_ordered(sym_info[2])) : 0.0f;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_leaves; t += gridDim.x * blockDim.x) {
         const uint32_t q = __ldg(&sgo[t]);
         const uint2 ed = __ldg(&edges[q]);
         const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
         const v3 mn = min3(min3(s0, s1), min3(e0, e1)), mx = max3(max3(s0, s1), max3(e0, e1));
-        const float4 own_mn = make_float4(mn.x, mn.y, mn.z, 0.f), own_mx = make_float4(mx.x, mx.y, mx.z, 0.f);
+        const float th = PerEdge ? __ldg(&thickness[ed.x]) : 0.0f;
+        const float r = PerEdge ? th + __ldg(&dhat[ed.x]) : uniform_r;
+        const float4 own_mn = make_float4(PerEdge ? mn.x - th : mn.x, PerEdge ? mn.y - th : mn.y, PerEdge ? mn.z - th : mn.z, 0.f);
+        const float4 own_mx = make_float4(PerEdge ? mx.x + th : mx.x, PerEdge ? mx.y + th : mx.y, PerEdge ? mx.z + th : mx.z, 0.f);
         const float box[6] = {mn.x - r, mn.y - r, mn.z - r, mx.x + r, mx.y + r, mx.z + r};
         float cull[6];
         {
-            const float mgx = (fabsf(mn.x) + fabsf(mx.x) + r) * 9.5367431640625e-07f;  // 2^-20
-            const float mgy = (fabsf(mn.y) + fabsf(mx.y) + r) * 9.5367431640625e-07f;
-            const float mgz = (fabsf(mn.z) + fabsf(mx.z) + r) * 9.5367431640625e-07f;
-            cull[0] = box[0] - mgx; cull[1] = box[1] - mgy; cull[2] = box[2] - mgz;
-            cull[3] = box[3] + mgx; cull[4] = box[4] + mgy; cull[5] = box[5] + mgz;
+            const float rc = PerEdge ? fmaxf(r, th + d_max) : r;
+            const float rm = PerEdge ? fabsf(rc) + r_max + fabsf(th) + fabsf(d_max) : r;
+            const float mgx = (fabsf(mn.x) + fabsf(mx.x) + rm) * 9.5367431640625e-07f;  // 2^-20
+            const float mgy = (fabsf(mn.y) + fabsf(mx.y) + rm) * 9.5367431640625e-07f;
+            const float mgz = (fabsf(mn.z) + fabsf(mx.z) + rm) * 9.5367431640625e-07f;
+            cull[0] = mn.x - rc - mgx; cull[1] = mn.y - rc - mgy; cull[2] = mn.z - rc - mgz;
+            cull[3] = mx.x + rc + mgx; cull[4] = mx.y + rc + mgy; cull[5] = mx.z + rc + mgz;
         }
         uint32_t stack[kStack4];
         int sp = 0;
@@ -849,7 +1124,16 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
                         if (q < e) {
                             if (overlap(cmn, cmx, box)) hit[nhit++] = make_uint2(q, e);
                         } else {
-                            const float qe[6] = {cmn.x - r, cmn.y - r, cmn.z - r, cmx.x + r, cmx.y + r, cmx.z + r};
+                            v3 en = mk3(cmn.x, cmn.y, cmn.z), ex = mk3(cmx.x, cmx.y, cmx.z);
+                            float re = r;
+                            if (PerEdge) {
+                                const uint2 ee = __ldg(&edges[e]);
+                                const v3 a0 = ld3(x0, ee.x), a1 = ld3(x0, ee.y), b0 = ld3(x1, ee.x), b1 = ld3(x1, ee.y);
+                                en = min3(min3(a0, a1), min3(b0, b1));
+                                ex = max3(max3(a0, a1), max3(b0, b1));
+                                re = __ldg(&thickness[ee.x]) + __ldg(&dhat[ee.x]);
+                            }
+                            const float qe[6] = {en.x - re, en.y - re, en.z - re, ex.x + re, ex.y + re, ex.z + re};
                             if (overlap(own_mn, own_mx, qe)) hit[nhit++] = make_uint2(e, q);
                         }
                     } else if (sp < kStack4) {
@@ -1000,8 +1284,12 @@ extern "C" int lcs_bvh_create(int kind, uint32_t n_leaves, lcs_bvh** out)
     A(alloc(h->seg_box, 2 * chunks * kRefitSegs));
     A(alloc(h->chunk_box, 2 * chunks));
     A(alloc(h->healthy, 1));
-    A(alloc(h->maxdepth, 1));
-    if (e == cudaSuccess) e = cudaMemset(h->maxdepth, 0, sizeof(uint32_t));
+    A(alloc(h->turns, 2 + kMaxTops));
+    A(alloc(h->top_lefts, 32 * kMaxTops));
+    A(alloc(h->early, kSymSlots));
+    if (kind == LCS_TREE_EDGE) A(alloc(h->sym_info, 4 * kSymSlots));
+    if (e == cudaSuccess) e = cudaMemset(h->turns, 0, 2 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(h->early, 0, kSymSlots * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(h->span_count, 0, sizeof(uint32_t));
     const uint32_t np1 = n_leaves + 1;
     if (e == cudaSuccess) e = cudaMemcpy(h->n_plus_1, &np1, sizeof(uint32_t), cudaMemcpyHostToDevice);
@@ -1025,7 +1313,8 @@ extern "C" int lcs_bvh_destroy(lcs_bvh* h)
     void* ptrs[] = {h->centers, h->block_aabb, h->gaabb, h->m30, h->keys, h->keys_alt, h->vals, h->vals_alt,
                     h->hist, h->ms64, h->parent, h->children, h->slot, h->wide, h->wide4, h->even, h->range,
                     h->swap_diff, h->swap_cov, h->scan_tmp, h->n_plus_1, h->leaf_at, h->node_at,
-                    h->order_range, h->spans, h->span_count, h->seg_box, h->chunk_box, h->healthy, h->maxdepth};
+                    h->order_range, h->spans, h->span_count, h->seg_box, h->chunk_box, h->healthy, h->turns, h->top_lefts, h->early,
+                    h->sym_info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete h;
@@ -1085,11 +1374,11 @@ extern "C" int lcs_bvh_construct(lcs_bvh* h, lcs_stream stream)
         const int gi = grid_for(h->ni, 256);
         LCS_CUDA_TRY(cudaMemsetAsync(h->swap_diff, 0, sizeof(uint32_t) * ((size_t)h->n + 1), s));
         k_build_inner<<<gi, 256, 0, s>>>(h->ms64, h->sgo, h->n, h->parent, h->children, h->slot, h->wide,
-                                         h->maxdepth, h->range, h->swap_diff);
+                                         h->turns, h->range, h->swap_diff);
         lcs_count_launch();
         k_check<<<gi, 256, 0, s>>>(h->children, h->parent, h->ni, h->healthy);
         lcs_count_launch();
-        k_depth_parity<<<gi, 256, 0, s>>>(h->parent, h->ni, h->even, h->maxdepth);
+        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->turns, h->top_lefts);
         lcs_count_launch();
         LCS_CUDA_TRY(union_order(h, s));
     } else {
@@ -1128,11 +1417,11 @@ int lcs_bvh_construct_host_sort(lcs_bvh* h, lcs_stream stream)
         const int gi = grid_for(h->ni, 256);
         LCS_CUDA_TRY(cudaMemsetAsync(h->swap_diff, 0, sizeof(uint32_t) * ((size_t)h->n + 1), s));
         k_build_inner<<<gi, 256, 0, s>>>(h->ms64, h->sgo, h->n, h->parent, h->children, h->slot, h->wide,
-                                         h->maxdepth, h->range, h->swap_diff);
+                                         h->turns, h->range, h->swap_diff);
         lcs_count_launch();
         k_check<<<gi, 256, 0, s>>>(h->children, h->parent, h->ni, h->healthy);
         lcs_count_launch();
-        k_depth_parity<<<gi, 256, 0, s>>>(h->parent, h->ni, h->even, h->maxdepth);
+        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->turns, h->top_lefts);
         lcs_count_launch();
         LCS_CUDA_TRY(union_order(h, s));
     }
@@ -1198,6 +1487,24 @@ extern "C" int lcs_bvh_update_refit(lcs_bvh* h, const float* thickness, const fl
     return leaves_refit(h, thickness, x0, x1, elems, 1, 1, stream);
 }
 
+// k_may_end of a call, and its answer
+template <bool EE>
+static Early ask_early(const lcs_bvh* t, const float* x0, const float* x1, const uint32_t* edges, uint32_t n, const float* dhat,
+                       const float* thickness, float uniform_r, const uint32_t* order, cudaStream_t s)
+{
+    uint32_t call = __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);
+    if (call == 0) call = __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);  // 0 marks nothing
+    uint32_t* flag = t->early + call % kSymSlots;
+    if (t->ni > 0) {
+        k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, reinterpret_cast<const float4*>(x0),
+                                                      reinterpret_cast<const float4*>(x1),
+                                                      reinterpret_cast<const uint2*>(edges), n, dhat, thickness, uniform_r,
+                                                      order, call, flag);
+        lcs_count_launch();
+    }
+    return Early{t->turns, flag, call};
+}
+
 extern "C" int lcs_bvh_query_vf(const lcs_bvh* t, const float* x0, const float* x1, uint32_t n_verts,
                                 const float* d_hat, const float* thickness, uint32_t* pairs, uint32_t capacity,
                                 uint32_t* d_count, lcs_stream stream)
@@ -1213,14 +1520,15 @@ int lcs_bvh_query_vf_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: bad argument (needs a face tree)");
     if (t->n == 0 || n_verts == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: the tree has not been constructed");
+    const Early early = ask_early<false>(t, x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr, (cudaStream_t)stream);
     k_query<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts,
-        d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity, d_count, nullptr, capped, t->maxdepth);
+        d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity, d_count, nullptr, capped, early, nullptr);
     lcs_count_launch();
     if (t->ni > 0) {
         k_query_ref<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
             t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts, d_hat,
-            thickness, 0.0f, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, t->maxdepth);
+            thickness, 0.0f, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
         lcs_count_launch();
     }
     LCS_LAUNCH_CHECK();
@@ -1244,16 +1552,35 @@ int lcs_bvh_query_ee_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee: bad argument (needs an edge tree)");
     if (t->n == 0 || n_edges == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee: the tree has not been constructed");
+    const Early early = ask_early<true>(t, x0, x1, edges, n_edges, d_hat, thickness, 0.0f,
+                                        n_edges == t->n ? t->sgo : nullptr, (cudaStream_t)stream);
+    // The tree's own edges in earnest numbers: once per pair, if the device finds the leaf boxes to be those of the
+    // arguments (the check and its two extra launches cost 8 us; below 8,192 edges that is what the walk would save).
+    const uint32_t* info = nullptr;
+    if (n_edges == t->n && n_edges >= 8192) {
+        uint32_t* slot = t->sym_info + 4 * (early.call % kSymSlots);
+        const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
+        const uint2* e2 = reinterpret_cast<const uint2*>(edges);
+        cudaStream_t s = (cudaStream_t)stream;
+        LCS_CUDA_TRY(cudaMemsetAsync(slot, 0, 16, s));
+        k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat, thickness, slot);
+        lcs_count_launch();
+        const auto walk = t->n >= kPacketLeaves ? k_query_ee_sym<true> : k_query_ee_sym_lane<true>;
+        walk<<<grid_for(n_edges, 128, 16), 128, 0, s>>>(t->wide4, t->sgo, t->n, p0, p1, e2, 0.0f, d_hat, thickness, slot,
+                                                        reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
+        lcs_count_launch();
+        info = slot;
+    }
     k_query<true><<<grid_for(n_edges, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
         reinterpret_cast<const uint2*>(edges), n_edges, d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity,
-        d_count, n_edges == t->n ? t->sgo : nullptr, capped, t->maxdepth);
+        d_count, n_edges == t->n ? t->sgo : nullptr, capped, early, info);
     lcs_count_launch();
     if (t->ni > 0) {
         k_query_ref<true><<<grid_for(n_edges, 128, 16), 128, 0, (cudaStream_t)stream>>>(
             t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
             reinterpret_cast<const uint2*>(edges), n_edges, d_hat, thickness, 0.0f, reinterpret_cast<uint2*>(pairs),
-            capacity, d_count, capped, t->maxdepth);
+            capacity, d_count, capped, early);
         lcs_count_launch();
     }
     LCS_LAUNCH_CHECK();
@@ -1276,16 +1603,18 @@ int lcs_bvh_query_ee_sym_capped(const lcs_bvh* t, const float* x0, const float* 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: bad argument (needs an edge tree, d_hat >= 0)");
     if (t->n == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: the tree has not been constructed");
-    k_query_ee_sym<<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
+    const Early early = ask_early<true>(t, x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo, (cudaStream_t)stream);
+    const auto walk = t->n >= kPacketLeaves ? k_query_ee_sym<false> : k_query_ee_sym_lane<false>;
+    walk<<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-        reinterpret_cast<const uint2*>(edges), d_hat, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped,
-        t->maxdepth);
+        reinterpret_cast<const uint2*>(edges), d_hat, nullptr, nullptr, nullptr, reinterpret_cast<uint2*>(pairs), capacity,
+        d_count, capped, early);
     lcs_count_launch();
-    if (t->ni > 0) {  // a deep tree: the reference's full EE walk (its early exits break the symmetry)
+    if (t->ni > 0) {  // a call in which the stack may fill: the reference's full EE walk (its early exits break the symmetry)
         k_query_ref<true><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
             t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
             reinterpret_cast<const uint2*>(edges), t->n, nullptr, nullptr, d_hat, reinterpret_cast<uint2*>(pairs),
-            capacity, d_count, capped, t->maxdepth);
+            capacity, d_count, capped, early);
         lcs_count_launch();
     }
     LCS_LAUNCH_CHECK();

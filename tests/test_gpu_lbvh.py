@@ -400,3 +400,67 @@ def test_deep_tree_once_per_pair_query_falls_back_to_the_reference_walk():
         n = int(counts(cnt)[0])
         assert n == n_want, (rad, n, n_want)
         np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n]), SC.sorted_pairs(want))
+
+
+@pytest.mark.parametrize("side,swept,foreign", [(40, False, False), (53, False, False), (53, True, False), (60, True, True),
+                                                (150, True, False)])
+def test_general_ee_query_once_per_pair_and_its_fallback(side, swept, foreign):
+    """The general EE query around the 8,192 edges from which it meets each pair once (side 53 has 8,216), with per-vertex
+    thickness and d_hat, and at the 65,536 from which a warp walks for 32 queries (side 150 has 66,901); `foreign` queries with other positions than the tree's, which the full walk has to answer."""
+    i = np.arange(side)
+    X, Z = np.meshgrid(i, i, indexing="ij")
+    v = X * side + Z
+    pair = lambda a, b: np.stack([a.ravel(), b.ravel()], 1)  # noqa: E731
+    el = np.concatenate([pair(v[:-1], v[1:]), pair(v[:, :-1], v[:, 1:]), pair(v[:-1, :-1], v[1:, 1:])]).astype(np.uint32)
+    rng = np.random.default_rng(side)
+    n = side * side
+    x = np.zeros((n, 4), np.float32)
+    x[:, 0], x[:, 2] = X.ravel() * 0.01, Z.ravel() * 0.01
+    x[:, 1] = 2e-3 * rng.random(n)
+    x1 = x + (rng.normal(0, 3e-3, x.shape).astype(np.float32) if swept else 0)
+    th = rng.uniform(0, 2e-3, n).astype(np.float32)
+    dh = rng.uniform(1e-4, 3e-3, n).astype(np.float32)
+    t_o = O.lbvh_build(O.TREE_EDGE, x, el, n)
+    O.lbvh_refit(t_o, x, x1, el, th)
+    bvh = LBVH(O.TREE_EDGE, el.shape[0])
+    xd, x1d, ed = dev(x), dev(x1), dev(el)
+    bvh.reduce_edge_tree_aabb(xd, ed)
+    bvh.construct_tree()
+    bvh.update_and_refit(dev(th), xd, x1d, ed)
+    qx = x1 if foreign else x
+    want, n_want = O.lbvh_query_ee(t_o, qx, x1, el, dh, th)
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pairs = torch.zeros((n_want + 64, 2), dtype=torch.int32, device="cuda")
+    bvh.broad_phase_query_from_edges(dev(qx), x1d, ed, cnt, pairs, dev(dh), dev(th))
+    assert int(counts(cnt)[0]) == n_want > 0
+    np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
+
+
+@pytest.mark.parametrize("kind_name", ["face", "edge"])
+@pytest.mark.parametrize("rad", [0.1, 300.0, 800.0])
+def test_deep_tree_without_pending_nodes(kind_name, rad):
+    """The deep tree mirrored: its longest path turns left throughout, so that the reference's stack never fills, at any
+    radius, and the 4-wide walks serve a tree of more than 32 levels."""
+    x, el = SC.deep_tree_elements(kind_name)
+    x[:, :3] = np.float32(1024.0) - x[:, :3]
+    V = x.shape[0]
+    ee = kind_name == "edge"
+    t_o = O.lbvh_build(KINDS[kind_name][0], x, el, V)
+    z = np.zeros(V, np.float32)
+    O.lbvh_refit(t_o, x, x, el, z)
+    bvh = LBVH(KINDS[kind_name][0], el.shape[0])
+    xd, ed = dev(x), dev(el)
+    (bvh.reduce_edge_tree_aabb if ee else bvh.reduce_face_tree_aabb)(xd, ed)
+    bvh.construct_tree()
+    bvh.update_and_refit(dev(z), xd, xd, ed)
+    r = np.full(V, rad, np.float32)
+    want, n_want = (O.lbvh_query_ee(t_o, x, x, el, r, z) if ee else O.lbvh_query_vf(t_o, x, x, r, z))
+    assert n_want == _brute_force_count(x, el, r, ee)  # no early exit
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pairs = torch.zeros((n_want + 64, 2), dtype=torch.int32, device="cuda")
+    if ee:
+        bvh.broad_phase_query_from_edges_sym(xd, xd, ed, cnt, pairs, rad)
+    else:
+        bvh.broad_phase_query_from_verts(xd, xd, cnt, pairs, dev(r), dev(z))
+    assert int(counts(cnt)[0]) == n_want
+    np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
