@@ -1,11 +1,11 @@
 // row_stage.cuh -- products of 32-row slices of a 3x3-block CSR matrix, one warp per slice.
 //
 // Four lanes share a row (lane g of four takes blocks rp + g, rp + g + 4, ...), which read straight from global
-// memory costs nine 4-byte loads at a 36-byte stride: every load of a warp touches 8 to 16 cache lines for 128 bytes,
-// and the L1's tag rate, not HBM, bounds the product.  So the blocks of 8 consecutive rows -- one contiguous run of
-// the CSR -- are brought into shared memory by bulk copies (two stages per warp, the next run in flight while one is
-// multiplied); there the 9-word stride of the blocks is free of bank conflicts.  Measured figures stand at the
-// kernels that use it.
+// memory costs nine 4-byte loads at a 36-byte stride.  With 2,048 threads per SM those loads hide each other's latency
+// (k_spmv); a cluster that owns a scene has 256 to 512 threads per SM and waits for them.  So the blocks of 8
+// consecutive rows -- one contiguous run of the CSR -- are brought into shared memory by bulk copies (two stages per
+// warp, the next run in flight while one is multiplied); there the 9-word stride of the blocks is free of bank
+// conflicts.  Measured figures stand at the kernels that use it.
 #pragma once
 #include <cstdint>
 
