@@ -365,6 +365,12 @@ LCS_API const lcs_pcg_stats* lcs_pcg_device_stats(const lcs_pcg* p);
  * the context stays usable. */
 LCS_API int lcs_debug_pcg_wait(int32_t which, int32_t missing_block, uint32_t blocks, uint32_t spin_limit,
                                lcs_stream stream);
+/* The same for the batched solve's copies of the matrix to shared memory: y = A x (off-diagonal blocks; x, y: 4 floats a
+ * row) by one warp through those copies.  omit_copy != 0: the first copy's barrier waits for 16 bytes that nothing sends
+ * and gives up after poll_limit polls (1..2^20; the solves use 2^20) of at most a microsecond; the warp then reads the
+ * blocks directly, so that y is right all the same, and the call returns LCS_ERR_TIMEOUT. */
+LCS_API int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* y, int32_t omit_copy, uint32_t poll_limit,
+                                    lcs_stream stream);
 
 /* Allocation-free variant of lcs_pcg_solve (fused solve only); it has no counterpart in the
  * reference.  For callers that cannot allocate device memory while they run: cudaMalloc and

@@ -2189,7 +2189,32 @@ __global__ void __launch_bounds__(32 * W, !Staged ? 4 : W > 8 ? 1 : 2) k_pcg_bat
         a.stats[s] = out;
     }
     cluster_sync_all();  // a copy that never came in any CTA outlives rank 0's verdict
+    st.drain();
     if (st.failed && lane == 0) a.stats[s].status = LCS_ERR_TIMEOUT;
+}
+
+// Test hook of the staged copies (lcs_debug_pcg_copy_wait): one warp forms A x slice by slice as k_pcg_batch does.  With
+// `omit` the first copy's barrier also expects 16 bytes that nothing sends, so that the wait for it runs out.
+__global__ void __launch_bounds__(32) k_copy_wait_probe(Bsr A, uint32_t n, const float4* x, float4* y, int omit, uint32_t limit,
+                                                        lcs_pcg_stats* stats)
+{
+    extern __shared__ __align__(128) unsigned char s_stage[];
+    __shared__ __align__(8) uint64_t s_bar[2];
+    stage::Warp st;
+    st.init(s_stage, s_bar, stage::Csr{A.rp, A.col, A.val}, stage::Csr{nullptr, nullptr, nullptr}, n);
+    st.limit = limit;
+    if (omit && lane_id() == 0) stage::bar_expect_more(&s_bar[0], 16);
+    __syncwarp();
+    stage::Slice cur, next;
+    cur.load(st, 0, n);
+    for (uint32_t base = 0; base < n; base += 32) {
+        next.load(st, base + 32, n);
+        const float3 v = stage::slice_product<true>(st, cur, next, [&](uint32_t c) { return x[c]; });
+        cur = next;
+        if (base + lane_id() < n) y[base + lane_id()] = make_float4(v.x, v.y, v.z, 0.0f);
+    }
+    st.drain();
+    if (st.failed && lane_id() == 0) stats->status = LCS_ERR_TIMEOUT;
 }
 
 }  // namespace
@@ -2278,6 +2303,33 @@ extern "C" int lcs_debug_pcg_wait(int32_t which, int32_t missing_block, uint32_t
     if (rc != LCS_OK) return lcs_fail(rc, cudaGetErrorString(err));
     if (h.status == LCS_ERR_TIMEOUT)
         return lcs_fail(LCS_ERR_TIMEOUT, "lcs_debug_pcg_wait: a bounded wait ran out (LCS_ERR_TIMEOUT)");
+    return h.status;
+}
+
+extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* y, int32_t omit_copy, uint32_t poll_limit,
+                                       lcs_stream stream)
+{
+    if (!A || !A->row_ptr || !A->col || !A->val || A->n_rows == 0 || !x || !y)
+        return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_copy_wait: bad argument");
+    if (poll_limit == 0 || poll_limit > stage::kWaitLimit)
+        return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_copy_wait: poll_limit must be in [1, 2^20]");
+    cudaStream_t s = (cudaStream_t)stream;
+    lcs_pcg_stats* st = nullptr;
+    lcs_pcg_stats h{};
+    LCS_CUDA_TRY(cudaMalloc(&st, sizeof(h)));
+    cudaError_t e = cudaMemsetAsync(st, 0, sizeof(h), s);
+    if (e == cudaSuccess) {
+        k_copy_wait_probe<<<1, 32, stage::kWarpBytes, s>>>(Bsr{A->row_ptr, A->col, A->val}, A->n_rows, reinterpret_cast<const float4*>(x),
+                                                           reinterpret_cast<float4*>(y), omit_copy, poll_limit, st);
+        e = cudaGetLastError();
+        lcs_count_launch();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFree(st);
+    LCS_CUDA_TRY(e);
+    if (h.status == LCS_ERR_TIMEOUT)
+        return lcs_fail(LCS_ERR_TIMEOUT, "lcs_debug_pcg_copy_wait: a bounded wait ran out (LCS_ERR_TIMEOUT)");
     return h.status;
 }
 

@@ -22,7 +22,8 @@ constexpr uint32_t kColBytes = kWin * 4 + 16;
 constexpr uint32_t kStageBytes = kValBytes + kColBytes;
 constexpr uint32_t kWarpBytes = 2 * kStageBytes;
 static_assert(kValBytes % 16 == 0 && kColBytes % 16 == 0, "bulk copies are 16-byte aligned");
-constexpr uint32_t kWaitLimit = 1u << 22;  // polls of a copy's barrier (each suspends in hardware for a while)
+constexpr uint32_t kPollNs = 1000;         // a poll of a copy's barrier suspends for at most this long
+constexpr uint32_t kWaitLimit = 1u << 20;  // polls before a warp gives up on a copy: about a second
 
 struct Csr {
     const uint32_t* rp;
@@ -42,11 +43,17 @@ __device__ __forceinline__ void bar_expect(uint64_t* bar, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
+// the barrier's phase waits for `bytes` more than the copies bring
+__device__ __forceinline__ void bar_expect_more(uint64_t* bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(kPollNs) : "memory");
     return ok != 0;
 }
 
@@ -70,9 +77,10 @@ struct Warp {
     uint64_t* bar;        // two barriers (null: nothing is staged)
     Csr A, B;
     uint32_t nnz;         // blocks of A (the copies never read past them)
-    bool bulk;            // A's arrays are 16-byte aligned; else the blocks are read directly
+    bool bulk;            // A's arrays are 16-byte aligned and no copy has failed; else the blocks are read directly
     uint32_t use = 0;     // copies consumed: stage use & 1, parity (use >> 1) & 1
     uint32_t ahead = 0;   // copies in flight (0 to 2)
+    uint32_t limit = kWaitLimit;
     bool failed = false;  // a copy did not arrive within the limit
 
     __device__ __forceinline__ void init(unsigned char* b, uint64_t* barriers, const Csr& a, const Csr& extra, uint32_t n_rows)
@@ -113,18 +121,30 @@ struct Warp {
         ++ahead;
     }
 
-    __device__ __forceinline__ void wait()
+    // whether the oldest copy in flight has arrived, within the limit
+    __device__ __forceinline__ bool arrived()
     {
         const uint32_t s = use & 1u, parity = (use >> 1) & 1u;
-        if (!failed) {
-            uint32_t it = 0;
-            while (!bar_try(&bar[s], parity))
-                if (++it > kWaitLimit) {
-                    failed = true;
-                    break;
-                }
+        uint32_t it = 0;
+        bool ok;
+        while (!(ok = bar_try(&bar[s], parity)) && ++it < limit) {
         }
-        failed = __any_sync(0xFFFFFFFFu, failed);
+        return __all_sync(0xFFFFFFFFu, ok);
+    }
+
+    // Waits for the oldest copy.  A warp that gives up never looks at a stage again (its words may be anything): it
+    // issues no further copies and reads the blocks directly from there on.
+    __device__ __forceinline__ void wait()
+    {
+        if (arrived()) return;
+        failed = true;
+        bulk = false;
+    }
+
+    // before the end of a warp that gave up: one more bounded wait for each copy it left in flight
+    __device__ __forceinline__ void drain()
+    {
+        for (; ahead > 0; ++use, --ahead) arrived();
     }
 };
 
@@ -210,16 +230,13 @@ __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const
         const uint32_t ge = __shfl_sync(0xFFFFFFFFu, cur.hi, 8 * j + 7);
         const uint32_t rs = __shfl_sync(0xFFFFFFFFu, cur.lo, 8 * j + g), re = __shfl_sync(0xFFFFFFFFu, cur.hi, 8 * j + g);
         uint32_t k = rs + lig;
-        if (!Staged || !w.bulk) {
-            direct_blocks<4>(w.A, k, re, ld, acc);
-            k0 = ge;
-        }
-        while (Staged && k0 < ge) {
+        while (Staged && w.bulk && k0 < ge) {
             const uint32_t nb = min(kWin, ge - k0), k1 = k0 + nb;
             if (w.ahead == 0) w.issue(k0, nb);
             if (k1 < a_last) cur.prefetch(w, k1);
             else next.prefetch(w, next.first());
             w.wait();
+            if (w.failed) break;
             unsigned char* d = w.buf + (w.use & 1u) * kStageBytes;
             float* sv = reinterpret_cast<float*>(d) + ((9u * k0) & 3u);
             uint32_t* sc = reinterpret_cast<uint32_t*>(d + kValBytes) + (k0 & 3u);
@@ -247,6 +264,10 @@ __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const
             ++w.use;
             --w.ahead;
             k0 = k1;
+        }
+        if (!Staged || !w.bulk) {  // k: the lane's next block, also where the copies ended in the middle of the row
+            direct_blocks<4>(w.A, k, re, ld, acc);
+            k0 = ge;
         }
         if (has_b) {
             const uint32_t bs = __shfl_sync(0xFFFFFFFFu, cur.blo, 8 * j + g), be = __shfl_sync(0xFFFFFFFFu, cur.bhi, 8 * j + g);

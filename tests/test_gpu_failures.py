@@ -11,12 +11,12 @@ import pytest
 import torch
 
 from luisacomputesimulator_b200 import _capi as A
-from luisacomputesimulator_b200.collision import LBVH, stream
-from luisacomputesimulator_b200.linear import ConjugateGradientSolver
+from luisacomputesimulator_b200.collision import LBVH, ptr, stream
+from luisacomputesimulator_b200.linear import ConjugateGradientSolver, make_bsr
 from luisacomputesimulator_b200.newton import NewtonSolver
 from oracle import oracle as O
 from tests import scenarios as SC
-from tests.gpu_util import dev
+from tests.gpu_util import dev, host
 from tests.test_gpu_pcg import _dev_bsr, contact_system
 
 pytestmark = pytest.mark.gpu
@@ -143,3 +143,33 @@ def test_wait_probe_rejects_bad_arguments():
     assert A.STATUS[lib.lcs_debug_pcg_wait(0, -1, 64, 16, s)] == "LCS_ERR_INVALID"
     assert A.STATUS[lib.lcs_debug_pcg_wait(0, 9, 8, 16, s)] == "LCS_ERR_INVALID"
     assert A.STATUS[lib.lcs_debug_pcg_wait(0, -1, 8, 0, s)] == "LCS_ERR_INVALID"
+
+
+def test_copies_that_do_not_arrive_run_out_and_leave_the_product_right():
+    """The batched solve's copies of the matrix to shared memory, one of which never completes: the warp gives up after a
+    short poll limit, looks at no stage again (its words could be any column) and reads the blocks directly, so the
+    product is that of the completed copies bit for bit and the call returns LCS_ERR_TIMEOUT."""
+    lib = A.load()
+    n = 97
+    rng = np.random.default_rng(3)
+    rp = np.concatenate([[0], np.cumsum(rng.integers(0, 40, n))]).astype(np.int32)
+    col = rng.integers(0, n, rp[-1]).astype(np.int32)
+    val = rng.normal(size=9 * rp[-1]).astype(np.float32)
+    x = rng.normal(size=(n, 4)).astype(np.float32)
+    keep = [dev(rp), dev(col), dev(val), dev(x)]
+    M = make_bsr(n, *keep[:3])
+    got = {}
+    for omit, limit, want in ((0, 1 << 20, "LCS_OK"), (1, 1 << 12, "LCS_ERR_TIMEOUT"), (0, 1 << 20, "LCS_OK")):
+        y = torch.full((n, 4), 9.0, dtype=torch.float32, device="cuda")
+        rc = lib.lcs_debug_pcg_copy_wait(M, ptr(keep[3]), ptr(y), omit, limit, stream())
+        assert A.STATUS[rc] == want, (omit, rc)
+        got[omit] = host(y)[:, :3]
+    np.testing.assert_array_equal(got[1], got[0])
+    r = np.repeat(np.arange(n), np.diff(rp))
+    t = np.einsum("kcr,kc->kr", val.reshape(-1, 3, 3).astype(np.float64), x[col, :3].astype(np.float64))
+    y64, mag = np.zeros((n, 3)), np.zeros((n, 3))
+    np.add.at(y64, r, t)
+    np.add.at(mag, r, np.einsum("kcr,kc->kr", np.abs(val.reshape(-1, 3, 3).astype(np.float64)), np.abs(x[col, :3])))
+    # each of a lane's up to 10 blocks, the 4 lanes and the 3 columns round once: (10 + 2 + 3) 2^-24 of the magnitudes
+    assert (np.abs(got[1] - y64) <= 15 * 2.0 ** -24 * mag).all()
+    assert A.STATUS[lib.lcs_debug_pcg_copy_wait(M, ptr(keep[3]), ptr(y), 0, 0, stream())] == "LCS_ERR_INVALID"
