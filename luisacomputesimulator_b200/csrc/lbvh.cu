@@ -23,6 +23,7 @@ using namespace lcs;
 
 // query calls on one tree that may be in flight at once with different arguments
 constexpr uint32_t kSymSlots = 1024;
+constexpr uint32_t kSymWords = 8;    // words of a call's slot in sym_info
 constexpr uint32_t kMaxTops = 4096;  // listed tops of the parts of a tree where a walk may end early
 
 struct lcs_bvh {
@@ -60,10 +61,10 @@ struct lcs_bvh {
     float4* seg_box = nullptr;       // 2 per 32 union-order positions (whole refit chunks): {min | 0}{max | 0}
     float4* chunk_box = nullptr;     // 2 per refit chunk: its union
     uint32_t* healthy = nullptr;     // 1
-    uint32_t* turns = nullptr;       // 2 + kMaxTops: see k_depth_parity
+    uint32_t* turns = nullptr;       // 3 + kMaxTops: see k_depth_parity
     uint32_t* top_lefts = nullptr;   // 32 * kMaxTops: slots of the 31 inner left siblings above each listed top
     uint32_t* early = nullptr;       // kSymSlots: number of the query call that may end early, a slot per call in turn
-    uint32_t* sym_info = nullptr;    // kSymSlots x 4: k_sym_check's findings, a slot per query call in turn
+    uint32_t* sym_info = nullptr;    // kSymSlots x kSymWords: k_sym_check's findings, a slot per query call in turn
     mutable uint32_t calls = 0;
     bool built = false;              // a construct has written the topology, slots and refit tables
 };
@@ -174,11 +175,11 @@ static_assert((1u << kRefitLevels) == kRefitSegs, "one sparse-table level per do
 // its left child's range in swap_diff (see k_eorder)
 __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* __restrict__ sgo, uint32_t n,
                               uint32_t* __restrict__ parent, uint2* __restrict__ children,
-                              uint32_t* __restrict__ slot, float4* __restrict__ wide, uint32_t* __restrict__ max_pending,
+                              uint32_t* __restrict__ slot, float4* __restrict__ wide, uint32_t* __restrict__ turns,
                               uint2* __restrict__ range, uint32_t* __restrict__ swap_diff)
 {
     const int ni = (int)n - 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) max_pending[0] = max_pending[1] = 0u;  // raised by k_depth_parity, launched after this
+    if (blockIdx.x == 0 && threadIdx.x == 0) turns[0] = turns[1] = turns[2] = 0u;  // raised by k_depth_parity, launched after this
     for (int nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
         int i = 0, j = ni;
         if (nid != 0) {
@@ -246,7 +247,8 @@ __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* _
 // It also counts, for each inner node, the nodes that a walk of the reference can at most have pending when it pops it:
 // one for every ancestor whose second child the path takes and whose first child is an inner node.  turns: [0] the
 // largest count, [1] how many nodes reach kRefPending by their own turn (every node with as many descends from one of
-// them), [2...] the slots of the first kMaxTops of those, whose 31 inner left siblings top_lefts lists.
+// them), [2] the depth of the deepest inner node, [3...] the slots of the first kMaxTops of those that reach kRefPending,
+// whose 31 inner left siblings top_lefts lists.
 constexpr uint32_t kRefStack = 32;
 constexpr uint32_t kRefPending = kRefStack - 1;
 
@@ -254,7 +256,7 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
                                uint8_t* __restrict__ even, uint32_t* __restrict__ turns,
                                uint32_t* __restrict__ top_lefts)
 {
-    uint32_t most = 0;
+    uint32_t most = 0, deepest = 0;
     for (uint32_t nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
         uint32_t p = nid, d = 0, pending = 0;
         bool own = false;
@@ -269,10 +271,11 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
         }
         even[nid] = (d & 1u) == 0u ? 1 : 0;
         most = pending > most ? pending : most;
+        deepest = d > deepest ? d : deepest;
         if (own && pending == kRefPending) {
             const uint32_t k = atomicAdd(&turns[1], 1u);
             if (k < kMaxTops) {
-                turns[2 + k] = slot[nid];
+                turns[3 + k] = slot[nid];
                 uint32_t i = 0;
                 for (p = nid; p != 0u && i < kRefPending;) {
                     const uint32_t s = slot[p];
@@ -283,7 +286,9 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
         }
     }
     most = __reduce_max_sync(0xFFFFFFFFu, most);
+    deepest = __reduce_max_sync(0xFFFFFFFFu, deepest);
     if (lane_id() == 0 && most) atomicMax(&turns[0], most);
+    if (lane_id() == 0 && deepest) atomicMax(&turns[2], deepest);
 }
 
 // the 4-wide record of inner node b from the binary records (leaf_only: a one-leaf tree, whose two slots
@@ -711,6 +716,144 @@ __device__ __forceinline__ void query_box(const float4* x0, const float4* x1, co
     }
 }
 
+// floats as unsigned integers of the same order
+__device__ __forceinline__ uint32_t ordered(float f)
+{
+    const uint32_t u = __float_as_uint(f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(uint32_t u)
+{
+    return __uint_as_float(u & 0x80000000u ? u & 0x7FFFFFFFu : ~u);
+}
+
+// Whether the once-per-pair walk serves a general EE query, by k_sym_check's findings.  It has to look as far around each
+// edge as the largest d_hat reaches, which is many times as much as most need where one body or vertex stands out.  The
+// line: the largest d_hat exceeds the mean one by a tenth of the query boxes' mean extent (two sheets of 448 x 448
+// vertices: 4.5 ms with equal d_hat, 5.0 at the line, 6.8 at twice that, 5.7 by k_query<true> at any).
+constexpr float kSymSpread = 0.1f;
+__device__ __forceinline__ bool sym_serves(const uint32_t* info, uint32_t n)
+{
+    if (info[0] != 0u) return false;
+    return from_ordered(info[1]) - __uint_as_float(info[3]) / (float)n <= kSymSpread * (__uint_as_float(info[4]) / (float)n);
+}
+
+// an edge as a query of the once-per-pair walks (see k_query_ee_sym)
+struct SymQuery {
+    float r;                // radius of its query box
+    float4 own_mn, own_mx;  // its leaf box
+    float box[6], cull[6];  // its query box; what the walk culls with
+};
+
+template <bool PerEdge>
+__device__ __forceinline__ SymQuery sym_query(const float4* x0, const float4* x1, const uint2* edges, float uniform_r,
+                                              const float* dhat, const float* thickness, float d_max, float r_max, uint32_t q)
+{
+    SymQuery Q;
+    const uint2 ed = __ldg(&edges[q]);
+    const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
+    const v3 mn = min3(min3(s0, s1), min3(e0, e1)), mx = max3(max3(s0, s1), max3(e0, e1));
+    const float th = PerEdge ? __ldg(&thickness[ed.x]) : 0.0f;
+    const float r = PerEdge ? th + __ldg(&dhat[ed.x]) : uniform_r;
+    Q.r = r;
+    Q.own_mn = make_float4(PerEdge ? mn.x - th : mn.x, PerEdge ? mn.y - th : mn.y, PerEdge ? mn.z - th : mn.z, 0.f);
+    Q.own_mx = make_float4(PerEdge ? mx.x + th : mx.x, PerEdge ? mx.y + th : mx.y, PerEdge ? mx.z + th : mx.z, 0.f);
+    Q.box[0] = mn.x - r; Q.box[1] = mn.y - r; Q.box[2] = mn.z - r;
+    Q.box[3] = mx.x + r; Q.box[4] = mx.y + r; Q.box[5] = mx.z + r;
+    const float rc = PerEdge ? fmaxf(r, th + d_max) : r;
+    const float rm = PerEdge ? fabsf(rc) + r_max + fabsf(th) + fabsf(d_max) : r;
+    const float mgx = (fabsf(mn.x) + fabsf(mx.x) + rm) * 9.5367431640625e-07f;  // 2^-20
+    const float mgy = (fabsf(mn.y) + fabsf(mx.y) + rm) * 9.5367431640625e-07f;
+    const float mgz = (fabsf(mn.z) + fabsf(mx.z) + rm) * 9.5367431640625e-07f;
+    Q.cull[0] = mn.x - rc - mgx; Q.cull[1] = mn.y - rc - mgy; Q.cull[2] = mn.z - rc - mgz;
+    Q.cull[3] = mx.x + rc + mgx; Q.cull[4] = mx.y + rc + mgy; Q.cull[5] = mx.z + rc + mgz;
+    return Q;
+}
+
+// the query box of the met edge e, whose leaf box is {cmn, cmx}: that box widened by the one radius, or formed anew
+template <bool PerEdge>
+__device__ __forceinline__ void met_box(const float4* x0, const float4* x1, const uint2* edges, const float* dhat,
+                                        const float* thickness, float uniform_r, uint32_t e, float4 cmn, float4 cmx, float* box)
+{
+    v3 en = mk3(cmn.x, cmn.y, cmn.z), ex = mk3(cmx.x, cmx.y, cmx.z);
+    float re = uniform_r;
+    if (PerEdge) {
+        const uint2 ee = __ldg(&edges[e]);
+        const v3 a0 = ld3(x0, ee.x), a1 = ld3(x0, ee.y), b0 = ld3(x1, ee.x), b1 = ld3(x1, ee.y);
+        en = min3(min3(a0, a1), min3(b0, b1));
+        ex = max3(max3(a0, a1), max3(b0, b1));
+        re = __ldg(&thickness[ee.x]) + __ldg(&dhat[ee.x]);
+    }
+    box[0] = en.x - re; box[1] = en.y - re; box[2] = en.z - re;
+    box[3] = ex.x + re; box[4] = ex.y + re; box[5] = ex.z + re;
+}
+
+constexpr uint32_t kRefNodes = 100000;  // popped nodes after which a walk ends
+
+// Whether a walk of the box pops more than kRefNodes inner nodes: the tree's, less every subtree found apart from the
+// box, until they are no more than that.  Large subtrees are looked at first, so that a box that is small beside the tree
+// is done after some dozens of steps; what is never done is looked at to the leaves (not `exact`: counts as "yes").
+__device__ __forceinline__ bool exceeds(const float4* wide, uint32_t ni, const float* box, bool exact)
+{
+    for (uint32_t small = 16384;; small >>= 3) {  // subtrees of so many inner nodes count whole
+        uint2 stack[64];                          // node, first sorted position under it; a path has at most 62 levels
+        uint32_t left = ni;
+        int sp = 0;
+        stack[sp++] = make_uint2(0u, 0u);
+        while (sp > 0) {
+            const uint2 b = stack[--sp];
+            float4 mn[2], mx[2];
+#pragma unroll
+            for (int side = 0; side < 2; ++side) ld_slot(wide + 4 * (size_t)b.x + 2 * side, mn[side], mx[side]);
+            const uint32_t last[2] = {__float_as_uint(mx[0].w), __float_as_uint(mx[1].w)};
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const uint32_t code = __float_as_uint(mn[side].w);
+                if (code & 0x80000000u) continue;
+                const uint32_t first = last[side ^ 1] < last[side] ? last[side ^ 1] + 1u : b.y, inner = last[side] - first;
+                if (!overlap(mn[side], mx[side], box)) left -= inner;
+                else if (inner > small && sp < 64) stack[sp++] = make_uint2(code, first);
+            }
+            if (left <= kRefNodes) return false;
+        }
+        if (small == 0 || !exact) return true;
+    }
+}
+
+// the union of the warp's boxes
+__device__ __forceinline__ void warp_union(const float* box, float* all)
+{
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        all[c] = box[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(0xFFFFFFFFu, all[c], o);
+            all[c] = c < 3 ? fminf(all[c], v) : fmaxf(all[c], v);
+        }
+    }
+}
+
+// Takes a general EE query off the once-per-pair walk where the largest d_hat could make an edge's walk pop so many nodes
+// that it would end: only the edge's own reach may end it.  A warp asks for the union of its 32 edges, neighbours in the
+// tree's order, and each edge for itself only where that is not enough (1.2 million edges: 0.14 ms).
+__global__ void __launch_bounds__(256) k_may_exceed(const float4* __restrict__ wide, uint32_t ni, const float4* __restrict__ x0, const float4* __restrict__ x1,
+                                                    const uint2* __restrict__ edges, const float* __restrict__ dhat,
+                                                    const float* __restrict__ thickness, const uint32_t* __restrict__ sgo,
+                                                    uint32_t* __restrict__ info)
+{
+    const uint32_t n = ni + 1;
+    if (!sym_serves(info, n)) return;
+    const float d_max = from_ordered(info[1]), r_max = fabsf(from_ordered(info[2]));
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ((n + 31u) & ~31u); t += gridDim.x * blockDim.x) {
+        const SymQuery Q = sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, d_max, r_max, __ldg(&sgo[min(t, n - 1)]));
+        float all[6];
+        warp_union(Q.cull, all);
+        if (exceeds(wide, ni, all, false) && exceeds(wide, ni, Q.cull, true)) atomicOr(&info[0], 1u);
+        __syncwarp();
+    }
+}
+
 // Marks the call if one of its queries overlaps a listed top with so many overlapping inner left siblings above it that,
 // were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's walk
 // reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and a near
@@ -750,7 +893,7 @@ __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide
             uint32_t top = 0;
             bool near = false;
             if (k0 + lane < tops) {
-                top = turns[2 + k0 + lane];
+                top = turns[3 + k0 + lane];
                 float4 mn, mx;
                 ld_slot(wide + 2 * (size_t)top, mn, mx);
                 near = overlap(mn, mx, all);
@@ -794,7 +937,7 @@ __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4,
                                                const uint32_t* __restrict__ sym_info)
 {
     if (early()) return;
-    if (EE && sym_info && sym_info[0] == 0u) return;  // k_query_ee_sym<true> serves the call
+    if (EE && sym_info && sym_serves(sym_info, n_leaves)) return;  // k_query_ee_sym<true> serves the call
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_queries; t += gridDim.x * blockDim.x) {
         // queries in the order of `order` (the tree's Morton order when the queries are its own
         // leaves): neighbouring threads then walk nearly the same nodes
@@ -894,29 +1037,32 @@ constexpr uint32_t kPacketPairs = 256;  // pairs a warp collects before it appen
 // Leaves from which the warp walk is taken: 6,658 vertices (19,900 edges) 52 us a query by the lane walk, 67 by the
 // warp walk; 88,800 vertices (265,800 edges) 447 and 343.
 constexpr uint32_t kPacketLeaves = 65536;
-constexpr int kPacketStack = 128;       // two nodes per turn on paths of at most 62 levels, and a record's four
-
-// floats as unsigned integers of the same order
-__device__ __forceinline__ uint32_t ordered(float f)
-{
-    const uint32_t u = __float_as_uint(f);
-    return u & 0x80000000u ? ~u : u | 0x80000000u;
-}
-__device__ __forceinline__ float from_ordered(uint32_t u)
-{
-    return __uint_as_float(u & 0x80000000u ? u & 0x7FFFFFFFu : ~u);
-}
+constexpr uint32_t kSymEdges = 131072;  // edges from which the general query asks for the once-per-pair walk
+static_assert(kSymEdges >= kPacketLeaves, "the lane walk has no per-edge form");
+// Codes and ids differ within 62 bits, so paths have at most 62 levels, 31 of them 4-wide; each leaves at most three
+// nodes pending and the last adds four: 94.
+constexpr int kSymStack = 96, kPacketStack = 128;
 
 // Whether a general EE query may take the once-per-pair walk: its edges, positions and thicknesses are, bit for bit,
-// those of the tree's leaf boxes.  info (zeroed before): [0] leaves that differ or whose radius is not finite, [1] the
-// largest d_hat, [2] the largest thickness + d_hat (as `ordered`).
+// those of the tree's leaf boxes, and the tree has 32 levels or more.  Codes repeat there, so that boxes of neighbouring
+// subtrees overlap and a warp's queries share many records (two sheets of 448 x 448 vertices: 4.5 ms a call so, 5.7 by
+// k_query<true>); a tube of 134,000 edges, whose tree has fewer levels, takes 0.20 and 0.11 ms.
+// info (zeroed before): [0] leaves that differ or are not finite, [1] the largest d_hat, [2] the largest thickness + d_hat
+// (as `ordered`), [3] the sum of d_hat, [4] of the query boxes' largest extents.
 __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wide, const uint32_t* __restrict__ sgo,
                                                    const uint32_t* __restrict__ slot, uint32_t n,
                                                    const float4* __restrict__ x0, const float4* __restrict__ x1,
                                                    const uint2* __restrict__ edges, const float* __restrict__ dhat,
-                                                   const float* __restrict__ thickness, uint32_t* __restrict__ info)
+                                                   const float* __restrict__ thickness, const uint32_t* __restrict__ turns,
+                                                   uint32_t* __restrict__ info)
 {
+    __shared__ float s_sum[8][2];
+    if (turns[2] < kRefStack) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) info[0] = 1u;
+        return;
+    }
     uint32_t bad = 0, dm = 0, rm = 0;
+    float sum[2] = {0.0f, 0.0f};
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t q = sgo[t], s = slot[n - 1 + t];
         v3 mn, mx;
@@ -925,19 +1071,36 @@ __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wi
         ld_slot(wide + 4 * (size_t)(s >> 1) + 2 * (s & 1u), a, b);
         const uint32_t v0 = __ldg(&edges[q].x);
         const float d = __ldg(&dhat[v0]), r = __ldg(&thickness[v0]) + d;
+        const float ext = fmaxf(mx.x - mn.x, fmaxf(mx.y - mn.y, mx.z - mn.z)) + 2.0f * d;  // the leaf box has the thickness
         if (!(mn.x == a.x && mn.y == a.y && mn.z == a.z && mx.x == b.x && mx.y == b.y && mx.z == b.z) || !isfinite(d) ||
-            !isfinite(r))
+            !isfinite(r) || !isfinite(mn.x + mn.y + mn.z) || !isfinite(mx.x + mx.y + mx.z))
             bad = 1;
         dm = max(dm, ordered(d));
         rm = max(rm, ordered(r));
+        sum[0] += d;
+        sum[1] += ext;
     }
     bad = __reduce_max_sync(0xFFFFFFFFu, bad);
     dm = __reduce_max_sync(0xFFFFFFFFu, dm);
     rm = __reduce_max_sync(0xFFFFFFFFu, rm);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], o);
+    }
     if (lane_id() == 0) {
         if (bad) atomicOr(&info[0], 1u);
         atomicMax(&info[1], dm);
         atomicMax(&info[2], rm);
+        s_sum[threadIdx.x >> 5][0] = sum[0];
+        s_sum[threadIdx.x >> 5][1] = sum[1];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += s_sum[w][threadIdx.x];
+        atomicAdd(reinterpret_cast<float*>(&info[3 + threadIdx.x]), v);
     }
 }
 
@@ -970,7 +1133,7 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
     __shared__ uint2 s_stack[4][kPacketStack];
     __shared__ uint2 s_pairs[4][kPacketPairs];
     if (early()) return;  // k_query_ref<true> (the full EE walk) instead
-    if (PerEdge && sym_info[0] != 0u) return;       // k_query<true> instead
+    if (PerEdge && !sym_serves(sym_info, n_leaves)) return;  // k_query<true> instead
     const float d_max = PerEdge ? from_ordered(sym_info[1]) : 0.0f;
     const float r_max = PerEdge ? fabsf(from_ordered(sym_info[2])) : 0.0f;
     const uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
@@ -980,24 +1143,7 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_round; t += gridDim.x * blockDim.x) {
         const bool on = t < n_leaves;
         const uint32_t q = __ldg(&sgo[on ? t : n_leaves - 1]);
-        const uint2 ed = __ldg(&edges[q]);
-        const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
-        const v3 mn = min3(min3(s0, s1), min3(e0, e1)), mx = max3(max3(s0, s1), max3(e0, e1));
-        const float th = PerEdge ? __ldg(&thickness[ed.x]) : 0.0f;
-        const float r = PerEdge ? th + __ldg(&dhat[ed.x]) : uniform_r;
-        const float4 own_mn = make_float4(PerEdge ? mn.x - th : mn.x, PerEdge ? mn.y - th : mn.y, PerEdge ? mn.z - th : mn.z, 0.f);
-        const float4 own_mx = make_float4(PerEdge ? mx.x + th : mx.x, PerEdge ? mx.y + th : mx.y, PerEdge ? mx.z + th : mx.z, 0.f);
-        const float box[6] = {mn.x - r, mn.y - r, mn.z - r, mx.x + r, mx.y + r, mx.z + r};
-        float cull[6];
-        {
-            const float rc = PerEdge ? fmaxf(r, th + d_max) : r;
-            const float rm = PerEdge ? fabsf(rc) + r_max + fabsf(th) + fabsf(d_max) : r;
-            const float mgx = (fabsf(mn.x) + fabsf(mx.x) + rm) * 9.5367431640625e-07f;  // 2^-20
-            const float mgy = (fabsf(mn.y) + fabsf(mx.y) + rm) * 9.5367431640625e-07f;
-            const float mgz = (fabsf(mn.z) + fabsf(mx.z) + rm) * 9.5367431640625e-07f;
-            cull[0] = mn.x - rc - mgx; cull[1] = mn.y - rc - mgy; cull[2] = mn.z - rc - mgz;
-            cull[3] = mx.x + rc + mgx; cull[4] = mx.y + rc + mgy; cull[5] = mx.z + rc + mgz;
-        }
+        const SymQuery Q = sym_query<PerEdge>(x0, x1, edges, uniform_r, dhat, thickness, d_max, r_max, q);
         uint32_t steps = 0, held = 0;
         bool dead = false;
         auto flush = [&]() {
@@ -1027,23 +1173,15 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float4 cmn = rec[2 * k], cmx = rec[2 * k + 1];
-                const bool ov = act && !dead && __float_as_uint(cmx.w) > t && overlap(cmn, cmx, cull);
+                const bool ov = act && !dead && __float_as_uint(cmx.w) > t && overlap(cmn, cmx, Q.cull);
                 const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, ov);
                 if (lanes == 0) continue;
                 const uint32_t code = __float_as_uint(cmn.w);
                 if (code & 0x80000000u) {
                     const uint32_t e = code & 0x7FFFFFFFu;
-                    v3 en = mk3(cmn.x, cmn.y, cmn.z), ex = mk3(cmx.x, cmx.y, cmx.z);
-                    float re = r;
-                    if (PerEdge) {  // e's own query box, the same for every lane
-                        const uint2 ee = __ldg(&edges[e]);
-                        const v3 a0 = ld3(x0, ee.x), a1 = ld3(x0, ee.y), b0 = ld3(x1, ee.x), b1 = ld3(x1, ee.y);
-                        en = min3(min3(a0, a1), min3(b0, b1));
-                        ex = max3(max3(a0, a1), max3(b0, b1));
-                        re = __ldg(&thickness[ee.x]) + __ldg(&dhat[ee.x]);
-                    }
-                    const float qe[6] = {en.x - re, en.y - re, en.z - re, ex.x + re, ex.y + re, ex.z + re};
-                    const bool hit = ov && (q < e ? overlap(cmn, cmx, box) : overlap(own_mn, own_mx, qe));
+                    float qe[6];
+                    met_box<PerEdge>(x0, x1, edges, dhat, thickness, Q.r, e, cmn, cmx, qe);
+                    const bool hit = ov && (q < e ? overlap(cmn, cmx, Q.box) : overlap(Q.own_mn, Q.own_mx, qe));
                     const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
                     if (hit) buf[held + __popc(hits & lt)] = q < e ? make_uint2(q, e) : make_uint2(e, q);
                     held += __popc(hits);
@@ -1065,43 +1203,19 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
     }
 }
 
-// The same walk, one query per thread, for trees that leave most of the GPU's warps idle: a warp's union of paths is
-// longer than its longest path, which is what the time is there.
-template <bool PerEdge>
+// The same walk with one radius, one query per thread, for trees that leave most of the GPU's warps idle: a warp's union
+// of paths is longer than its longest path, which is what the time is there.
 __global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restrict__ wide4, const uint32_t* __restrict__ sgo,
-                                                      uint32_t n_leaves, const float4* __restrict__ x0,
-                                                      const float4* __restrict__ x1, const uint2* __restrict__ edges,
-                                                      float uniform_r, const float* __restrict__ dhat,
-                                                      const float* __restrict__ thickness,
-                                                      const uint32_t* __restrict__ sym_info, uint2* __restrict__ pairs,
-                                                      uint32_t capacity, uint32_t* d_count, uint32_t* capped,
-                                                      const Early early)
+                                                           uint32_t n_leaves, const float4* __restrict__ x0,
+                                                           const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                           float uniform_r, uint2* __restrict__ pairs, uint32_t capacity,
+                                                           uint32_t* d_count, uint32_t* capped, const Early early)
 {
     if (early()) return;  // k_query_ref<true> (the full EE walk) instead
-    if (PerEdge && sym_info[0] != 0u) return;       // k_query<true> instead
-    const float d_max = PerEdge ? from_ordered(sym_info[1]) : 0.0f;
-    const float r_max = PerEdge ? fabsf(from_ordered(sym_info[2])) : 0.0f;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_leaves; t += gridDim.x * blockDim.x) {
         const uint32_t q = __ldg(&sgo[t]);
-        const uint2 ed = __ldg(&edges[q]);
-        const v3 s0 = ld3(x0, ed.x), s1 = ld3(x0, ed.y), e0 = ld3(x1, ed.x), e1 = ld3(x1, ed.y);
-        const v3 mn = min3(min3(s0, s1), min3(e0, e1)), mx = max3(max3(s0, s1), max3(e0, e1));
-        const float th = PerEdge ? __ldg(&thickness[ed.x]) : 0.0f;
-        const float r = PerEdge ? th + __ldg(&dhat[ed.x]) : uniform_r;
-        const float4 own_mn = make_float4(PerEdge ? mn.x - th : mn.x, PerEdge ? mn.y - th : mn.y, PerEdge ? mn.z - th : mn.z, 0.f);
-        const float4 own_mx = make_float4(PerEdge ? mx.x + th : mx.x, PerEdge ? mx.y + th : mx.y, PerEdge ? mx.z + th : mx.z, 0.f);
-        const float box[6] = {mn.x - r, mn.y - r, mn.z - r, mx.x + r, mx.y + r, mx.z + r};
-        float cull[6];
-        {
-            const float rc = PerEdge ? fmaxf(r, th + d_max) : r;
-            const float rm = PerEdge ? fabsf(rc) + r_max + fabsf(th) + fabsf(d_max) : r;
-            const float mgx = (fabsf(mn.x) + fabsf(mx.x) + rm) * 9.5367431640625e-07f;  // 2^-20
-            const float mgy = (fabsf(mn.y) + fabsf(mx.y) + rm) * 9.5367431640625e-07f;
-            const float mgz = (fabsf(mn.z) + fabsf(mx.z) + rm) * 9.5367431640625e-07f;
-            cull[0] = mn.x - rc - mgx; cull[1] = mn.y - rc - mgy; cull[2] = mn.z - rc - mgz;
-            cull[3] = mx.x + rc + mgx; cull[4] = mx.y + rc + mgy; cull[5] = mx.z + rc + mgz;
-        }
-        uint32_t stack[kStack4];
+        const SymQuery Q = sym_query<false>(x0, x1, edges, uniform_r, nullptr, nullptr, 0.0f, 0.0f, q);
+        uint32_t stack[kSymStack];
         int sp = 0;
         uint32_t loop = 0;
         stack[sp++] = 0;
@@ -1117,26 +1231,18 @@ __global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restr
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float4 cmn = rec[2 * k], cmx = rec[2 * k + 1];
-                if (!stop && __float_as_uint(cmx.w) > t && overlap(cmn, cmx, cull)) {
+                if (!stop && __float_as_uint(cmx.w) > t && overlap(cmn, cmx, Q.cull)) {
                     const uint32_t code = __float_as_uint(cmn.w);
                     if (code & 0x80000000u) {
                         const uint32_t e = code & 0x7FFFFFFFu;
                         if (q < e) {
-                            if (overlap(cmn, cmx, box)) hit[nhit++] = make_uint2(q, e);
+                            if (overlap(cmn, cmx, Q.box)) hit[nhit++] = make_uint2(q, e);
                         } else {
-                            v3 en = mk3(cmn.x, cmn.y, cmn.z), ex = mk3(cmx.x, cmx.y, cmx.z);
-                            float re = r;
-                            if (PerEdge) {
-                                const uint2 ee = __ldg(&edges[e]);
-                                const v3 a0 = ld3(x0, ee.x), a1 = ld3(x0, ee.y), b0 = ld3(x1, ee.x), b1 = ld3(x1, ee.y);
-                                en = min3(min3(a0, a1), min3(b0, b1));
-                                ex = max3(max3(a0, a1), max3(b0, b1));
-                                re = __ldg(&thickness[ee.x]) + __ldg(&dhat[ee.x]);
-                            }
-                            const float qe[6] = {en.x - re, en.y - re, en.z - re, ex.x + re, ex.y + re, ex.z + re};
-                            if (overlap(own_mn, own_mx, qe)) hit[nhit++] = make_uint2(e, q);
+                            float qe[6];
+                            met_box<false>(x0, x1, edges, nullptr, nullptr, Q.r, e, cmn, cmx, qe);
+                            if (overlap(Q.own_mn, Q.own_mx, qe)) hit[nhit++] = make_uint2(e, q);
                         }
-                    } else if (sp < kStack4) {
+                    } else if (sp < kSymStack) {
                         stack[sp++] = code;
                     } else {
                         stop = true;
@@ -1284,11 +1390,11 @@ extern "C" int lcs_bvh_create(int kind, uint32_t n_leaves, lcs_bvh** out)
     A(alloc(h->seg_box, 2 * chunks * kRefitSegs));
     A(alloc(h->chunk_box, 2 * chunks));
     A(alloc(h->healthy, 1));
-    A(alloc(h->turns, 2 + kMaxTops));
+    A(alloc(h->turns, 3 + kMaxTops));
     A(alloc(h->top_lefts, 32 * kMaxTops));
     A(alloc(h->early, kSymSlots));
-    if (kind == LCS_TREE_EDGE) A(alloc(h->sym_info, 4 * kSymSlots));
-    if (e == cudaSuccess) e = cudaMemset(h->turns, 0, 2 * sizeof(uint32_t));
+    if (kind == LCS_TREE_EDGE) A(alloc(h->sym_info, kSymWords * kSymSlots));
+    if (e == cudaSuccess) e = cudaMemset(h->turns, 0, 3 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(h->early, 0, kSymSlots * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(h->span_count, 0, sizeof(uint32_t));
     const uint32_t np1 = n_leaves + 1;
@@ -1487,13 +1593,17 @@ extern "C" int lcs_bvh_update_refit(lcs_bvh* h, const float* thickness, const fl
     return leaves_refit(h, thickness, x0, x1, elems, 1, 1, stream);
 }
 
+static uint32_t next_call(const lcs_bvh* t)
+{
+    const uint32_t call = __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);
+    return call ? call : __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);  // 0 marks nothing
+}
+
 // k_may_end of a call, and its answer
 template <bool EE>
-static Early ask_early(const lcs_bvh* t, const float* x0, const float* x1, const uint32_t* edges, uint32_t n, const float* dhat,
-                       const float* thickness, float uniform_r, const uint32_t* order, cudaStream_t s)
+static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const float* x1, const uint32_t* edges, uint32_t n,
+                       const float* dhat, const float* thickness, float uniform_r, const uint32_t* order, cudaStream_t s)
 {
-    uint32_t call = __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);
-    if (call == 0) call = __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);  // 0 marks nothing
     uint32_t* flag = t->early + call % kSymSlots;
     if (t->ni > 0) {
         k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, reinterpret_cast<const float4*>(x0),
@@ -1520,7 +1630,8 @@ int lcs_bvh_query_vf_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: bad argument (needs a face tree)");
     if (t->n == 0 || n_verts == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: the tree has not been constructed");
-    const Early early = ask_early<false>(t, x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr, (cudaStream_t)stream);
+    const Early early = ask_early<false>(t, next_call(t), x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr,
+                                         (cudaStream_t)stream);
     k_query<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts,
         d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity, d_count, nullptr, capped, early, nullptr);
@@ -1552,24 +1663,31 @@ int lcs_bvh_query_ee_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee: bad argument (needs an edge tree)");
     if (t->n == 0 || n_edges == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee: the tree has not been constructed");
-    const Early early = ask_early<true>(t, x0, x1, edges, n_edges, d_hat, thickness, 0.0f,
-                                        n_edges == t->n ? t->sgo : nullptr, (cudaStream_t)stream);
-    // The tree's own edges in earnest numbers: once per pair, if the device finds the leaf boxes to be those of the
-    // arguments (the check and its two extra launches cost 8 us; below 8,192 edges that is what the walk would save).
-    const uint32_t* info = nullptr;
-    if (n_edges == t->n && n_edges >= 8192) {
-        uint32_t* slot = t->sym_info + 4 * (early.call % kSymSlots);
-        const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
-        const uint2* e2 = reinterpret_cast<const uint2*>(edges);
-        cudaStream_t s = (cudaStream_t)stream;
-        LCS_CUDA_TRY(cudaMemsetAsync(slot, 0, 16, s));
-        k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat, thickness, slot);
+    const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
+    const uint2* e2 = reinterpret_cast<const uint2*>(edges);
+    cudaStream_t s = (cudaStream_t)stream;
+    const uint32_t call = next_call(t);
+    // The tree's own edges in earnest numbers: once per pair, if the device finds the arguments fit for it.  Two sheets of
+    // 74,000, 268,000 and 1.2 million edges: 376, 966 and 4,525 us so, 350, 1,033 and 5,700 by k_query<true> alone.
+    uint32_t* info = nullptr;
+    if (n_edges == t->n && n_edges >= kSymEdges) {
+        info = t->sym_info + kSymWords * (call % kSymSlots);
+        LCS_CUDA_TRY(cudaMemsetAsync(info, 0, 4 * kSymWords, s));
+        k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat, thickness, t->turns,
+                                                             info);
         lcs_count_launch();
-        const auto walk = t->n >= kPacketLeaves ? k_query_ee_sym<true> : k_query_ee_sym_lane<true>;
-        walk<<<grid_for(n_edges, 128, 16), 128, 0, s>>>(t->wide4, t->sgo, t->n, p0, p1, e2, 0.0f, d_hat, thickness, slot,
-                                                        reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
+        if (t->ni > kRefNodes) {
+            k_may_exceed<<<grid_for(t->n, 256), 256, 0, s>>>(t->wide, t->ni, p0, p1, e2, d_hat, thickness, t->sgo, info);
+            lcs_count_launch();
+        }
+    }
+    const Early early = ask_early<true>(t, call, x0, x1, edges, n_edges, d_hat, thickness, 0.0f,
+                                        n_edges == t->n ? t->sgo : nullptr, s);
+    if (info) {
+        k_query_ee_sym<true><<<grid_for(n_edges, 128, 16), 128, 0, s>>>(t->wide4, t->sgo, t->n, p0, p1, e2, 0.0f, d_hat,
+                                                                        thickness, info, reinterpret_cast<uint2*>(pairs),
+                                                                        capacity, d_count, capped, early);
         lcs_count_launch();
-        info = slot;
     }
     k_query<true><<<grid_for(n_edges, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
@@ -1603,12 +1721,17 @@ int lcs_bvh_query_ee_sym_capped(const lcs_bvh* t, const float* x0, const float* 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: bad argument (needs an edge tree, d_hat >= 0)");
     if (t->n == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: the tree has not been constructed");
-    const Early early = ask_early<true>(t, x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo, (cudaStream_t)stream);
-    const auto walk = t->n >= kPacketLeaves ? k_query_ee_sym<false> : k_query_ee_sym_lane<false>;
-    walk<<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-        t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-        reinterpret_cast<const uint2*>(edges), d_hat, nullptr, nullptr, nullptr, reinterpret_cast<uint2*>(pairs), capacity,
-        d_count, capped, early);
+    const Early early = ask_early<true>(t, next_call(t), x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo,
+                                        (cudaStream_t)stream);
+    if (t->n >= kPacketLeaves)
+        k_query_ee_sym<false><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
+            t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
+            reinterpret_cast<const uint2*>(edges), d_hat, nullptr, nullptr, nullptr, reinterpret_cast<uint2*>(pairs), capacity,
+            d_count, capped, early);
+    else
+        k_query_ee_sym_lane<<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
+            t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
+            reinterpret_cast<const uint2*>(edges), d_hat, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
     lcs_count_launch();
     if (t->ni > 0) {  // a call in which the stack may fill: the reference's full EE walk (its early exits break the symmetry)
         k_query_ref<true><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(

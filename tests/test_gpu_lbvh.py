@@ -11,6 +11,7 @@ from luisacomputesimulator_b200.collision import LBVH
 from oracle import oracle as O
 from tests import scenarios as SC
 from tests.gpu_util import SceneOnDevice, counts, dev, host
+from tests.test_oracle_deep_tree import _max_inner_depth
 
 pytestmark = pytest.mark.gpu
 
@@ -402,25 +403,40 @@ def test_deep_tree_once_per_pair_query_falls_back_to_the_reference_walk():
         np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n]), SC.sorted_pairs(want))
 
 
-@pytest.mark.parametrize("side,swept,foreign", [(40, False, False), (53, False, False), (53, True, False), (60, True, True),
-                                                (150, True, False)])
-def test_general_ee_query_once_per_pair_and_its_fallback(side, swept, foreign):
-    """The general EE query around the 8,192 edges from which it meets each pair once (side 53 has 8,216), with per-vertex
-    thickness and d_hat, and at the 65,536 from which a warp walks for 32 queries (side 150 has 66,901); `foreign` queries with other positions than the tree's, which the full walk has to answer."""
+def _sheet(side):
     i = np.arange(side)
     X, Z = np.meshgrid(i, i, indexing="ij")
     v = X * side + Z
     pair = lambda a, b: np.stack([a.ravel(), b.ravel()], 1)  # noqa: E731
     el = np.concatenate([pair(v[:-1], v[1:]), pair(v[:, :-1], v[:, 1:]), pair(v[:-1, :-1], v[1:, 1:])]).astype(np.uint32)
-    rng = np.random.default_rng(side)
-    n = side * side
-    x = np.zeros((n, 4), np.float32)
+    x = np.zeros((side * side, 4), np.float32)
     x[:, 0], x[:, 2] = X.ravel() * 0.01, Z.ravel() * 0.01
-    x[:, 1] = 2e-3 * rng.random(n)
+    return x, el
+
+
+def _deep_sheet(side):
+    """A sheet, uneven by 2 mm, and a few edges beside it that give the tree one path of 32 levels."""
+    x, el = _sheet(side)
+    x[:, 1] = 2e-3 * np.random.default_rng(side).random(len(x))
+    deep, deep_el = SC.deep_tree_elements("edge")
+    return np.concatenate([deep / 256, x]), np.concatenate([deep_el, el + np.uint32(len(deep))])
+
+
+@pytest.mark.parametrize("side,swept,foreign", [(40, False, False), (53, False, False), (53, True, False), (60, True, True),
+                                                (150, True, False), (209, True, False), (210, True, False), (210, False, False),
+                                                (210, True, True)])
+def test_general_ee_query_once_per_pair_and_its_fallback(side, swept, foreign):
+    """The general EE query around the 131,072 edges from which it meets each pair once (side 210 has 131,530) on a tree of
+    more than 32 levels (a few edges beside the sheet make one path of it that deep), with per-vertex thickness and d_hat;
+    `foreign` queries with other positions than the tree's, which the full walk has to answer."""
+    x, el = _deep_sheet(side)
+    rng = np.random.default_rng(side)
+    n = len(x)
     x1 = x + (rng.normal(0, 3e-3, x.shape).astype(np.float32) if swept else 0)
     th = rng.uniform(0, 2e-3, n).astype(np.float32)
-    dh = rng.uniform(1e-4, 3e-3, n).astype(np.float32)
+    dh = rng.uniform(1e-3, 3e-3, n).astype(np.float32)
     t_o = O.lbvh_build(O.TREE_EDGE, x, el, n)
+    assert _max_inner_depth(t_o) >= 32
     O.lbvh_refit(t_o, x, x1, el, th)
     bvh = LBVH(O.TREE_EDGE, el.shape[0])
     xd, x1d, ed = dev(x), dev(x1), dev(el)
@@ -464,3 +480,86 @@ def test_deep_tree_without_pending_nodes(kind_name, rad):
         bvh.broad_phase_query_from_verts(xd, xd, cnt, pairs, dev(r), dev(z))
     assert int(counts(cnt)[0]) == n_want
     np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
+
+
+def _ee_query(bvh, x, el, want, n_want, dh, th=None):
+    """The general query (dh an array) or the once-per-pair one (dh a number) of an edge tree against an expected set."""
+    xd, ed = dev(x), dev(el)
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pairs = torch.zeros((n_want + 64, 2), dtype=torch.int32, device="cuda")
+    if np.ndim(dh):
+        bvh.broad_phase_query_from_edges(xd, xd, ed, cnt, pairs, dev(dh), dev(th))
+    else:
+        bvh.broad_phase_query_from_edges_sym(xd, xd, ed, cnt, pairs, dh)
+    assert int(counts(cnt)[0]) == n_want
+    np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
+
+
+def _edge_trees(x, el, th):
+    t_o = O.lbvh_build(O.TREE_EDGE, x, el, x.shape[0])
+    O.lbvh_refit(t_o, x, x, el, th)
+    bvh = LBVH(O.TREE_EDGE, el.shape[0])
+    xd, ed = dev(x), dev(el)
+    bvh.reduce_edge_tree_aabb(xd, ed)
+    bvh.construct_tree()
+    bvh.update_and_refit(dev(th), xd, xd, ed)
+    return t_o, bvh
+
+
+@pytest.mark.parametrize("side,far", [(60, 0.05), (290, 10.3)])
+def test_general_ee_query_with_one_far_reaching_edge(side, far):
+    """One edge reaches fifty times and ten thousand times as far as the others.  It lies beside the sheet and meets a
+    tenth of it, so that its own walk ends nowhere; looked at with its reach, the others' walks of 251,000 edges would end early."""
+    x, el = _deep_sheet(side)
+    away = np.zeros((2, 4), np.float32)
+    away[:, 0], away[1, 2] = 0.001 * side - far, 0.01
+    el = np.concatenate([el, np.array([[len(x), len(x) + 1]], np.uint32)])
+    x = np.concatenate([x, away])
+    dh, th = np.full(len(x), 1e-3, np.float32), np.random.default_rng(1).uniform(0, 1e-3, len(x)).astype(np.float32)
+    dh[-2:] = far
+    t_o, bvh = _edge_trees(x, el, th)
+    want, n_want = O.lbvh_query_ee(t_o, x, x, el, dh, th)
+    assert n_want > len(el)
+    _ee_query(bvh, x, el, want, n_want, dh, th)
+
+
+def _turning_tree(n, chain):
+    """Edges whose tree turns right `chain` times past subtrees of four (all bits but one of the last `chain` of the code
+    set) and then holds the others, of one code, split by their ids: up to chain + 14 right turns past inner nodes."""
+    cells = []
+    for k in range(chain):
+        c = np.full(3, 1023.5)
+        c[2 - k % 3] -= 2 ** (k // 3)
+        cells += [[c - 0.25, c + 0.25]] * 4
+    m = n - len(cells) - 1
+    s = int(np.ceil(m ** (1 / 3)))
+    g = np.stack(np.unravel_index(np.arange(m), (s, s, s)), 1) / s * 0.999 + 1023.0005
+    top = np.stack([g, g + 1e-3], 1)
+    top[-1, 1] = 1024.0
+    pts = np.concatenate([[[np.zeros(3), np.ones(3)]], cells, top]).reshape(-1, 3)
+    x = np.zeros((2 * n, 4), np.float32)
+    x[:, :3] = pts
+    return x, np.arange(2 * n, dtype=np.uint32).reshape(-1, 2)
+
+
+@pytest.mark.parametrize("n", [65535, 66001, 131072])  # a thread per edge, a warp per 32, also in the general query
+@pytest.mark.parametrize("chain", [30, 24])    # 44 turns at most; more nodes of 31 turns than are listed
+@pytest.mark.parametrize("mode", ["once", "general", "far", "ends"])
+def test_ee_queries_of_a_tree_with_many_turns(n, chain, mode):
+    """`far`: the edge at the far corner reaches through three quarters of the scene, and meets nothing; the walks of the
+    others would keep more than 64 nodes pending with its reach.  `ends`: eight edges reach so far that their stacks of 32
+    fill, as the oracle's do."""
+    x, el = _turning_tree(n, chain)
+    z = np.zeros(len(x), np.float32)
+    dh = np.full(len(x), 1e-3, np.float32)
+    if mode == "far":
+        dh[:2] = 768.0
+    if mode == "ends":
+        dh[2:18] = 1200.0
+    t_o, bvh = _edge_trees(x, el, z)
+    want, n_want = O.lbvh_query_ee(t_o, x, x, el, dh, z)
+    if mode == "ends":
+        assert n_want < 8 * (n - 9)  # their walks ended: alone they would meet every edge of a higher id
+    else:
+        assert n_want >= 6 * chain
+    _ee_query(bvh, x, el, want, n_want, 1e-3 if mode == "once" else dh, z)
