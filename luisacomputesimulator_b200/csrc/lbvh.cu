@@ -66,6 +66,7 @@ struct lcs_bvh {
     uint32_t* early = nullptr;       // kSymSlots: number of the query call that may end early, a slot per call in turn
     uint32_t* sym_info = nullptr;    // kSymSlots x kSymWords: k_sym_check's findings, a slot per query call in turn
     mutable uint32_t calls = 0;
+    bool leaves_newer = false;       // leaf boxes were written after the last refit (the binary records alone hold them)
     bool built = false;              // a construct has written the topology, slots and refit tables
 };
 
@@ -680,10 +681,9 @@ constexpr int kStack4 = 64;  // entries of the 4-wide traversal stack
 // synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
 // with a few paths of 31 turns near one corner, but no query keeps more than a handful of nodes pending.
 struct Early {
-    const uint32_t* turns;
     const uint32_t* flag;  // the call's slot: its number if it may end early
     uint32_t call;
-    __device__ __forceinline__ bool operator()() const { return __ldg(&turns[0]) >= kRefPending && *flag == call; }
+    __device__ __forceinline__ bool operator()() const { return *flag == call; }
 };
 
 // the box of query q: an edge (EE) or a vertex, swept, widened by per-vertex thickness + d_hat, or by one radius for
@@ -858,7 +858,8 @@ __global__ void __launch_bounds__(256) k_may_exceed(const float4* __restrict__ w
 // were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's walk
 // reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and a near
 // top's left siblings, one per lane, against the union of its 32 queries' boxes; only where that is not enough does each
-// query climb.
+// query climb.  A tree of 32 levels whose leaf boxes are newer than its inner ones is walked the reference's way as well:
+// the 4-wide records have the leaf boxes of the last refit.
 template <bool EE>
 __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide, const uint32_t* __restrict__ slot,
                                                  const uint32_t* __restrict__ turns, const uint32_t* __restrict__ top_lefts,
@@ -866,11 +867,13 @@ __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide
                                                  const float4* __restrict__ x1, const uint2* __restrict__ edges,
                                                  uint32_t n_queries, const float* __restrict__ dhat,
                                                  const float* __restrict__ thickness, float uniform_r,
-                                                 const uint32_t* __restrict__ order, uint32_t call, uint32_t* __restrict__ flag)
+                                                 const uint32_t* __restrict__ order, bool leaves_newer, uint32_t call,
+                                                 uint32_t* __restrict__ flag)
 {
     const uint32_t most = turns[0], tops = turns[1];
-    if (most < kRefPending) return;
-    if (tops > kMaxTops) {
+    const bool newer = leaves_newer && turns[2] >= kRefStack;
+    if (most < kRefPending && !newer) return;
+    if (tops > kMaxTops || newer) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *flag = call;
         return;
     }
@@ -1548,6 +1551,7 @@ static int leaves_refit(lcs_bvh* h, const float* thickness, const float* x0, con
     cudaStream_t s = (cudaStream_t)stream;
     const float4* px0 = reinterpret_cast<const float4*>(x0);
     const float4* px1 = reinterpret_cast<const float4*>(x1);
+    h->leaves_newer = h->n > 1 && !climb && (write_leaf || h->leaves_newer);
     if (climb && h->n > 1) {
         const uint32_t chunks = (h->n + kRefitChunk - 1) / kRefitChunk;
         k_refit_chunks<<<chunks, kRefitChunk, 0, s>>>(h->kind, h->n, h->sgo, h->slot, h->leaf_at, h->node_at,
@@ -1609,10 +1613,10 @@ static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const f
         k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, reinterpret_cast<const float4*>(x0),
                                                       reinterpret_cast<const float4*>(x1),
                                                       reinterpret_cast<const uint2*>(edges), n, dhat, thickness, uniform_r,
-                                                      order, call, flag);
+                                                      order, t->leaves_newer, call, flag);
         lcs_count_launch();
     }
-    return Early{t->turns, flag, call};
+    return Early{flag, call};
 }
 
 extern "C" int lcs_bvh_query_vf(const lcs_bvh* t, const float* x0, const float* x1, uint32_t n_verts,

@@ -563,3 +563,26 @@ def test_ee_queries_of_a_tree_with_many_turns(n, chain, mode):
     else:
         assert n_want >= 6 * chain
     _ee_query(bvh, x, el, want, n_want, 1e-3 if mode == "once" else dh, z)
+
+
+@pytest.mark.parametrize("side", [53, 210])
+def test_queries_between_a_leaf_update_and_its_refit(side):
+    """Leaf boxes written by themselves are what the queries of a tree of 32 levels meet, inner boxes being those of the
+    refit before; after the refit all are new."""
+    x, el = _deep_sheet(side)
+    z = np.zeros(len(x), np.float32)
+    dh = np.full(len(x), 2e-3, np.float32)
+    t_o, bvh = _edge_trees(x, el, z)
+    y = x + np.random.default_rng(1).normal(0, 4e-3, x.shape).astype(np.float32)
+    O.lib().orc_lbvh_update_leaves(t_o.kind, O._p(t_o.sorted_get_original), t_o.n, O._p(z), O._p(y), O._p(y), O._p(el),
+                                   O._p(t_o.node_aabb))
+    bvh.update_leaves(dev(z), dev(y), dev(y), dev(el))
+    want, n_want = O.lbvh_query_ee(t_o, y, y, el, dh, z)
+    for d in (dh, 2e-3):
+        _ee_query(bvh, y, el, want, n_want, d, z)
+    O.lbvh_refit(t_o, y, y, el, z)
+    bvh.refit()
+    all_pairs, n_all = O.lbvh_query_ee(t_o, y, y, el, dh, z)
+    assert n_all > n_want
+    for d in (dh, 2e-3):
+        _ee_query(bvh, y, el, all_pairs, n_all, d, z)
