@@ -680,6 +680,7 @@ constexpr int kStack4 = 64;  // entries of the 4-wide traversal stack
 // launch reads the answer and returns at once if it is the other's call, so the choice costs no host
 // synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
 // with a few paths of 31 turns near one corner, but no query keeps more than a handful of nodes pending.
+// The other limit of the reference's walk, 100,000 popped nodes, is asked for by k_may_exceed.
 struct Early {
     const uint32_t* flag;  // the call's slot: its number if it may end early
     uint32_t call;
@@ -834,22 +835,43 @@ __device__ __forceinline__ void warp_union(const float* box, float* all)
     }
 }
 
-// Takes a general EE query off the once-per-pair walk where the largest d_hat could make an edge's walk pop so many nodes
-// that it would end: only the edge's own reach may end it.  A warp asks for the union of its 32 edges, neighbours in the
-// tree's order, and each edge for itself only where that is not enough (1.2 million edges: 0.14 ms).
-__global__ void __launch_bounds__(256) k_may_exceed(const float4* __restrict__ wide, uint32_t ni, const float4* __restrict__ x0, const float4* __restrict__ x1,
-                                                    const uint2* __restrict__ edges, const float* __restrict__ dhat,
-                                                    const float* __restrict__ thickness, const uint32_t* __restrict__ sgo,
-                                                    uint32_t* __restrict__ info)
+// Marks the call if one of its queries pops so many nodes that its walk ends, on a tree of 32 levels or more (as the stack
+// does, see Early; trees of fewer levels are walked by their own records, counted 4-wide).  A general EE query is also
+// taken off the once-per-pair walk (info) where the largest d_hat would make an edge's walk end: only its own reach may.
+// A warp asks for the union of its 32 queries, and each query for itself only where that is not enough (1.2 million edges
+// in the tree's order: 0.14 ms).
+template <bool EE>
+__global__ void __launch_bounds__(256) k_may_exceed(const float4* __restrict__ wide, uint32_t ni, const float4* __restrict__ x0,
+                                                    const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                    uint32_t n_queries, const float* __restrict__ dhat,
+                                                    const float* __restrict__ thickness, float uniform_r,
+                                                    const uint32_t* __restrict__ order, const uint32_t* __restrict__ turns,
+                                                    uint32_t call, uint32_t* __restrict__ flag, uint32_t* __restrict__ info)
 {
-    const uint32_t n = ni + 1;
-    if (!sym_serves(info, n)) return;
-    const float d_max = from_ordered(info[1]), r_max = fabsf(from_ordered(info[2]));
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ((n + 31u) & ~31u); t += gridDim.x * blockDim.x) {
-        const SymQuery Q = sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, d_max, r_max, __ldg(&sgo[min(t, n - 1)]));
-        float all[6];
-        warp_union(Q.cull, all);
-        if (exceeds(wide, ni, all, false) && exceeds(wide, ni, Q.cull, true)) atomicOr(&info[0], 1u);
+    if (turns[2] < kRefStack) return;
+    const bool sym = EE && info && sym_serves(info, ni + 1);
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ((n_queries + 31u) & ~31u); t += gridDim.x * blockDim.x) {
+        const uint32_t i = min(t, n_queries - 1), q = order ? __ldg(&order[i]) : i;
+        float box[6], all[6];
+        if (EE && (sym || !dhat)) {  // what the once-per-pair walk culls with
+            const SymQuery Q = sym ? sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, from_ordered(info[1]),
+                                                     fabsf(from_ordered(info[2])), q)
+                                   : sym_query<false>(x0, x1, edges, uniform_r, nullptr, nullptr, 0.0f, 0.0f, q);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) box[c] = Q.cull[c];
+        } else {
+            query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
+        }
+        warp_union(box, all);
+        if (exceeds(wide, ni, all, false) && exceeds(wide, ni, box, true)) {
+            bool ends = true;
+            if (EE && sym) {
+                atomicOr(&info[0], 1u);
+                query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
+                ends = exceeds(wide, ni, box, true);
+            }
+            if (ends) *flag = call;
+        }
         __syncwarp();
     }
 }
@@ -1603,17 +1625,23 @@ static uint32_t next_call(const lcs_bvh* t)
     return call ? call : __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);  // 0 marks nothing
 }
 
-// k_may_end of a call, and its answer
+// k_may_end and k_may_exceed of a call, and their answer
 template <bool EE>
 static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const float* x1, const uint32_t* edges, uint32_t n,
-                       const float* dhat, const float* thickness, float uniform_r, const uint32_t* order, cudaStream_t s)
+                       const float* dhat, const float* thickness, float uniform_r, const uint32_t* order, uint32_t* info,
+                       cudaStream_t s)
 {
+    const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
+    const uint2* e2 = reinterpret_cast<const uint2*>(edges);
     uint32_t* flag = t->early + call % kSymSlots;
     if (t->ni > 0) {
-        k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, reinterpret_cast<const float4*>(x0),
-                                                      reinterpret_cast<const float4*>(x1),
-                                                      reinterpret_cast<const uint2*>(edges), n, dhat, thickness, uniform_r,
-                                                      order, t->leaves_newer, call, flag);
+        k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, p0, p1, e2, n, dhat, thickness,
+                                                      uniform_r, order, t->leaves_newer, call, flag);
+        lcs_count_launch();
+    }
+    if (t->ni > kRefNodes) {
+        k_may_exceed<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->ni, p0, p1, e2, n, dhat, thickness, uniform_r, order,
+                                                         t->turns, call, flag, info);
         lcs_count_launch();
     }
     return Early{flag, call};
@@ -1634,7 +1662,7 @@ int lcs_bvh_query_vf_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: bad argument (needs a face tree)");
     if (t->n == 0 || n_verts == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: the tree has not been constructed");
-    const Early early = ask_early<false>(t, next_call(t), x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr,
+    const Early early = ask_early<false>(t, next_call(t), x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr, nullptr,
                                          (cudaStream_t)stream);
     k_query<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
         t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts,
@@ -1680,13 +1708,9 @@ int lcs_bvh_query_ee_capped(const lcs_bvh* t, const float* x0, const float* x1, 
         k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat, thickness, t->turns,
                                                              info);
         lcs_count_launch();
-        if (t->ni > kRefNodes) {
-            k_may_exceed<<<grid_for(t->n, 256), 256, 0, s>>>(t->wide, t->ni, p0, p1, e2, d_hat, thickness, t->sgo, info);
-            lcs_count_launch();
-        }
     }
     const Early early = ask_early<true>(t, call, x0, x1, edges, n_edges, d_hat, thickness, 0.0f,
-                                        n_edges == t->n ? t->sgo : nullptr, s);
+                                        n_edges == t->n ? t->sgo : nullptr, info, s);
     if (info) {
         k_query_ee_sym<true><<<grid_for(n_edges, 128, 16), 128, 0, s>>>(t->wide4, t->sgo, t->n, p0, p1, e2, 0.0f, d_hat,
                                                                         thickness, info, reinterpret_cast<uint2*>(pairs),
@@ -1725,7 +1749,7 @@ int lcs_bvh_query_ee_sym_capped(const lcs_bvh* t, const float* x0, const float* 
         return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: bad argument (needs an edge tree, d_hat >= 0)");
     if (t->n == 0) return LCS_OK;
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: the tree has not been constructed");
-    const Early early = ask_early<true>(t, next_call(t), x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo,
+    const Early early = ask_early<true>(t, next_call(t), x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo, nullptr,
                                         (cudaStream_t)stream);
     if (t->n >= kPacketLeaves)
         k_query_ee_sym<false><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(

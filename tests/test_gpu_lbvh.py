@@ -586,3 +586,63 @@ def test_queries_between_a_leaf_update_and_its_refit(side):
     assert n_all > n_want
     for d in (dh, 2e-3):
         _ee_query(bvh, y, el, all_pairs, n_all, d, z)
+
+
+def _pairs_across(n_pairs, m):
+    """Elements (m corners each) of one code whose neighbours by id lie at both sides of a gap: one long element in the gap,
+    of the first id, meets every inner node above them and a leaf in fifty.  A mirrored deep tree beside them makes it a
+    tree of more than 32 levels, on which no stack fills."""
+    x, el = SC.deep_tree_elements("edge" if m == 2 else "face")
+    x[:, :3] = np.float32(1024.0) - x[:, :3]
+    corner = x[:, :3].max(1) <= 1  # the elements of the pairs' cell: thin, or they would meet all of them
+    x[corner, :2] *= 0.01
+    if (len(el) + 1) % 2:  # pairs start at an even id
+        el = np.concatenate([el, el[-1:]])
+    i = np.arange(n_pairs)
+    p = np.zeros((1 + 2 * n_pairs, m, 3))
+    p[:, :, 2] = 0.5
+    p[0, 0, :2], p[0, 1:, :2] = [0.5, 0.05], [0.5, 0.95]
+    p[1::2, :, 0], p[2::2, :, 0] = 0.1, np.where(i % 50 == 0, 0.5, 0.9)[:, None]
+    p[1:, 1:, 0] += 1e-4
+    p[1:, :, 1] = np.repeat(0.05 + 0.9 * i / n_pairs, 2)[:, None]
+    new = np.arange(m * len(p), dtype=np.uint32).reshape(-1, m) + np.uint32(len(x))
+    if m == 3:
+        new = np.concatenate([new, np.zeros((len(new), 1), np.uint32)], 1)
+    xn = np.zeros((m * len(p), 4), np.float32)
+    xn[:, :3] = p.reshape(-1, 3)
+    return np.concatenate([x, xn]), np.concatenate([el, new]), len(x)
+
+
+@pytest.mark.parametrize("kind_name,n_pairs", [("face", 49900), ("face", 55000), ("edge", 49900), ("edge", 55000), ("edge", 70000)])
+@pytest.mark.parametrize("once", [False, True])
+def test_queries_of_more_than_a_hundred_thousand_nodes(kind_name, n_pairs, once):
+    """The query of the long element pops more than 100,000 nodes (fewer with 49,900 pairs) and ends there, as the oracle's
+    does, without the pairs it would meet after that."""
+    ee = kind_name == "edge"
+    if once and not ee:
+        pytest.skip("vertices have no once-per-pair form")
+    x, el, first = _pairs_across(n_pairs, 2 if ee else 3)
+    kind = KINDS[kind_name][0]
+    t_o = O.lbvh_build(kind, x, el, len(x))
+    assert _max_inner_depth(t_o) >= 32
+    z, r = np.zeros(len(x), np.float32), np.full(len(x), 1e-6, np.float32)
+    O.lbvh_refit(t_o, x, x, el, z)
+    bvh = LBVH(kind, el.shape[0])
+    xd, ed = dev(x), dev(el)
+    (bvh.reduce_edge_tree_aabb if ee else bvh.reduce_face_tree_aabb)(xd, ed)
+    bvh.construct_tree()
+    bvh.update_and_refit(dev(z), xd, xd, ed)
+    x1 = x.copy()
+    if not ee:
+        x1[first, 1] = 0.95  # one vertex moves along the gap
+    want, n_want = O.lbvh_query_ee(t_o, x, x, el, r, z) if ee else O.lbvh_query_vf(t_o, x, x1, r, z)
+    met = int((want[:, 0] == (len(el) - 2 * n_pairs - 1 if ee else first)).sum())
+    assert (met >= n_pairs // 50) == (n_pairs < 50000)
+    if ee:
+        _ee_query(bvh, x, el, want, n_want, 1e-6 if once else r, z)
+        return
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pairs = torch.zeros((n_want + 64, 2), dtype=torch.int32, device="cuda")
+    bvh.broad_phase_query_from_verts(xd, dev(x1), cnt, pairs, dev(r), dev(z))
+    assert int(counts(cnt)[0]) == n_want
+    np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
