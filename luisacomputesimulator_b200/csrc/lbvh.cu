@@ -261,13 +261,15 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
     for (uint32_t nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
         uint32_t p = nid, d = 0, pending = 0;
         bool own = false;
+        uint32_t s = nid != 0u ? slot[nid] : 0u;
         while (p != 0u && p < ni && d < 256u) {
-            const uint32_t s = slot[p];
-            p = s >> 1;
-            if ((s & 1u) && p < ni && children[p].x < ni) {
-                ++pending;
-                own = own || d == 0u;
-            }
+            const uint32_t up = s >> 1;  // the next level's load does not wait for this one's
+            const uint32_t next = up != 0u && up < ni ? slot[up] : 0u;
+            const bool turn = (s & 1u) && up < ni && children[up].x < ni;
+            pending += turn ? 1u : 0u;
+            own = own || (turn && d == 0u);
+            p = up;
+            s = next;
             ++d;
         }
         even[nid] = (d & 1u) == 0u ? 1 : 0;
@@ -279,9 +281,9 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
                 turns[3 + k] = slot[nid];
                 uint32_t i = 0;
                 for (p = nid; p != 0u && i < kRefPending;) {
-                    const uint32_t s = slot[p];
-                    p = s >> 1;
-                    if ((s & 1u) && children[p].x < ni) top_lefts[32 * k + i++] = s & ~1u;
+                    const uint32_t at = slot[p];
+                    p = at >> 1;
+                    if ((at & 1u) && children[p].x < ni) top_lefts[32 * k + i++] = at & ~1u;
                 }
             }
         }
@@ -676,11 +678,10 @@ constexpr int kStack4 = 64;  // entries of the 4-wide traversal stack
 // pending node for each right turn of the path past an inner left child that overlaps the query, so it can only fill --
 // and end a query early -- below one of the tops that k_depth_parity lists.  Every call first asks (k_may_end) whether
 // any of its queries could meet a full stack there; if none can, the 4-wide walks below serve it (their own 64-entry
-// stack holds at most two nodes per turn), else k_query_ref restates the reference's walk, early exit included.  Each
-// launch reads the answer and returns at once if it is the other's call, so the choice costs no host
-// synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
+// stack holds at most two nodes per turn), else query_ref restates the reference's walk, early exit included.  The
+// walks' kernels read the answer, so the choice costs no host synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
 // with a few paths of 31 turns near one corner, but no query keeps more than a handful of nodes pending.
-// The other limit of the reference's walk, 100,000 popped nodes, is asked for by k_may_exceed.
+// The other limit of the reference's walk, 100,000 popped nodes, is asked for there too.
 struct Early {
     const uint32_t* flag;  // the call's slot: its number if it may end early
     uint32_t call;
@@ -835,85 +836,58 @@ __device__ __forceinline__ void warp_union(const float* box, float* all)
     }
 }
 
-// Marks the call if one of its queries pops so many nodes that its walk ends, on a tree of 32 levels or more (as the stack
-// does, see Early; trees of fewer levels are walked by their own records, counted 4-wide).  A general EE query is also
-// taken off the once-per-pair walk (info) where the largest d_hat would make an edge's walk end: only its own reach may.
-// A warp asks for the union of its 32 queries, and each query for itself only where that is not enough (1.2 million edges
-// in the tree's order: 0.14 ms).
-template <bool EE>
-__global__ void __launch_bounds__(256) k_may_exceed(const float4* __restrict__ wide, uint32_t ni, const float4* __restrict__ x0,
-                                                    const float4* __restrict__ x1, const uint2* __restrict__ edges,
-                                                    uint32_t n_queries, const float* __restrict__ dhat,
-                                                    const float* __restrict__ thickness, float uniform_r,
-                                                    const uint32_t* __restrict__ order, const uint32_t* __restrict__ turns,
-                                                    uint32_t call, uint32_t* __restrict__ flag, uint32_t* __restrict__ info)
-{
-    if (turns[2] < kRefStack) return;
-    const bool sym = EE && info && sym_serves(info, ni + 1);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ((n_queries + 31u) & ~31u); t += gridDim.x * blockDim.x) {
-        const uint32_t i = min(t, n_queries - 1), q = order ? __ldg(&order[i]) : i;
-        float box[6], all[6];
-        if (EE && (sym || !dhat)) {  // what the once-per-pair walk culls with
-            const SymQuery Q = sym ? sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, from_ordered(info[1]),
-                                                     fabsf(from_ordered(info[2])), q)
-                                   : sym_query<false>(x0, x1, edges, uniform_r, nullptr, nullptr, 0.0f, 0.0f, q);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) box[c] = Q.cull[c];
-        } else {
-            query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
-        }
-        warp_union(box, all);
-        if (exceeds(wide, ni, all, false) && exceeds(wide, ni, box, true)) {
-            bool ends = true;
-            if (EE && sym) {
-                atomicOr(&info[0], 1u);
-                query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
-                ends = exceeds(wide, ni, box, true);
-            }
-            if (ends) *flag = call;
-        }
-        __syncwarp();
-    }
-}
-
 // Marks the call if one of its queries overlaps a listed top with so many overlapping inner left siblings above it that,
 // were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's walk
 // reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and a near
 // top's left siblings, one per lane, against the union of its 32 queries' boxes; only where that is not enough does each
 // query climb.  A tree of 32 levels whose leaf boxes are newer than its inner ones is walked the reference's way as well:
 // the 4-wide records have the leaf boxes of the last refit.
-template <bool EE>
+// Count (trees of more than kRefNodes inner nodes): on trees of 32 levels or more it also marks the call if one of its
+// queries pops so many nodes that its walk ends (trees of fewer levels are walked by their own records, counted 4-wide), and
+// takes a general EE query off the once-per-pair walk (info) where the largest d_hat would make an edge's walk end: only
+// its own reach may.  The union is asked first here too (1.2 million edges in the tree's order: 0.14 ms).
+template <bool EE, bool Count>
 __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide, const uint32_t* __restrict__ slot,
                                                  const uint32_t* __restrict__ turns, const uint32_t* __restrict__ top_lefts,
-                                                 const float4* __restrict__ x0,
-                                                 const float4* __restrict__ x1, const uint2* __restrict__ edges,
-                                                 uint32_t n_queries, const float* __restrict__ dhat,
-                                                 const float* __restrict__ thickness, float uniform_r,
-                                                 const uint32_t* __restrict__ order, bool leaves_newer, uint32_t call,
-                                                 uint32_t* __restrict__ flag)
+                                                 const float4* __restrict__ x0, const float4* __restrict__ x1,
+                                                 const uint2* __restrict__ edges, uint32_t n_queries,
+                                                 const float* __restrict__ dhat, const float* __restrict__ thickness,
+                                                 float uniform_r, const uint32_t* __restrict__ order, bool leaves_newer,
+                                                 uint32_t ni, uint32_t call, uint32_t* __restrict__ flag,
+                                                 uint32_t* __restrict__ info)
 {
-    const uint32_t most = turns[0], tops = turns[1];
-    const bool newer = leaves_newer && turns[2] >= kRefStack;
-    if (most < kRefPending && !newer) return;
-    if (tops > kMaxTops || newer) {
+    const uint32_t most = turns[0], tops = most < kRefPending ? 0u : turns[1];
+    const bool deep = turns[2] >= kRefStack;
+    if (tops > kMaxTops || (leaves_newer && deep)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *flag = call;
         return;
     }
+    if (tops == 0 && !(Count && deep)) return;
+    const bool sym = Count && EE && info && sym_serves(info, ni + 1);
     const uint32_t lane = lane_id(), n_round = (n_queries + 31u) & ~31u;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_round; t += gridDim.x * blockDim.x) {
         float box[6], all[6];
         box[0] = box[1] = box[2] = __int_as_float(0x7f800000);
         box[3] = box[4] = box[5] = __int_as_float(0xff800000);
-        if (t < n_queries) query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, order ? __ldg(&order[t]) : t, box);
+        const uint32_t q = t < n_queries && order ? __ldg(&order[t]) : t;
+        if (t < n_queries) query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
+        if (Count && deep) {
+            float cull[6] = {box[0], box[1], box[2], box[3], box[4], box[5]};
+            if (EE && (sym || !dhat) && t < n_queries) {  // what the once-per-pair walk culls with
+                const SymQuery Q = sym ? sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, from_ordered(info[1]),
+                                                         fabsf(from_ordered(info[2])), q)
+                                       : sym_query<false>(x0, x1, edges, uniform_r, nullptr, nullptr, 0.0f, 0.0f, q);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            all[c] = box[c];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float v = __shfl_xor_sync(0xFFFFFFFFu, all[c], o);
-                all[c] = c < 3 ? fminf(all[c], v) : fmaxf(all[c], v);
+                for (int c = 0; c < 6; ++c) cull[c] = Q.cull[c];
             }
+            warp_union(cull, all);
+            if (exceeds(wide, ni, all, false) && exceeds(wide, ni, cull, true)) {
+                if (sym) atomicOr(&info[0], 1u);
+                if (!sym || exceeds(wide, ni, box, true)) *flag = call;
+            }
+            __syncwarp();
         }
+        warp_union(box, all);
         for (uint32_t k0 = 0; k0 < tops; k0 += 32) {
             uint32_t top = 0;
             bool near = false;
@@ -951,9 +925,72 @@ __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide
     }
 }
 
+// query_template2 as the reference runs it (lbvh.cpp:293-360) on the binary records, for calls in
+// which the stack may fill (see Early): a stack of 32 inner nodes starting at the root, the two
+// children tested in order (left, then right) and the right one popped first; an inner child that meets a
+// full stack ends the whole query (the pairs found so far stay), and so does the 100001st popped node.
+// Both early exits are reported through `capped`.  EE keeps the reference's eid < adj filter.
+// Below kPacketLeaves queries it is the other branch of the wide walks' kernels, which saves the calls that do not need it,
+// nearly all, a launch; from there on a kernel of its own, with half their registers and so twice their warps in flight.
 template <bool EE>
-__global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4, uint32_t n_leaves,
-                                               const float4* __restrict__ x0, const float4* __restrict__ x1,
+__device__ __forceinline__ void query_ref(const float4* __restrict__ wide, const float4* __restrict__ x0,
+                                          const float4* __restrict__ x1, const uint2* __restrict__ edges, uint32_t n_queries,
+                                          const float* __restrict__ dhat, const float* __restrict__ thickness, float uniform_r,
+                                          uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count, uint32_t* capped)
+{
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n_queries; q += gridDim.x * blockDim.x) {
+        float box[6];
+        query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
+        uint32_t stack[kRefStack];
+        int sp = 0;
+        uint32_t loop = 0;
+        stack[sp++] = 0;
+        while (sp > 0) {
+            const uint32_t node = stack[--sp];
+            const float4* rec = wide + 4 * node;
+            bool stop = false;
+            uint2 hit[2];
+            uint32_t nhit = 0;
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                float4 mn, mx;
+                ld_slot(rec + 2 * side, mn, mx);
+                if (!stop && overlap(mn, mx, box)) {
+                    const uint32_t code = __float_as_uint(mn.w);
+                    if (code & 0x80000000u) {
+                        const uint32_t obj = code & 0x7FFFFFFFu;
+                        if (!EE || q < obj) hit[nhit++] = make_uint2(q, obj);
+                    } else if (sp < (int)kRefStack) {
+                        stack[sp++] = code;
+                    } else {
+                        stop = true;  // lbvh.cpp:344-351: the whole query ends here
+                    }
+                }
+            }
+            emit_pairs(hit, nhit, pairs, capacity, d_count);
+            if (stop || ++loop > 100000u) {
+                if (capped) atomicOr(capped, 1u);
+                break;
+            }
+        }
+    }
+}
+
+template <bool EE>
+__global__ void __launch_bounds__(128) k_query_ref(const float4* __restrict__ wide, const float4* __restrict__ x0,
+                                                   const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                   uint32_t n_queries, const float* __restrict__ dhat,
+                                                   const float* __restrict__ thickness, float uniform_r,
+                                                   uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count,
+                                                   uint32_t* capped, const Early early)
+{
+    if (early()) query_ref<EE>(wide, x0, x1, edges, n_queries, dhat, thickness, uniform_r, pairs, capacity, d_count, capped);
+}
+
+// The queries of a call, each by its own box (wide: the binary records, or null where k_query_ref serves marked calls)
+template <bool EE>
+__global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide, const float4* __restrict__ wide4,
+                                               uint32_t n_leaves, const float4* __restrict__ x0, const float4* __restrict__ x1,
                                                const uint2* __restrict__ edges, uint32_t n_queries,
                                                const float* __restrict__ dhat, const float* __restrict__ thickness,
                                                uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count,
@@ -961,7 +998,10 @@ __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4,
                                                const Early early,
                                                const uint32_t* __restrict__ sym_info)
 {
-    if (early()) return;
+    if (early()) {
+        if (wide) query_ref<EE>(wide, x0, x1, edges, n_queries, dhat, thickness, 0.0f, pairs, capacity, d_count, capped);
+        return;
+    }
     if (EE && sym_info && sym_serves(sym_info, n_leaves)) return;  // k_query_ee_sym<true> serves the call
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_queries; t += gridDim.x * blockDim.x) {
         // queries in the order of `order` (the tree's Morton order when the queries are its own
@@ -1000,58 +1040,6 @@ __global__ void __launch_bounds__(128) k_query(const float4* __restrict__ wide4,
             emit_pairs(hit, nhit, pairs, capacity, d_count);
             if (stop || ++loop > 100000u) {  // the reference's early exits; reported so callers know the
                 if (capped) atomicOr(capped, 1u);  // list may lack pairs a complete traversal would find
-                break;
-            }
-        }
-    }
-}
-
-// query_template2 as the reference runs it (lbvh.cpp:293-360) on the binary records, for calls in
-// which the stack may fill (see Early): a stack of 32 inner nodes starting at the root, the two
-// children tested in order (left, then right) and the right one popped first; an inner child that meets a
-// full stack ends the whole query (the pairs found so far stay), and so does the 100001st popped node.
-// Both early exits are reported through `capped`.  EE keeps the reference's eid < adj filter.
-template <bool EE>
-__global__ void __launch_bounds__(128) k_query_ref(const float4* __restrict__ wide, const float4* __restrict__ x0,
-                                                   const float4* __restrict__ x1, const uint2* __restrict__ edges,
-                                                   uint32_t n_queries, const float* __restrict__ dhat,
-                                                   const float* __restrict__ thickness, float uniform_r,
-                                                   uint2* __restrict__ pairs, uint32_t capacity, uint32_t* d_count,
-                                                   uint32_t* capped, const Early early)
-{
-    if (!early()) return;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n_queries; q += gridDim.x * blockDim.x) {
-        float box[6];
-        query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
-        uint32_t stack[kRefStack];
-        int sp = 0;
-        uint32_t loop = 0;
-        stack[sp++] = 0;
-        while (sp > 0) {
-            const uint32_t node = stack[--sp];
-            const float4* rec = wide + 4 * node;
-            bool stop = false;
-            uint2 hit[2];
-            uint32_t nhit = 0;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                float4 mn, mx;
-                ld_slot(rec + 2 * side, mn, mx);
-                if (!stop && overlap(mn, mx, box)) {
-                    const uint32_t code = __float_as_uint(mn.w);
-                    if (code & 0x80000000u) {
-                        const uint32_t obj = code & 0x7FFFFFFFu;
-                        if (!EE || q < obj) hit[nhit++] = make_uint2(q, obj);
-                    } else if (sp < (int)kRefStack) {
-                        stack[sp++] = code;
-                    } else {
-                        stop = true;  // lbvh.cpp:344-351: the whole query ends here
-                    }
-                }
-            }
-            emit_pairs(hit, nhit, pairs, capacity, d_count);
-            if (stop || ++loop > 100000u) {
-                if (capped) atomicOr(capped, 1u);
                 break;
             }
         }
@@ -1143,7 +1131,7 @@ __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wi
 // {node, the lanes it overlaps} in shared memory: a record is then one broadcast line for the warp instead of up to 32
 // scattered ones, no lane waits for another's longer walk, and the pairs leave in runs.  Each lane still counts its own
 // steps.
-// Static and swept queries of two sheets of 448 x 448 vertices with a thickness: 12.9 ms as k_query_ref, 8.6 ms so; of
+// Static and swept queries of two sheets of 448 x 448 vertices with a thickness: 12.9 ms as query_ref, 8.6 ms so; of
 // 212 x 212 vertices of thickness 0: 2.3 and 1.3 ms.
 template <bool PerEdge>
 __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__ wide4, const uint32_t* __restrict__ sgo,
@@ -1230,13 +1218,14 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
 
 // The same walk with one radius, one query per thread, for trees that leave most of the GPU's warps idle: a warp's union
 // of paths is longer than its longest path, which is what the time is there.
-__global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restrict__ wide4, const uint32_t* __restrict__ sgo,
-                                                           uint32_t n_leaves, const float4* __restrict__ x0,
+__global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restrict__ wide, const float4* __restrict__ wide4,
+                                                           const uint32_t* __restrict__ sgo, uint32_t n_leaves, const float4* __restrict__ x0,
                                                            const float4* __restrict__ x1, const uint2* __restrict__ edges,
                                                            float uniform_r, uint2* __restrict__ pairs, uint32_t capacity,
                                                            uint32_t* d_count, uint32_t* capped, const Early early)
 {
-    if (early()) return;  // k_query_ref<true> (the full EE walk) instead
+    if (early())
+        return query_ref<true>(wide, x0, x1, edges, n_leaves, nullptr, nullptr, uniform_r, pairs, capacity, d_count, capped);
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_leaves; t += gridDim.x * blockDim.x) {
         const uint32_t q = __ldg(&sgo[t]);
         const SymQuery Q = sym_query<false>(x0, x1, edges, uniform_r, nullptr, nullptr, 0.0f, 0.0f, q);
@@ -1625,7 +1614,7 @@ static uint32_t next_call(const lcs_bvh* t)
     return call ? call : __atomic_add_fetch(&t->calls, 1u, __ATOMIC_RELAXED);  // 0 marks nothing
 }
 
-// k_may_end and k_may_exceed of a call, and their answer
+// k_may_end of a call, and its answer
 template <bool EE>
 static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const float* x1, const uint32_t* edges, uint32_t n,
                        const float* dhat, const float* thickness, float uniform_r, const uint32_t* order, uint32_t* info,
@@ -1635,13 +1624,9 @@ static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const f
     const uint2* e2 = reinterpret_cast<const uint2*>(edges);
     uint32_t* flag = t->early + call % kSymSlots;
     if (t->ni > 0) {
-        k_may_end<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, p0, p1, e2, n, dhat, thickness,
-                                                      uniform_r, order, t->leaves_newer, call, flag);
-        lcs_count_launch();
-    }
-    if (t->ni > kRefNodes) {
-        k_may_exceed<EE><<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->ni, p0, p1, e2, n, dhat, thickness, uniform_r, order,
-                                                         t->turns, call, flag, info);
+        const auto ask = t->ni > kRefNodes ? k_may_end<EE, true> : k_may_end<EE, false>;
+        ask<<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, p0, p1, e2, n, dhat, thickness, uniform_r,
+                                             order, t->leaves_newer, t->ni, call, flag, info);
         lcs_count_launch();
     }
     return Early{flag, call};
@@ -1664,14 +1649,17 @@ int lcs_bvh_query_vf_capped(const lcs_bvh* t, const float* x0, const float* x1, 
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_vf: the tree has not been constructed");
     const Early early = ask_early<false>(t, next_call(t), x0, x1, nullptr, n_verts, d_hat, thickness, 0.0f, nullptr, nullptr,
                                          (cudaStream_t)stream);
-    k_query<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-        t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts,
-        d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity, d_count, nullptr, capped, early, nullptr);
+    cudaStream_t s = (cudaStream_t)stream;
+    const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
+    const int grid = grid_for(n_verts, 128, 16);
+    uint2* out = reinterpret_cast<uint2*>(pairs);
+    const bool apart = n_verts >= kPacketLeaves;
+    k_query<false><<<grid, 128, 0, s>>>(apart ? nullptr : t->wide, t->wide4, t->n, p0, p1, nullptr, n_verts, d_hat, thickness,
+                                        out, capacity, d_count, nullptr, capped, early, nullptr);
     lcs_count_launch();
-    if (t->ni > 0) {
-        k_query_ref<false><<<grid_for(n_verts, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-            t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1), nullptr, n_verts, d_hat,
-            thickness, 0.0f, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
+    if (apart) {
+        k_query_ref<false><<<grid, 128, 0, s>>>(t->wide, p0, p1, nullptr, n_verts, d_hat, thickness, 0.0f, out, capacity,
+                                                d_count, capped, early);
         lcs_count_launch();
     }
     LCS_LAUNCH_CHECK();
@@ -1717,16 +1705,15 @@ int lcs_bvh_query_ee_capped(const lcs_bvh* t, const float* x0, const float* x1, 
                                                                         capacity, d_count, capped, early);
         lcs_count_launch();
     }
-    k_query<true><<<grid_for(n_edges, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-        t->wide4, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-        reinterpret_cast<const uint2*>(edges), n_edges, d_hat, thickness, reinterpret_cast<uint2*>(pairs), capacity,
-        d_count, n_edges == t->n ? t->sgo : nullptr, capped, early, info);
+    const int grid = grid_for(n_edges, 128, 16);
+    uint2* out = reinterpret_cast<uint2*>(pairs);
+    const bool apart = n_edges >= kPacketLeaves;
+    k_query<true><<<grid, 128, 0, s>>>(apart ? nullptr : t->wide, t->wide4, t->n, p0, p1, e2, n_edges, d_hat, thickness, out,
+                                       capacity, d_count, n_edges == t->n ? t->sgo : nullptr, capped, early, info);
     lcs_count_launch();
-    if (t->ni > 0) {
-        k_query_ref<true><<<grid_for(n_edges, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-            t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-            reinterpret_cast<const uint2*>(edges), n_edges, d_hat, thickness, 0.0f, reinterpret_cast<uint2*>(pairs),
-            capacity, d_count, capped, early);
+    if (apart) {
+        k_query_ref<true><<<grid, 128, 0, s>>>(t->wide, p0, p1, e2, n_edges, d_hat, thickness, 0.0f, out, capacity, d_count,
+                                               capped, early);
         lcs_count_launch();
     }
     LCS_LAUNCH_CHECK();
@@ -1751,23 +1738,22 @@ int lcs_bvh_query_ee_sym_capped(const lcs_bvh* t, const float* x0, const float* 
     if (!t->built) return lcs_fail(LCS_ERR_INVALID, "lcs_bvh_query_ee_sym: the tree has not been constructed");
     const Early early = ask_early<true>(t, next_call(t), x0, x1, edges, t->n, nullptr, nullptr, d_hat, t->sgo, nullptr,
                                         (cudaStream_t)stream);
-    if (t->n >= kPacketLeaves)
-        k_query_ee_sym<false><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-            t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-            reinterpret_cast<const uint2*>(edges), d_hat, nullptr, nullptr, nullptr, reinterpret_cast<uint2*>(pairs), capacity,
-            d_count, capped, early);
-    else
-        k_query_ee_sym_lane<<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-            t->wide4, t->sgo, t->n, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-            reinterpret_cast<const uint2*>(edges), d_hat, reinterpret_cast<uint2*>(pairs), capacity, d_count, capped, early);
-    lcs_count_launch();
-    if (t->ni > 0) {  // a call in which the stack may fill: the reference's full EE walk (its early exits break the symmetry)
-        k_query_ref<true><<<grid_for(t->n, 128, 16), 128, 0, (cudaStream_t)stream>>>(
-            t->wide, reinterpret_cast<const float4*>(x0), reinterpret_cast<const float4*>(x1),
-            reinterpret_cast<const uint2*>(edges), t->n, nullptr, nullptr, d_hat, reinterpret_cast<uint2*>(pairs),
-            capacity, d_count, capped, early);
+    cudaStream_t s = (cudaStream_t)stream;
+    const float4 *p0 = reinterpret_cast<const float4*>(x0), *p1 = reinterpret_cast<const float4*>(x1);
+    const uint2* e2 = reinterpret_cast<const uint2*>(edges);
+    uint2* out = reinterpret_cast<uint2*>(pairs);
+    const int grid = grid_for(t->n, 128, 16);
+    if (t->n >= kPacketLeaves) {
+        k_query_ee_sym<false><<<grid, 128, 0, s>>>(t->wide4, t->sgo, t->n, p0, p1, e2, d_hat, nullptr, nullptr, nullptr, out,
+                                                   capacity, d_count, capped, early);
         lcs_count_launch();
+        k_query_ref<true><<<grid, 128, 0, s>>>(t->wide, p0, p1, e2, t->n, nullptr, nullptr, d_hat, out, capacity, d_count,
+                                               capped, early);
+    } else {
+        k_query_ee_sym_lane<<<grid, 128, 0, s>>>(t->wide, t->wide4, t->sgo, t->n, p0, p1, e2, d_hat, out, capacity, d_count,
+                                                 capped, early);
     }
+    lcs_count_launch();
     LCS_LAUNCH_CHECK();
     return LCS_OK;
 }

@@ -646,3 +646,26 @@ def test_queries_of_more_than_a_hundred_thousand_nodes(kind_name, n_pairs, once)
     bvh.broad_phase_query_from_verts(xd, dev(x1), cnt, pairs, dev(r), dev(z))
     assert int(counts(cnt)[0]) == n_want
     np.testing.assert_array_equal(SC.sorted_pairs(host(pairs, np.uint32)[:n_want]), SC.sorted_pairs(want))
+
+
+def test_queries_of_small_scenes_take_two_launches():
+    """The question whether a walk may end early and the walk itself, which holds both ways of walking."""
+    lib = A.load()
+    x, el = _sheet(30)
+    th, dh = np.zeros(len(x), np.float32), np.full(len(x), 1e-3, np.float32)
+    _, edges = _edge_trees(x, el, th)
+    quads = el.reshape(-1, 2)[:400]
+    fa = np.concatenate([quads, np.roll(quads, 1, 0)], 1).astype(np.uint32)
+    faces = LBVH(O.TREE_FACE, len(fa))
+    xd, fd, ed = dev(x), dev(fa), dev(el)
+    faces.reduce_face_tree_aabb(xd, fd)
+    faces.construct_tree()
+    faces.update_and_refit(dev(th), xd, xd, fd)
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pairs = torch.zeros((200000, 2), dtype=torch.int32, device="cuda")
+    for query in (lambda: faces.broad_phase_query_from_verts(xd, xd, cnt, pairs, dev(dh), dev(th)),
+                  lambda: edges.broad_phase_query_from_edges(xd, xd, ed, cnt, pairs, dev(dh), dev(th)),
+                  lambda: edges.broad_phase_query_from_edges_sym(xd, xd, ed, cnt, pairs, 1e-3)):
+        before = lib.lcs_launch_count()
+        query()
+        assert lib.lcs_launch_count() - before == 2
