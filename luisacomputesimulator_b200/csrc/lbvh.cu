@@ -61,10 +61,11 @@ struct lcs_bvh {
     float4* seg_box = nullptr;       // 2 per 32 union-order positions (whole refit chunks): {min | 0}{max | 0}
     float4* chunk_box = nullptr;     // 2 per refit chunk: its union
     uint32_t* healthy = nullptr;     // 1
-    uint32_t* turns = nullptr;       // 3 + kMaxTops: see k_depth_parity
-    uint32_t* top_lefts = nullptr;   // 32 * kMaxTops: slots of the 31 inner left siblings above each listed top
+    uint32_t max_tops = 0;           // tops are disjoint and hold two leaves each: at most n / 2, and kMaxTops
+    uint32_t* turns = nullptr;       // 3 + max_tops: see k_depth_parity
+    uint32_t* top_lefts = nullptr;   // 32 * max_tops: slots of the 31 inner left siblings above each listed top
     uint32_t* early = nullptr;       // kSymSlots: number of the query call that may end early, a slot per call in turn
-    uint32_t* sym_info = nullptr;    // kSymSlots x kSymWords: k_sym_check's findings, a slot per query call in turn
+    uint32_t* sym_info = nullptr;    // (edge trees of kSymEdges leaves and more) kSymSlots x kSymWords: k_sym_check's findings, a slot per query call in turn
     mutable uint32_t calls = 0;
     bool leaves_newer = false;       // leaf boxes were written after the last refit (the binary records alone hold them)
     bool built = false;              // a construct has written the topology, slots and refit tables
@@ -248,13 +249,13 @@ __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* _
 // It also counts, for each inner node, the nodes that a walk of the reference can at most have pending when it pops it:
 // one for every ancestor whose second child the path takes and whose first child is an inner node.  turns: [0] the
 // largest count, [1] how many nodes reach kRefPending by their own turn (every node with as many descends from one of
-// them), [2] the depth of the deepest inner node, [3...] the slots of the first kMaxTops of those that reach kRefPending,
+// them), [2] the depth of the deepest inner node, [3...] the slots of the first max_tops of those that reach kRefPending,
 // whose 31 inner left siblings top_lefts lists.
 constexpr uint32_t kRefStack = 32;
 constexpr uint32_t kRefPending = kRefStack - 1;
 
 __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* __restrict__ children, uint32_t ni,
-                               uint8_t* __restrict__ even, uint32_t* __restrict__ turns,
+                               uint8_t* __restrict__ even, uint32_t max_tops, uint32_t* __restrict__ turns,
                                uint32_t* __restrict__ top_lefts)
 {
     uint32_t most = 0, deepest = 0;
@@ -277,7 +278,7 @@ __global__ void k_depth_parity(const uint32_t* __restrict__ slot, const uint2* _
         deepest = d > deepest ? d : deepest;
         if (own && pending == kRefPending) {
             const uint32_t k = atomicAdd(&turns[1], 1u);
-            if (k < kMaxTops) {
+            if (k < max_tops) {
                 turns[3 + k] = slot[nid];
                 uint32_t i = 0;
                 for (p = nid; p != 0u && i < kRefPending;) {
@@ -1404,10 +1405,11 @@ extern "C" int lcs_bvh_create(int kind, uint32_t n_leaves, lcs_bvh** out)
     A(alloc(h->seg_box, 2 * chunks * kRefitSegs));
     A(alloc(h->chunk_box, 2 * chunks));
     A(alloc(h->healthy, 1));
-    A(alloc(h->turns, 3 + kMaxTops));
-    A(alloc(h->top_lefts, 32 * kMaxTops));
+    h->max_tops = std::min(kMaxTops, n_leaves / 2);
+    A(alloc(h->turns, 3 + h->max_tops));
+    A(alloc(h->top_lefts, 32 * h->max_tops));
     A(alloc(h->early, kSymSlots));
-    if (kind == LCS_TREE_EDGE) A(alloc(h->sym_info, kSymWords * kSymSlots));
+    if (kind == LCS_TREE_EDGE && n_leaves >= kSymEdges) A(alloc(h->sym_info, kSymWords * kSymSlots));
     if (e == cudaSuccess) e = cudaMemset(h->turns, 0, 3 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(h->early, 0, kSymSlots * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(h->span_count, 0, sizeof(uint32_t));
@@ -1498,7 +1500,7 @@ extern "C" int lcs_bvh_construct(lcs_bvh* h, lcs_stream stream)
         lcs_count_launch();
         k_check<<<gi, 256, 0, s>>>(h->children, h->parent, h->ni, h->healthy);
         lcs_count_launch();
-        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->turns, h->top_lefts);
+        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->max_tops, h->turns, h->top_lefts);
         lcs_count_launch();
         LCS_CUDA_TRY(union_order(h, s));
     } else {
@@ -1541,7 +1543,7 @@ int lcs_bvh_construct_host_sort(lcs_bvh* h, lcs_stream stream)
         lcs_count_launch();
         k_check<<<gi, 256, 0, s>>>(h->children, h->parent, h->ni, h->healthy);
         lcs_count_launch();
-        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->turns, h->top_lefts);
+        k_depth_parity<<<gi, 256, 0, s>>>(h->slot, h->children, h->ni, h->even, h->max_tops, h->turns, h->top_lefts);
         lcs_count_launch();
         LCS_CUDA_TRY(union_order(h, s));
     }

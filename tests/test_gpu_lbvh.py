@@ -669,3 +669,13 @@ def test_queries_of_small_scenes_take_two_launches():
         before = lib.lcs_launch_count()
         query()
         assert lib.lcs_launch_count() - before == 2
+
+
+def test_small_trees_hold_little_memory():
+    """A tree's memory goes by its leaves: 100 trees of 500 faces, 41 KB each for the boxes and topology and 34 KB for the
+    parts where a walk may end early, fit 20 MB."""
+    LBVH(O.TREE_FACE, 500)
+    free = torch.cuda.mem_get_info()[0]
+    trees = [LBVH(O.TREE_FACE, 500) for _ in range(100)]
+    assert free - torch.cuda.mem_get_info()[0] <= 20 << 20
+    del trees
