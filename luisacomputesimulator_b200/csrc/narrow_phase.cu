@@ -6,6 +6,7 @@
 // can stay on the device (no host read-back between broad and narrow phase).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <new>
 
 #include "lcs_common.cuh"
@@ -424,8 +425,8 @@ __global__ void k_segments(const uint64_t* __restrict__ keys, const uint32_t* __
 // The (row, column, triplet) order of the contact triplets without a global radix sort (pairs without affine
 // bodies): the 12 directed vertex pairs of every contact pair are bucketed by row (a count, a scan and a
 // scatter with per-row cursors), and each entry finds its place in its row's bucket by counting the entries
-// that precede it in (column, triplet index) order -- the order the stable radix sort gives.  Rows hold at
-// most a few hundred entries.  k_heads, k_segments and k_row_ptr then run on the result as after the sort.
+// that precede it in (column, triplet index) order -- the order the stable radix sort gives.  Most rows hold at
+// most a few hundred entries; a vertex that many others touch has thousands.  k_heads, k_segments and k_row_ptr then run on the result as after the sort.
 __global__ void k_row_count(const lcs_pair* __restrict__ pairs, const uint32_t* d_count, uint32_t cap,
                             uint32_t* __restrict__ rcnt)
 {
@@ -438,9 +439,12 @@ __global__ void k_row_count(const lcs_pair* __restrict__ pairs, const uint32_t* 
     }
 }
 
+// entries of a row that k_row_rank takes with one warp; *any_long is set if a row has more
+constexpr uint32_t kRankCap = 512, kRankWarps = 8;
+
 __global__ void k_row_scatter(const lcs_pair* __restrict__ pairs, const uint32_t* d_count, uint32_t cap, int bits,
                               const uint32_t* __restrict__ rstart, uint32_t* __restrict__ rcur,
-                              uint64_t* __restrict__ tkeys, uint32_t* __restrict__ tvals)
+                              uint64_t* __restrict__ tkeys, uint32_t* __restrict__ tvals, uint32_t* __restrict__ any_long)
 {
     const uint32_t n = pair_count(d_count, cap);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -448,7 +452,8 @@ __global__ void k_row_scatter(const lcs_pair* __restrict__ pairs, const uint32_t
         if (!P.type) continue;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t base = rstart[P.v[i]] + atomicAdd(&rcur[P.v[i]], 3u);
+            const uint32_t before = atomicAdd(&rcur[P.v[i]], 3u), base = rstart[P.v[i]] + before;
+            if (before <= kRankCap && before + 3u > kRankCap) *any_long = 1u;
             uint32_t t = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -462,54 +467,80 @@ __global__ void k_row_scatter(const lcs_pair* __restrict__ pairs, const uint32_t
 }
 
 // A warp takes `rows` rows (at most 31), one after the other: the row's entries as (column, triplet) words in shared
-// memory, each lane counting the words below its own, two at a time.  Rows beyond kRankCap entries count from global memory.  One thread per entry over
-// 64-bit keys in global memory was bound by the latency of its serial loads: 401,408 vertices with 476,000 pairs 982 us,
-// 366 us so; 5,000 with 4,348 pairs 34 and 16.
-constexpr uint32_t kRankCap = 512, kRankWarps = 8;
+// memory, each lane counting the words below its own, two at a time.  One thread per entry over 64-bit keys in global
+// memory was bound by the latency of its serial loads: 401,408 vertices with 476,000 pairs 982 us, 366 us so; 5,000 with
+// 4,348 pairs 34 and 16.
+// The entries of rows beyond kRankCap, if there are any, are then dealt out to all warps, 32 at a time, each of which counts
+// through the whole row in pieces of kRankCap words, so that the GPU shares a work that grows by the square of the length
+// (an assembly with a row of 15,000 entries 0.26 ms, of 30,000 0.54; by one warp 342 ms and 1.4 s, by a thread per entry 1.3
+// and 2.6 ms).
+__device__ __forceinline__ uint32_t count_below(const unsigned long long* word, uint32_t len, unsigned long long mine)
+{
+    uint32_t rank = 0;
+#pragma unroll 8
+    for (uint32_t q = 0; q < len; q += 2) {
+        const ulonglong2 two = *reinterpret_cast<const ulonglong2*>(word + q);
+        rank += (two.x < mine ? 1u : 0u) + (two.y < mine ? 1u : 0u);
+    }
+    return rank;
+}
 
-__global__ void __launch_bounds__(32 * kRankWarps) k_row_rank(uint32_t n_rows, uint32_t rows, const uint32_t* __restrict__ rstart, int bits,
+__global__ void __launch_bounds__(32 * kRankWarps) k_row_rank(uint32_t n_rows, uint32_t rows,
+                                                              const uint32_t* __restrict__ rstart, int bits,
                                                               const uint64_t* __restrict__ tkeys,
                                                               const uint32_t* __restrict__ tvals, uint64_t* __restrict__ keys,
-                                                              uint32_t* __restrict__ vals, uint32_t* d_n)
+                                                              uint32_t* __restrict__ vals, uint32_t* d_n,
+                                                              const uint32_t* __restrict__ any_long)
 {
     __shared__ __align__(16) unsigned long long s_word[kRankWarps][kRankCap + 2];
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
     const uint64_t cmask = (1ull << bits) - 1ull;
     if (blockIdx.x == 0 && threadIdx.x == 0) *d_n = rstart[n_rows];
     unsigned long long* word = s_word[w];
+    auto word_of = [&](uint32_t e) { return ((unsigned long long)(tkeys[e] & cmask) << 32) | tvals[e]; };
+    // `len` words of the row from entry lo on
+    auto stage = [&](uint32_t lo, uint32_t len) {
+        for (uint32_t e = lane; e < len; e += 32) word[e] = word_of(lo + e);
+        if (lane == 0) word[len] = ~0ull;  // an odd row's partner, below nothing
+        __syncwarp();
+    };
     for (uint32_t r0 = (blockIdx.x * kRankWarps + w) * rows; r0 < n_rows; r0 += gridDim.x * kRankWarps * rows) {
         const uint32_t start = lane <= rows ? rstart[min(r0 + lane, n_rows)] : 0u;
         for (uint32_t j = 0; j < rows; ++j) {
-            const uint32_t lo = __shfl_sync(0xFFFFFFFFu, start, j), hi = __shfl_sync(0xFFFFFFFFu, start, j + 1);
-            const uint32_t len = hi - lo;
-            if (len == 0) continue;
+            const uint32_t lo = __shfl_sync(0xFFFFFFFFu, start, j), len = __shfl_sync(0xFFFFFFFFu, start, j + 1) - lo;
+            if (len == 0 || len > kRankCap) continue;
             const uint64_t row = (uint64_t)(r0 + j) << bits;
-            auto word_of = [&](uint32_t e) { return ((unsigned long long)(tkeys[e] & cmask) << 32) | tvals[e]; };
-            if (len <= kRankCap) {
-                for (uint32_t e = lane; e < len; e += 32) word[e] = word_of(lo + e);
-                if (lane == 0) word[len] = ~0ull;  // an odd row's partner, below nothing
+            stage(lo, len);
+            for (uint32_t e = lane; e < len; e += 32) {
+                const unsigned long long mine = word[e];
+                const uint32_t rank = count_below(word, len, mine);
+                keys[lo + rank] = row | (uint64_t)(mine >> 32);
+                vals[lo + rank] = (uint32_t)mine;
+            }
+            __syncwarp();
+        }
+    }
+    if (*any_long == 0u) return;
+    const uint32_t n = rstart[n_rows];
+    for (uint32_t e0 = 32u * (blockIdx.x * kRankWarps + w); e0 < n; e0 += 32u * kRankWarps * gridDim.x) {
+        const uint32_t e = e0 + lane, row = e < n ? (uint32_t)(tkeys[e] >> bits) : 0u;
+        const uint32_t lo = rstart[row], hi = rstart[row + 1];
+        const unsigned long long mine = e < n ? word_of(e) : 0ull;
+        bool todo = e < n && hi - lo > kRankCap;
+        for (uint32_t m; (m = __ballot_sync(0xFFFFFFFFu, todo)) != 0u;) {  // the 32 entries may touch several rows
+            const int src = __ffs(m) - 1;
+            const uint32_t rlo = __shfl_sync(0xFFFFFFFFu, lo, src), rhi = __shfl_sync(0xFFFFFFFFu, hi, src);
+            uint32_t rank = 0;
+            for (uint32_t at = rlo; at < rhi; at += kRankCap) {
+                const uint32_t len = min(kRankCap, rhi - at);
+                stage(at, len);
+                rank += count_below(word, len, mine);
                 __syncwarp();
-                for (uint32_t e = lane; e < len; e += 32) {
-                    const unsigned long long mine = word[e];
-                    uint32_t rank = 0;
-#pragma unroll 8
-                    for (uint32_t q = 0; q < len; q += 2) {
-                        const ulonglong2 two = *reinterpret_cast<const ulonglong2*>(word + q);
-                        rank += (two.x < mine ? 1u : 0u) + (two.y < mine ? 1u : 0u);
-                    }
-                    keys[lo + rank] = row | (uint64_t)(mine >> 32);
-                    vals[lo + rank] = (uint32_t)mine;
-                }
-                __syncwarp();
-            } else {
-                for (uint32_t e = lane; e < len; e += 32) {
-                    const unsigned long long mine = word_of(lo + e);
-                    uint32_t rank = 0;
-#pragma unroll 4
-                    for (uint32_t q = lo; q < hi; ++q) rank += word_of(q) < mine ? 1u : 0u;
-                    keys[lo + rank] = row | (uint64_t)(mine >> 32);
-                    vals[lo + rank] = (uint32_t)mine;
-                }
+            }
+            if (todo && lo == rlo) {
+                keys[lo + rank] = ((uint64_t)row << bits) | (uint64_t)(mine >> 32);
+                vals[lo + rank] = (uint32_t)mine;
+                todo = false;
             }
         }
     }
@@ -542,7 +573,8 @@ struct lcs_assembler {
     uint32_t *d_ntrip = nullptr, *d_nnzb = nullptr;
     uint32_t *row_ptr = nullptr, *col = nullptr, *brow = nullptr;
     float* val = nullptr;
-    // row bucketing (pairs without affine bodies): per-row counts / starts / cursors, n_rows + 1 each
+    // row bucketing (pairs without affine bodies): per-row counts / starts / cursors, n_rows + 1 each; one
+    // word behind the cursors: a row has more than kRankCap entries
     uint32_t *rcnt = nullptr, *rstart = nullptr, *rcur = nullptr, *d_rows1 = nullptr;
     uint32_t* rscan_tmp = nullptr;
 };
@@ -580,7 +612,7 @@ int assembler_create(uint32_t n_rows, uint32_t pair_capacity, bool abd, lcs_asse
     const size_t R1 = (size_t)n_rows + 1;
     A((void**)&a->rcnt, 4 * R1);
     A((void**)&a->rstart, 4 * R1);
-    A((void**)&a->rcur, 4 * R1);
+    A((void**)&a->rcur, 4 * (R1 + 1));
     A((void**)&a->d_rows1, 4);
     A((void**)&a->rscan_tmp, 4 * scan::tmp_words((uint32_t)R1));
     if (e == cudaSuccess) {
@@ -642,7 +674,8 @@ int offdiag_bsr(lcs_assembler* a, const lcs_pair* pairs, const uint32_t* d_count
     if (!abd) {  // row bucketing: count, scan, scatter, rank within the row
         const uint32_t R1 = a->n_rows + 1;
         LCS_CUDA_TRY(cudaMemsetAsync(a->rcnt, 0, 4 * (size_t)R1, s));
-        LCS_CUDA_TRY(cudaMemsetAsync(a->rcur, 0, 4 * (size_t)R1, s));
+        LCS_CUDA_TRY(cudaMemsetAsync(a->rcur, 0, 4 * ((size_t)R1 + 1), s));
+        uint32_t* any_long = a->rcur + R1;
         if (capacity) {
             k_row_count<<<grid_for(capacity, 256), 256, 0, s>>>(pairs, d_count, capacity, a->rcnt);
             lcs_count_launch();
@@ -650,13 +683,15 @@ int offdiag_bsr(lcs_assembler* a, const lcs_pair* pairs, const uint32_t* d_count
         scan::exclusive_u32(a->rcnt, a->rstart, a->d_rows1, R1, a->rscan_tmp, s);
         if (capacity) {
             k_row_scatter<<<grid_for(capacity, 256), 256, 0, s>>>(pairs, d_count, capacity, a->bits, a->rstart, a->rcur,
-                                                                   a->keys_alt, a->vals_alt);
+                                                                   a->keys_alt, a->vals_alt, any_long);
             lcs_count_launch();
         }
         // few rows: a warp each, so that the longest ones do not follow one another; many: four each, most of them empty
         const uint32_t rows = a->n_rows <= 32768 ? 1 : 4;
-        k_row_rank<<<(a->n_rows + kRankWarps * rows - 1) / (kRankWarps * rows), 32 * kRankWarps, 0, s>>>(
-            a->n_rows, rows, a->rstart, a->bits, a->keys_alt, a->vals_alt, a->keys, a->vals, a->d_ntrip);
+        // (two blocks per SM at least: the entries of long rows are dealt out to all)
+        const uint32_t blocks = std::max((a->n_rows + kRankWarps * rows - 1) / (kRankWarps * rows), 2u * kNumSMs);
+        k_row_rank<<<blocks, 32 * kRankWarps, 0, s>>>(a->n_rows, rows, a->rstart, a->bits, a->keys_alt, a->vals_alt, a->keys,
+                                                      a->vals, a->d_ntrip, any_long);
         lcs_count_launch();
         keys = a->keys;
         vals = a->vals;

@@ -201,3 +201,39 @@ def test_assembly_row_order_at_the_edges(n, shared):
     np.testing.assert_array_equal(host(g_rp, np.uint32), rp)
     np.testing.assert_array_equal(host(g_col, np.uint32), col)
     np.testing.assert_array_equal(host(g_val), val)
+
+
+def test_assembly_of_rows_that_thousands_of_pairs_share():
+    """Two vertices in 5,000 and 2,000 pairs (rows of 15,000 and 6,000 entries) among rows of a few: the order is the
+    oracle's, and all warps share the work (a row counted by one warp took over 40 ms)."""
+    n, shared = 20001, 5000
+    _, _, _, got, _ = _dcd("cloth_sphere")
+    rng = np.random.default_rng(1)
+    ms = {}
+    for apart in (True, False):
+        pairs = np.resize(got, shared)
+        bits = pairs["idx"] & np.uint32(0x80000000)
+        own = np.stack([rng.permutation(np.arange(c, n - 1, 4)) for c in range(4)], 1)
+        if not apart:
+            own[:, 0] = 0
+            own[1000:3000, 1] = n - 1
+        pairs["idx"] = own.astype(np.uint32) | bits
+        det = NarrowPhasesDetector(n, n)
+        assert len(pairs) <= det.cap_pairs
+        raw = torch.from_numpy(np.ascontiguousarray(pairs).view(np.uint8).copy()).cuda()
+        det.narrow_phase_list.view(torch.uint8).reshape(-1)[:raw.numel()] = raw
+        det.counts[2] = len(pairs)
+        det.device_assemble_contact_triplet()
+        rp, col, val = O.contact_offdiag_bsr(pairs, n)
+        g_rp, g_col, g_val = det.assembler.export(n, 12 * len(pairs))
+        np.testing.assert_array_equal(host(g_rp, np.uint32), rp)
+        np.testing.assert_array_equal(host(g_col, np.uint32), col)
+        np.testing.assert_array_equal(host(g_val), val)
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(5):
+            det.device_assemble_contact_triplet()
+        e1.record()
+        torch.cuda.synchronize()
+        ms[apart] = e0.elapsed_time(e1) / 5
+    assert ms[False] <= 20 * ms[True] + 1.0, ms
