@@ -252,7 +252,8 @@ struct FusedArgs {
     const float4* b;
     float4* x;
     float4 *r, *z, *p, *q, *minv;
-    double* part;        // 3 * gridDim
+    double* part;        // 3 * gridDim (k_pcg_small: 4)
+    uint64_t l2_bytes;   // of the device (set at the launch)
     unsigned* bar_count;
     unsigned* bar_gen;
     int max_iter;
@@ -345,11 +346,15 @@ __device__ __forceinline__ float3 mul3(const float4 m0, const float4 m1, const f
                        __fmaf_rn(m2.z, v.z, __fmaf_rn(m1.z, v.y, m0.z * v.x)));
 }
 
-// The persistent solve of systems beyond k_pcg_small.  Bound by HBM and L2 traffic, about 0.8 KB a row and iteration.
-// The matrix is larger than L2 here and is read once an iteration, so its loads ask L2 to evict them first: the vectors
-// and diagonal blocks then stay.  The step's x and r updates and the next preconditioner are one pass.
-// 401,322 rows (13 blocks each, FP64 dots): 6.44 ms with neither, 5.97 ms so; copies of the blocks to shared memory
-// (row_stage.cuh), which pay in k_pcg_batch's smaller blocks, took 8.4 ms against 1,024 threads that read directly.
+// The persistent solve of systems beyond k_pcg_small, whose passes over the vectors and the matrix (0.7 KB of HBM and 1.6 KB
+// of L2 traffic a row and iteration at 13 blocks a row) three grid barriers keep apart: 401,322 rows move 280 MB an iteration
+// from HBM at 3.5 TB/s and 660 MB from L2 at 8.4.  The step's x and r updates and the next preconditioner are one pass.
+// A matrix that does not fit L2 beside the vectors is read under evict_first, so that it does not push them out: 250,000
+// rows 3.71 ms, 4.39 without; 401,322 rows 5.96 and 6.24.  One that fits is read as it comes and stays: 88,800 rows 2.05 ms,
+// under evict_first 2.20.  The line is three quarters of L2: 148,000 rows (0.72 of it) take 2.56 and 2.57 ms, 160,000
+// (0.78) 3.00 and 3.19.  Copies of the blocks to shared memory (row_stage.cuh), which pay in k_pcg_batch's
+// smaller blocks, took 8.4 ms against 1,024 threads that read directly.
+constexpr uint64_t kRowBytes = 176;  // diag, minv and five vectors
 template <int G>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
 {
@@ -359,6 +364,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
     if (threadIdx.x == 0) s_fail = 0;
     const uint32_t n = a.n, w = threadIdx.x >> 5, lane = lane_id();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const bool stream = a.A.rp && 40ull * __ldg(&a.A.rp[n]) + kRowBytes * n > a.l2_bytes / 4 * 3;
     // the block's partial sums: one double per warp, added in warp order
     auto publish = [&](double v, int k) {
         v = warp_sum(v);
@@ -435,7 +441,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
         const uint32_t rows_round = (n + ngroups - 1) / ngroups * ngroups;
         for (uint32_t row = tid / G; row < rows_round; row += ngroups) {
             const uint32_t r = row < n ? row : n - 1;  // whole groups stay converged for the shuffles
-            const float3 qv = row_product<G, true>(r, lig, a.diag, a.A, a.B, a.p);
+            const float3 qv = stream ? row_product<G, true>(r, lig, a.diag, a.A, a.B, a.p)
+                                     : row_product<G>(r, lig, a.diag, a.A, a.B, a.p);
             if (row < n && lig == 0) {
                 a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
                 const float4 pv = __ldcg(&a.p[row]);
@@ -2765,6 +2772,10 @@ static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
         LCS_CUDA_TRY(cudaLaunchCooperativeKernel(bt == 256 ? (const void*)k_pcg_small<256> : (const void*)k_pcg_small<512>,
                                                  dim3(blocks), dim3(bt), args, 0, s));
     } else {
+        int dev = 0, l2 = 0;
+        LCS_CUDA_TRY(cudaGetDevice(&dev));
+        LCS_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+        a.l2_bytes = (uint64_t)l2;
         LCS_CUDA_TRY(cudaMemsetAsync(a.bar_count, 0, sizeof(unsigned), s));
         LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(grid), dim3(kFusedThreads), args, 0, s));
     }
