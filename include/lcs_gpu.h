@@ -365,6 +365,11 @@ LCS_API const lcs_pcg_stats* lcs_pcg_device_stats(const lcs_pcg* p);
  * the context stays usable. */
 LCS_API int lcs_debug_pcg_wait(int32_t which, int32_t missing_block, uint32_t blocks, uint32_t spin_limit,
                                lcs_stream stream);
+/* The same for the grid-wide sums of the persistent solve's small systems: `blocks` (2..32) blocks exchange values (device,
+ * two per block) twice; sums (device, 3): of the first values, of the second, of the second again in an exchange of its own.
+ * The partial sums cross as whole doubles. */
+LCS_API int lcs_debug_pcg_exchange(const double* values, double* sums, int32_t missing_block, uint32_t blocks,
+                                   uint32_t spin_limit, lcs_stream stream);
 /* The same for the batched solve's copies of the matrix to shared memory: y = A x (off-diagonal blocks; x, y: 4 floats a
  * row) by one warp through those copies.  omit_copy != 0: the first copy's barrier waits for 16 bytes that nothing sends
  * and gives up after poll_limit polls (1..2^20; the solves use 2^20) of at most a microsecond; the warp then reads the

@@ -102,6 +102,7 @@ SIGNATURES = {
     "lcs_bvh_create": (I32, [I32, U32, C.POINTER(P)]),
     "lcs_bvh_destroy": (I32, [P]),
     "lcs_debug_pcg_wait": (I32, [I32, I32, U32, U32, P]),
+    "lcs_debug_pcg_exchange": (I32, [P, P, I32, U32, U32, P]),
     "lcs_debug_pcg_copy_wait": (I32, [C.POINTER(Bsr), P, P, I32, U32, P]),
     "lcs_forest_query_tuning": (I32, [P, P, P]),
     "lcs_newton_batch_query_tuning": (I32, [P, P, P]),

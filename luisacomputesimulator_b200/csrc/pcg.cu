@@ -252,7 +252,7 @@ struct FusedArgs {
     const float4* b;
     float4* x;
     float4 *r, *z, *p, *q, *minv;
-    double* part;        // 3 * gridDim (k_pcg_small: 4)
+    double* part;        // 3 * gridDim (k_pcg_small: kSmallSumBytes a block)
     uint64_t l2_bytes;   // of the device (set at the launch)
     unsigned* bar_count;
     unsigned* bar_gen;
@@ -466,84 +466,131 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
     }
 }
 
-// The persistent solve of systems whose rows all have their four lanes at once (BT / 4 rows per block, one block per
-// SM).  Latency bounds it, so everything but the vectors that cross blocks stays in registers: the row's vectors and
-// diagonal blocks (the same on its four lanes) and up to four blocks of A per lane.  z crosses, and p is formed where
-// it is read, z + beta p_old, with two alternating buffers of p_old; that leaves two grid-wide exchanges per iteration,
-// and each exchange is one trip: a block's partial sums carry the exchange's number in their low four bits (see
-// res_allgather3) and are its arrival at the barrier too (release / acquire).
-// 100 iterations: 400 rows 1.19 ms as k_pcg_fused, 0.37 ms so; 4,096 rows 1.35 and 0.64; 10,000 rows 1.24 and 0.69.
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v)
+// A sum and the number of its exchange as one 16-byte word, which is written and read whole.
+struct __align__(16) TaggedSum {
+    double v;
+    unsigned long long tag;
+};
+template <bool Release>
+__device__ __forceinline__ void st_tagged(TaggedSum* p, double v, unsigned long long tag)
 {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    if (Release)
+        asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.release.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                     "l"(__double_as_longlong(v)), "l"(tag)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                     "l"(__double_as_longlong(v)), "l"(tag)
+                     : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p)
+__device__ __forceinline__ TaggedSum ld_tagged(const TaggedSum* p)
 {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
+    long long v;
+    unsigned long long tag;
+    asm volatile("{\n\t.reg .b128 w;\n\tld.acquire.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(v), "=l"(tag) : "l"(p) : "memory");
+    return TaggedSum{__longlong_as_double(v), tag};
 }
 constexpr int kSmallMaxBlocks = 256;
 constexpr int kSmallBlocksPerLane = 4;
+constexpr size_t kSmallSumBytes = 4 * sizeof(TaggedSum);  // per block: two sums in two alternating buffers
 
+template <int BT>
+struct SmallShared {
+    double warp[2][BT / 32];
+    double part[2][kSmallMaxBlocks];
+    int fail;  // 0 before the first exchange
+};
+
+// The sums of one or two values over the grid, the same in every warp of it, in one trip: a block's partial sums carry the
+// exchange's number (`step`, from 0; no word has step + 1 before) and are its arrival at the barrier too (release /
+// acquire).  False (in the block's every thread) once a wait has run out.
+template <int BT>
+__device__ __forceinline__ bool small_exchange(SmallShared<BT>& sh, TaggedSum* slots, unsigned step, double v0, double v1, int count,
+                                               double* out, lcs_pcg_stats* stats, unsigned limit = kBarrierSpinLimit)
+{
+    const uint32_t t = threadIdx.x, lane = lane_id();
+    const unsigned long long tag = step + 1ull;
+    TaggedSum* buf = slots + 2 * (size_t)(step & 1u) * gridDim.x;
+    v0 = warp_sum(v0);
+    if (count > 1) v1 = warp_sum(v1);
+    if (lane == 0) {
+        sh.warp[0][t >> 5] = v0;
+        sh.warp[1][t >> 5] = v1;
+    }
+    __syncthreads();
+    if (t == 0) {
+        double b0 = 0.0, b1 = 0.0;
+#pragma unroll
+        for (int w = 0; w < BT / 32; ++w) {
+            b0 += sh.warp[0][w];
+            b1 += sh.warp[1][w];
+        }
+        if (count > 1) st_tagged<false>(&buf[2 * blockIdx.x + 1], b1, tag);
+        st_tagged<true>(&buf[2 * blockIdx.x], b0, tag);
+    }
+    for (uint32_t k = t; k < (uint32_t)count * gridDim.x; k += BT) {
+        const uint32_t j = k / gridDim.x, b = k % gridDim.x;
+        TaggedSum got;
+        unsigned it = 0;
+        while ((got = ld_tagged(&buf[2 * b + j])).tag != tag) {
+            if (++it > limit) {
+                sh.fail = 1;
+                stats->status = LCS_ERR_TIMEOUT;
+                break;
+            }
+        }
+        sh.part[j][b] = got.v;
+    }
+    __syncthreads();
+    if (sh.fail) return false;
+    double o[2] = {0.0, 0.0};
+    for (uint32_t b = lane; b < gridDim.x; b += 32) {
+        o[0] += sh.part[0][b];
+        if (count > 1) o[1] += sh.part[1][b];
+    }
+    out[0] = warp_sum(o[0]);
+    if (count > 1) out[1] = warp_sum(o[1]);
+    return true;
+}
+
+// Test hook (lcs_debug_pcg_exchange): two exchanges of the blocks' values, of which block `missing` takes no part.
+__global__ void __launch_bounds__(256) k_exchange_probe(const double* values, TaggedSum* slots, int missing, unsigned limit, double* out,
+                                                        lcs_pcg_stats* stats)
+{
+    __shared__ SmallShared<256> sh;
+    if (threadIdx.x == 0) sh.fail = 0;
+    if ((int)blockIdx.x == missing) return;
+    const bool lead = threadIdx.x == 0;
+    const double a = lead ? values[2 * blockIdx.x] : 0.0, b = lead ? values[2 * blockIdx.x + 1] : 0.0;
+    double s[2], r;
+    if (!small_exchange<256>(sh, slots, 0u, a, b, 2, s, stats, limit)) return;
+    if (!small_exchange<256>(sh, slots, 1u, b, 0.0, 1, &r, stats, limit)) return;
+    if (lead && blockIdx.x == 0) {
+        out[0] = s[0];
+        out[1] = s[1];
+        out[2] = r;
+    }
+}
+
+// The persistent solve of systems whose rows all have their four lanes at once (BT / 4 rows per block, one block per
+// SM).  Latency bounds it, so everything but the vectors that cross blocks stays in registers: the row's vectors and
+// diagonal blocks (the same on its four lanes) and up to four blocks of A per lane.  z crosses, and p is formed where
+// it is read, z + beta p_old, with two alternating buffers of p_old; that leaves two grid-wide exchanges per iteration.
+// 400 rows 1.19 ms as k_pcg_fused, 0.39 ms so (50 to 100 iterations); 4,096 rows 1.35 and 0.54; 10,000 rows 1.24 and 0.63.
 template <int BT>
 __global__ void __launch_bounds__(BT, 1) k_pcg_small(FusedArgs a)
 {
-    __shared__ double s_warp[2][BT / 32];
-    __shared__ double s_part[2][kSmallMaxBlocks];
-    __shared__ int s_fail;
-    const uint32_t t = threadIdx.x, lane = lane_id(), lig = t & 3u, n = a.n;
+    __shared__ SmallShared<BT> sh;
+    const uint32_t t = threadIdx.x, lig = t & 3u, n = a.n;
     const uint32_t row = blockIdx.x * (BT / 4) + t / 4;
     const bool own = row < n, lead = own && lig == 0;
     const size_t i = own ? row : n - 1;
-    if (t == 0) s_fail = 0;
-    unsigned long long* slots = reinterpret_cast<unsigned long long*>(a.part);
+    if (t == 0) sh.fail = 0;
+    TaggedSum* slots = reinterpret_cast<TaggedSum*>(a.part);
     unsigned step = 0;  // exchanges done
-    auto exchange = [&](double v0, double v1, int count, double* out) -> bool {
-        const unsigned long long tag = step % 15u;
-        unsigned long long* buf = slots + 2 * (size_t)(step & 1u) * gridDim.x;
-        ++step;
-        v0 = warp_sum(v0);
-        if (count > 1) v1 = warp_sum(v1);
-        if (lane == 0) {
-            s_warp[0][t >> 5] = v0;
-            s_warp[1][t >> 5] = v1;
-        }
-        __syncthreads();
-        if (t == 0) {
-            double b0 = 0.0, b1 = 0.0;
-#pragma unroll
-            for (int w = 0; w < BT / 32; ++w) {
-                b0 += s_warp[0][w];
-                b1 += s_warp[1][w];
-            }
-            if (count > 1)
-                st_relaxed_u64(&buf[2 * blockIdx.x + 1], ((unsigned long long)__double_as_longlong(b1) & ~0xFull) | tag);
-            st_release_u64(&buf[2 * blockIdx.x], ((unsigned long long)__double_as_longlong(b0) & ~0xFull) | tag);
-        }
-        for (uint32_t k = t; k < (uint32_t)count * gridDim.x; k += BT) {
-            const uint32_t j = k / gridDim.x, b = k % gridDim.x;
-            unsigned long long bits;
-            unsigned it = 0;
-            while (((bits = ld_acquire_u64(&buf[2 * b + j])) & 0xFull) != tag) {
-                if (++it > kBarrierSpinLimit) {
-                    s_fail = 1;
-                    a.stats->status = LCS_ERR_TIMEOUT;
-                    break;
-                }
-            }
-            s_part[j][b] = __longlong_as_double((long long)(bits & ~0xFull));
-        }
-        __syncthreads();
-        if (s_fail) return false;
-        double o[2] = {0.0, 0.0};
-        for (uint32_t b = lane; b < gridDim.x; b += 32) {
-            o[0] += s_part[0][b];
-            if (count > 1) o[1] += s_part[1][b];
-        }
-        out[0] = warp_sum(o[0]);
-        if (count > 1) out[1] = warp_sum(o[1]);
-        return true;
+    auto exchange = [&](double v0, double v1, int count, double* out) {
+        return small_exchange<BT>(sh, slots, step++, v0, v1, count, out, a.stats);
     };
 
     // the row's blocks of A: the lane's first four in registers, the rest read again each time
@@ -2313,6 +2360,34 @@ extern "C" int lcs_debug_pcg_wait(int32_t which, int32_t missing_block, uint32_t
     return h.status;
 }
 
+extern "C" int lcs_debug_pcg_exchange(const double* values, double* sums, int32_t missing_block, uint32_t blocks,
+                                      uint32_t spin_limit, lcs_stream stream)
+{
+    if (!values || !sums) return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_exchange: bad argument");
+    if (blocks < 2 || blocks > 32 || missing_block >= (int32_t)blocks)
+        return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_exchange: blocks must be in [2, 32], the missing one among them");
+    if (spin_limit == 0 || spin_limit > kBarrierSpinLimit)
+        return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_exchange: spin_limit must be in [1, 2^24]");
+    cudaStream_t s = (cudaStream_t)stream;
+    unsigned char* mem = nullptr;  // the sums' words, then the status
+    lcs_pcg_stats h{};
+    const size_t bytes = kSmallSumBytes * blocks;
+    LCS_CUDA_TRY(cudaMalloc(&mem, bytes + sizeof(h)));
+    TaggedSum* slots = reinterpret_cast<TaggedSum*>(mem);
+    lcs_pcg_stats* st = reinterpret_cast<lcs_pcg_stats*>(mem + bytes);
+    cudaError_t e = cudaMemsetAsync(mem, 0, bytes + sizeof(h), s);
+    void* args[] = {&values, &slots, &missing_block, &spin_limit, &sums, &st};
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)k_exchange_probe, dim3(blocks), dim3(256), args, 0, s);
+    if (e == cudaSuccess) lcs_count_launch();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFree(mem);
+    LCS_CUDA_TRY(e);
+    if (h.status == LCS_ERR_TIMEOUT)
+        return lcs_fail(LCS_ERR_TIMEOUT, "lcs_debug_pcg_exchange: a bounded wait ran out (LCS_ERR_TIMEOUT)");
+    return h.status;
+}
+
 extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* y, int32_t omit_copy, uint32_t poll_limit,
                                        lcs_stream stream)
 {
@@ -2359,7 +2434,9 @@ extern "C" int lcs_pcg_create(uint32_t n, lcs_pcg** out)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     per_sm = fused_per_sm();
     p->fused_grid = sms * (per_sm > 0 ? per_sm : 1);
-    // fused: 3 doubles per block; row-resident: 4 per block, twice (alternate iterations) for up to kRowMaxBlocks
+    // fused: 3 doubles per block (small: 8 for up to kSmallMaxBlocks); row-resident: 4 per block, twice (alternate
+    // iterations) for up to kRowMaxBlocks
+    static_assert(kSmallSumBytes * kSmallMaxBlocks <= 8 * sizeof(double) * kRowMaxBlocks, "k_pcg_small's sums");
     const int parts = 8 * kRowMaxBlocks / 3 + 1 + (p->fused_grid > kPlainBlocks ? p->fused_grid : kPlainBlocks);
     cudaError_t e = cudaSuccess;
     auto A = [&](void** q, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(q, bytes); };
@@ -2757,7 +2834,7 @@ int lcs_pcg_solve_sell(lcs_pcg* P, const float* diag, const uint32_t* slice_ptr,
                       (cudaStream_t)stream, c_ptr, c_col, c_val, c_ok);
 }
 
-// The persistent solve on at most `grid` co-resident blocks (one per SM); a.part holds 4 doubles per block.  Rows that
+// The persistent solve on at most `grid` co-resident blocks (one per SM); a.part holds kSmallSumBytes per block.  Rows that
 // fit four lanes each in one block of 256 or 512 threads per SM take k_pcg_small.
 static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
 {
@@ -2768,7 +2845,7 @@ static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
     const uint64_t cap = (uint64_t)std::min(grid, kSmallMaxBlocks);
     if (a.n <= 128 * cap) {
         const uint32_t bt = a.n <= 64 * cap ? 256 : 512, blocks = (a.n + bt / 4 - 1) / (bt / 4);
-        LCS_CUDA_TRY(cudaMemsetAsync(a.part, 0xFF, 4 * sizeof(double) * blocks, s));
+        LCS_CUDA_TRY(cudaMemsetAsync(a.part, 0, kSmallSumBytes * blocks, s));
         LCS_CUDA_TRY(cudaLaunchCooperativeKernel(bt == 256 ? (const void*)k_pcg_small<256> : (const void*)k_pcg_small<512>,
                                                  dim3(blocks), dim3(bt), args, 0, s));
     } else {
@@ -2880,8 +2957,9 @@ constexpr uint32_t kNoAllocMaxBlocks = 1024;
 constexpr size_t kNaVec = 16ull * kNoAllocMaxRows;              // one float4 per row
 constexpr size_t kNaOffR = 0, kNaOffZ = kNaVec, kNaOffP = 2 * kNaVec, kNaOffQ = 3 * kNaVec;
 constexpr size_t kNaOffMinv = 4 * kNaVec;                        // three float4 per row
-constexpr size_t kNaOffPart = 7 * kNaVec;                        // 3 doubles per block
+constexpr size_t kNaOffPart = 7 * kNaVec;                        // 3 doubles per block, or k_pcg_small's sums
 constexpr size_t kNaOffBar = kNaOffPart + 24ull * kNoAllocMaxBlocks;
+static_assert(kSmallSumBytes * kSmallMaxBlocks <= 24ull * kNoAllocMaxBlocks && kNaOffPart % 16 == 0, "k_pcg_small's sums");
 constexpr size_t kNaOffStats = kNaOffBar + 256;
 constexpr size_t kNaBytes = kNaOffStats + 256;
 

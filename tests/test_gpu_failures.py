@@ -173,3 +173,22 @@ def test_copies_that_do_not_arrive_run_out_and_leave_the_product_right():
     # each of a lane's up to 10 blocks, the 4 lanes and the 3 columns round once: (10 + 2 + 3) 2^-24 of the magnitudes
     assert (np.abs(got[1] - y64) <= 15 * 2.0 ** -24 * mag).all()
     assert A.STATUS[lib.lcs_debug_pcg_copy_wait(M, ptr(keep[3]), ptr(y), 0, 0, stream())] == "LCS_ERR_INVALID"
+
+
+def test_exchange_of_small_systems_carries_whole_doubles_and_its_wait_runs_out():
+    """The grid-wide sums of the persistent solve's small systems: right to the last bits with every block, and a timeout,
+    after a short poll limit, with one that never takes part."""
+    lib = A.load()
+    rng = np.random.default_rng(2)
+    for blocks in (2, 3, 31, 32):
+        v = rng.normal(size=(blocks, 2)) * 10.0 ** rng.integers(-6, 6, (blocks, 2))
+        vd, sums = dev(v), torch.zeros(3, dtype=torch.float64, device="cuda")
+        assert lib.lcs_debug_pcg_exchange(ptr(vd), ptr(sums), -1, blocks, 1 << 20, stream()) == 0
+        want, mag = v.astype(np.longdouble).sum(0), np.abs(v).sum(0)
+        # five additions of a warp's tree round once each
+        for got, w, m in zip(host(sums), (want[0], want[1], want[1]), (mag[0], mag[1], mag[1])):
+            assert abs(got - w) <= 5 * 2.0 ** -53 * m, (blocks, got, w)
+        rc = lib.lcs_debug_pcg_exchange(ptr(vd), ptr(sums), blocks - 1, blocks, 1 << 12, stream())
+        assert A.STATUS[rc] == "LCS_ERR_TIMEOUT"
+    assert lib.lcs_debug_pcg_exchange(ptr(vd), ptr(sums), -1, 32, 1 << 20, stream()) == 0
+    assert A.STATUS[lib.lcs_debug_pcg_exchange(ptr(vd), ptr(sums), 32, 32, 16, stream())] == "LCS_ERR_INVALID"
