@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 #include <mutex>
@@ -350,7 +351,7 @@ __device__ __forceinline__ float3 mul3(const float4 m0, const float4 m1, const f
 // of L2 traffic a row and iteration at 13 blocks a row) three grid barriers keep apart: 401,322 rows move 280 MB an iteration
 // from HBM at 3.5 TB/s and 660 MB from L2 at 8.4.  The step's x and r updates and the next preconditioner are one pass.
 // A matrix that does not fit L2 beside the vectors is read under evict_first, so that it does not push them out: 250,000
-// rows 3.71 ms, 4.39 without; 401,322 rows 5.96 and 6.24.  One that fits is read as it comes and stays: 88,800 rows 2.05 ms,
+// rows 3.71 ms, 4.39 without; 401,322 rows 5.96 and 6.24.  One that fits is read as it comes and stays: 88,800 rows 2.06 ms,
 // under evict_first 2.20.  The line is three quarters of L2: 148,000 rows (0.72 of it) take 2.56 and 2.57 ms, 160,000
 // (0.78) 3.00 and 3.19.  Copies of the blocks to shared memory (row_stage.cuh), which pay in k_pcg_batch's
 // smaller blocks, took 8.4 ms against 1,024 threads that read directly.
@@ -439,18 +440,21 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
         float pq_f = 0.0f;
         const uint32_t lig = tid % G, ngroups = nthreads / G;
         const uint32_t rows_round = (n + ngroups - 1) / ngroups * ngroups;
-        for (uint32_t row = tid / G; row < rows_round; row += ngroups) {
-            const uint32_t r = row < n ? row : n - 1;  // whole groups stay converged for the shuffles
-            const float3 qv = stream ? row_product<G, true>(r, lig, a.diag, a.A, a.B, a.p)
-                                     : row_product<G>(r, lig, a.diag, a.A, a.B, a.p);
-            if (row < n && lig == 0) {
-                a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
-                const float4 pv = __ldcg(&a.p[row]);
-                const float d = __fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
-                pq_d += d;
-                pq_f += d;
+        auto product = [&](auto streamed) {
+            for (uint32_t row = tid / G; row < rows_round; row += ngroups) {
+                const uint32_t r = row < n ? row : n - 1;  // whole groups stay converged for the shuffles
+                const float3 qv = row_product<G, decltype(streamed)::value>(r, lig, a.diag, a.A, a.B, a.p);
+                if (row < n && lig == 0) {
+                    a.q[row] = make_float4(qv.x, qv.y, qv.z, 0.0f);
+                    const float4 pv = __ldcg(&a.p[row]);
+                    const float d = __fmaf_rn(pv.z, qv.z, __fmaf_rn(pv.y, qv.y, pv.x * qv.x));
+                    pq_d += d;
+                    pq_f += d;
+                }
             }
-        }
+        };
+        if (stream) product(std::true_type{});
+        else product(std::false_type{});
         publish(a.fp64 ? pq_d : (double)pq_f, 2);
         block_part(2, 1);
         if (!grid_barrier(a, &s_fail)) return;
