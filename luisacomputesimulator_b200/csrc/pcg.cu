@@ -3115,7 +3115,7 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         // so that the SMs of one GPC always hold them.
         const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
         const bool staged = cta_chunks >= 2;
-        const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= 148);
+        const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= (uint32_t)kNumSMs);
         const void* kernel = wide ? (const void*)k_pcg_batch<16, true>
                                   : staged ? (const void*)k_pcg_batch<8, true> : (const void*)k_pcg_batch<8, false>;
         const uint32_t warps = wide ? 16 : 8, smem = staged ? warps * stage::kWarpBytes : 0;

@@ -95,3 +95,47 @@ def test_batched_solves_at_the_edges(sizes, per_row, long_row, as_b, shift, clus
         err = np.linalg.norm(got[lo:hi].reshape(-1) - want) / np.linalg.norm(want)
         # |dx| / |x| <= cond(M) times the residual's 1e-6 and the 32-bit rounding of the blocks
         assert err <= np.linalg.cond(Ms) * (1e-6 + 2.0 ** -22), (err, lo, hi)
+
+
+def _residual(sys_, x):
+    D, rp, col, val, b = sys_
+    r = b - np.einsum("nij,nj->ni", D, x)
+    rows = np.repeat(np.arange(len(D)), np.diff(rp))
+    np.add.at(r, rows, -np.einsum("kij,kj->ki", val, x[col]))
+    return np.linalg.norm(r) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("sizes,cluster", [
+    ([600] + [20] * 148, 1), ([600] + [33] * 79, 2),  # more CTAs than SMs, the largest scene of two chunks a CTA and more
+    ([4200, 40], 16),                                 # clusters of 16
+    ([3000, 2100], 1),                                # eight chunks a CTA
+])
+def test_batched_solves_by_every_variant(sizes, cluster, fp64):
+    """The staged solve by 8 warps (the first three) and by 16, against 64-bit residuals."""
+    rng = np.random.default_rng(len(sizes))
+    systems = [_system(n, 9, rng) for n in sizes]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    n = int(off[-1])
+    diag = np.zeros((n, 3, 4), np.float32)
+    diag[:, :, :3] = np.concatenate([s[0] for s in systems]).transpose(0, 2, 1)
+    nnz = np.concatenate([[0], np.cumsum([len(s[2]) for s in systems])])
+    rp = np.concatenate([s[1][:-1] + o for s, o in zip(systems, nnz)] + [nnz[-1:]]).astype(np.uint32)
+    col = np.concatenate([s[2] + o for s, o in zip(systems, off)]).astype(np.uint32)
+    val = np.concatenate([s[3] for s in systems]).transpose(0, 2, 1).reshape(-1).astype(np.float32)
+    b = np.zeros((n, 4), np.float32)
+    b[:, :3] = np.concatenate([s[4] for s in systems])
+    M = make_bsr(n, dev(rp.view(np.int32)), dev(col.view(np.int32)), dev(val))
+    x = torch.full((n, 4), 5.0, dtype=torch.float32, device="cuda")
+    stats = torch.zeros((len(sizes), 4), dtype=torch.int32, device="cuda")
+    solve_batch(ConjugateGradientSolver(n), dev(off.astype(np.int32)), dev(diag), M, None, dev(b), x, stats, max_iter=400,
+                rel_tol=1e-5, abs_rz_tol=0.0, cluster=cluster, fp64_dots=fp64)
+    torch.cuda.synchronize()
+    st = host(stats)
+    assert (st[:, 3] == 0).all()
+    got = host(x)[:, :3].astype(np.float64)
+    for s, lo, hi, iters in zip(systems, off[:-1], off[1:], st[:, 0]):
+        # the recurrence stops at 1e-5 and leaves the true residual by a few roundings of A x an iteration; eigenvalues lie
+        # between 1 and 1 + 2 * 1.1 for each block of a row
+        cond = 1 + 2.2 * np.diff(s[1]).max()
+        assert _residual(s, got[lo:hi]) <= 1e-5 + 4 * 2.0 ** -24 * np.sqrt(max(iters, 1)) * cond
