@@ -65,9 +65,10 @@ struct lcs_bvh {
     uint32_t* turns = nullptr;       // 3 + max_tops: see k_depth_parity
     uint32_t* top_lefts = nullptr;   // 32 * max_tops: slots of the 31 inner left siblings above each listed top
     uint32_t* early = nullptr;       // kSymSlots: number of the query call that may end early, a slot per call in turn
-    uint32_t* sym_info = nullptr;    // (edge trees of kSymEdges leaves and more) kSymSlots x kSymWords: k_sym_check's findings, a slot per query call in turn
+    uint32_t* sym_info = nullptr;    // kSymSlots x kSymWords (edge trees of kSymEdges leaves and more): k_sym_check's
+                                     // findings, a slot per query call in turn
     mutable uint32_t calls = 0;
-    bool leaves_newer = false;       // leaf boxes were written after the last refit (the binary records alone hold them)
+    bool leaves_newer = false;       // leaf boxes were written after the last refit (only the binary records hold them)
     bool built = false;              // a construct has written the topology, slots and refit tables
 };
 
@@ -181,7 +182,7 @@ __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* _
                               uint2* __restrict__ range, uint32_t* __restrict__ swap_diff)
 {
     const int ni = (int)n - 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) turns[0] = turns[1] = turns[2] = 0u;  // raised by k_depth_parity, launched after this
+    if (blockIdx.x == 0 && threadIdx.x == 0) turns[0] = turns[1] = turns[2] = 0u;  // raised by k_depth_parity
     for (int nid = blockIdx.x * blockDim.x + threadIdx.x; nid < ni; nid += gridDim.x * blockDim.x) {
         int i = 0, j = ni;
         if (nid != 0) {
@@ -246,11 +247,11 @@ __global__ void k_build_inner(const uint64_t* __restrict__ ms, const uint32_t* _
 // overlap test passes.  A traversal then takes one dependent
 // 128-B fetch where the binary walk took two 64-B ones.  k_depth_parity marks the even-depth inner nodes
 // after each build (a climb to the root per node, at most 256 levels).
-// It also counts, for each inner node, the nodes that a walk of the reference can at most have pending when it pops it:
-// one for every ancestor whose second child the path takes and whose first child is an inner node.  turns: [0] the
+// It also counts, for each inner node, the nodes that a walk of the reference can at most have pending when it pops
+// it: one for every ancestor whose second child the path takes and whose first child is an inner node.  turns: [0] the
 // largest count, [1] how many nodes reach kRefPending by their own turn (every node with as many descends from one of
-// them), [2] the depth of the deepest inner node, [3...] the slots of the first max_tops of those that reach kRefPending,
-// whose 31 inner left siblings top_lefts lists.
+// them), [2] the depth of the deepest inner node, [3...] the slots of the first max_tops of those that reach
+// kRefPending, whose 31 inner left siblings top_lefts lists.
 constexpr uint32_t kRefStack = 32;
 constexpr uint32_t kRefPending = kRefStack - 1;
 
@@ -676,13 +677,14 @@ __global__ void k_refit_span_records(const uint32_t* __restrict__ spans, const u
 constexpr int kStack4 = 64;  // entries of the 4-wide traversal stack
 
 // The reference's stack (32 entries; children are pushed left, right and the right one is popped next) holds one
-// pending node for each right turn of the path past an inner left child that overlaps the query, so it can only fill --
-// and end a query early -- below one of the tops that k_depth_parity lists.  Every call first asks (k_may_end) whether
-// any of its queries could meet a full stack there; if none can, the 4-wide walks below serve it (their own 64-entry
-// stack holds at most two nodes per turn), else query_ref restates the reference's walk, early exit included.  The
-// walks' kernels read the answer, so the choice costs no host synchronisation.  Depth is no measure: sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels,
-// with a few paths of 31 turns near one corner, but no query keeps more than a handful of nodes pending.
-// The other limit of the reference's walk, 100,000 popped nodes, is asked for there too.
+// pending node for each right turn of the path past an inner left child that overlaps the query, so it can only fill
+// -- and end a query early -- below one of the tops that k_depth_parity lists.  Every call first asks (k_may_end)
+// whether any of its queries could meet a full stack there; if none can, the 4-wide walks below serve it (their own
+// 64-entry stack holds at most two nodes per turn), else query_ref restates the reference's walk, early exit
+// included.  The walks' kernels read the answer, so the choice costs no host synchronisation.  Depth is no measure:
+// sheets whose 30-bit Morton codes repeat make trees deeper than 32 levels, with a few paths of 31 turns near one
+// corner, but no query keeps more than a handful of nodes pending.  The other limit of the reference's walk, 100,000
+// popped nodes, is asked for there too.
 struct Early {
     const uint32_t* flag;  // the call's slot: its number if it may end early
     uint32_t call;
@@ -730,15 +732,16 @@ __device__ __forceinline__ float from_ordered(uint32_t u)
     return __uint_as_float(u & 0x80000000u ? u & 0x7FFFFFFFu : ~u);
 }
 
-// Whether the once-per-pair walk serves a general EE query, by k_sym_check's findings.  It has to look as far around each
-// edge as the largest d_hat reaches, which is many times as much as most need where one body or vertex stands out.  The
-// line: the largest d_hat exceeds the mean one by a tenth of the query boxes' mean extent (two sheets of 448 x 448
-// vertices: 4.5 ms with equal d_hat, 5.0 at the line, 6.8 at twice that, 5.7 by k_query<true> at any).
+// Whether the once-per-pair walk serves a general EE query, by k_sym_check's findings.  It has to look as far around
+// each edge as the largest d_hat reaches, which is many times as much as most need where one body or vertex stands
+// out.  The line: the largest d_hat exceeds the mean one by a tenth of the query boxes' mean extent (two sheets of 448
+// x 448 vertices: 4.5 ms with equal d_hat, 5.0 at the line, 6.8 at twice that, 5.7 by k_query<true> at any).
 constexpr float kSymSpread = 0.1f;
 __device__ __forceinline__ bool sym_serves(const uint32_t* info, uint32_t n)
 {
     if (info[0] != 0u) return false;
-    return from_ordered(info[1]) - __uint_as_float(info[3]) / (float)n <= kSymSpread * (__uint_as_float(info[4]) / (float)n);
+    const float mean = __uint_as_float(info[3]) / (float)n, extent = __uint_as_float(info[4]) / (float)n;
+    return from_ordered(info[1]) - mean <= kSymSpread * extent;
 }
 
 // an edge as a query of the once-per-pair walks (see k_query_ee_sym)
@@ -794,8 +797,9 @@ __device__ __forceinline__ void met_box(const float4* x0, const float4* x1, cons
 constexpr uint32_t kRefNodes = 100000;  // popped nodes after which a walk ends
 
 // Whether a walk of the box pops more than kRefNodes inner nodes: the tree's, less every subtree found apart from the
-// box, until they are no more than that.  Large subtrees are looked at first, so that a box that is small beside the tree
-// is done after some dozens of steps; what is never done is looked at to the leaves (not `exact`: counts as "yes").
+// box, until they are no more than that.  Large subtrees are looked at first, so that a box that is small beside the
+// tree is done after some dozens of steps; what is never done is looked at to the leaves (not `exact`: counts as
+// "yes").
 __device__ __forceinline__ bool exceeds(const float4* wide, uint32_t ni, const float* box, bool exact)
 {
     for (uint32_t small = 16384;; small >>= 3) {  // subtrees of so many inner nodes count whole
@@ -837,16 +841,17 @@ __device__ __forceinline__ void warp_union(const float* box, float* all)
     }
 }
 
-// Marks the call if one of its queries overlaps a listed top with so many overlapping inner left siblings above it that,
-// were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's walk
-// reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and a near
-// top's left siblings, one per lane, against the union of its 32 queries' boxes; only where that is not enough does each
-// query climb.  A tree of 32 levels whose leaf boxes are newer than its inner ones is walked the reference's way as well:
-// the 4-wide records have the leaf boxes of the last refit.
+// Marks the call if one of its queries overlaps a listed top with so many overlapping inner left siblings above it
+// that, were every turn below the top to leave one more pending, the stack could fill.  (It reads what the reference's
+// walk reads there; a call marked without need only takes the slower walk.)  A warp tests the tops, one per lane, and
+// a near top's left siblings, one per lane, against the union of its 32 queries' boxes; only where that is not enough
+// does each query climb.  A tree of 32 levels whose leaf boxes are newer than its inner ones is walked the reference's
+// way as well: the 4-wide records have the leaf boxes of the last refit.
 // Count (trees of more than kRefNodes inner nodes): on trees of 32 levels or more it also marks the call if one of its
-// queries pops so many nodes that its walk ends (trees of fewer levels are walked by their own records, counted 4-wide), and
-// takes a general EE query off the once-per-pair walk (info) where the largest d_hat would make an edge's walk end: only
-// its own reach may.  The union is asked first here too (1.2 million edges in the tree's order: 0.14 ms).
+// queries pops so many nodes that its walk ends (trees of fewer levels are walked by their own records, counted
+// 4-wide), and takes a general EE query off the once-per-pair walk (info) where the largest d_hat would make an edge's
+// walk end: only its own reach may.  The union is asked first here too (1.2 million edges in the tree's order: 0.14
+// ms).
 template <bool EE, bool Count>
 __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide, const uint32_t* __restrict__ slot,
                                                  const uint32_t* __restrict__ turns, const uint32_t* __restrict__ top_lefts,
@@ -931,8 +936,9 @@ __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide
 // children tested in order (left, then right) and the right one popped first; an inner child that meets a
 // full stack ends the whole query (the pairs found so far stay), and so does the 100001st popped node.
 // Both early exits are reported through `capped`.  EE keeps the reference's eid < adj filter.
-// Below kPacketLeaves queries it is the other branch of the wide walks' kernels, which saves the calls that do not need it,
-// nearly all, a launch; from there on a kernel of its own, with half their registers and so twice their warps in flight.
+// Below kPacketLeaves queries it is the other branch of the wide walks' kernels, which saves the calls that do not
+// need it, nearly all, a launch; from there on a kernel of its own, with half their registers and so twice their warps
+// in flight.
 template <bool EE>
 __device__ __forceinline__ void query_ref(const float4* __restrict__ wide, const float4* __restrict__ x0,
                                           const float4* __restrict__ x1, const uint2* __restrict__ edges, uint32_t n_queries,
@@ -1058,11 +1064,11 @@ static_assert(kSymEdges >= kPacketLeaves, "the lane walk has no per-edge form");
 constexpr int kSymStack = 96, kPacketStack = 128;
 
 // Whether a general EE query may take the once-per-pair walk: its edges, positions and thicknesses are, bit for bit,
-// those of the tree's leaf boxes, and the tree has 32 levels or more.  Codes repeat there, so that boxes of neighbouring
-// subtrees overlap and a warp's queries share many records (two sheets of 448 x 448 vertices: 4.5 ms a call so, 5.7 by
-// k_query<true>); a tube of 134,000 edges, whose tree has fewer levels, takes 0.20 and 0.11 ms.
-// info (zeroed before): [0] leaves that differ or are not finite, [1] the largest d_hat, [2] the largest thickness + d_hat
-// (as `ordered`), [3] the sum of d_hat, [4] of the query boxes' largest extents.
+// those of the tree's leaf boxes, and the tree has 32 levels or more.  Codes repeat there, so that boxes of
+// neighbouring subtrees overlap and a warp's queries share many records (two sheets of 448 x 448 vertices: 4.5 ms a
+// call so, 5.7 by k_query<true>); a tube of 134,000 edges, whose tree has fewer levels, takes 0.20 and 0.11 ms.
+// info (zeroed before): [0] leaves that differ or are not finite, [1] the largest d_hat, [2] the largest thickness +
+// d_hat (as `ordered`), [3] the sum of d_hat, [4] of the query boxes' largest extents.
 __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wide, const uint32_t* __restrict__ sgo,
                                                    const uint32_t* __restrict__ slot, uint32_t n,
                                                    const float4* __restrict__ x0, const float4* __restrict__ x1,
@@ -1085,7 +1091,8 @@ __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wi
         ld_slot(wide + 4 * (size_t)(s >> 1) + 2 * (s & 1u), a, b);
         const uint32_t v0 = __ldg(&edges[q].x);
         const float d = __ldg(&dhat[v0]), r = __ldg(&thickness[v0]) + d;
-        const float ext = fmaxf(mx.x - mn.x, fmaxf(mx.y - mn.y, mx.z - mn.z)) + 2.0f * d;  // the leaf box has the thickness
+        // (the leaf box has the thickness)
+        const float ext = fmaxf(mx.x - mn.x, fmaxf(mx.y - mn.y, mx.z - mn.z)) + 2.0f * d;
         if (!(mn.x == a.x && mn.y == a.y && mn.z == a.z && mx.x == b.x && mx.y == b.y && mx.z == b.z) || !isfinite(d) ||
             !isfinite(r) || !isfinite(mn.x + mn.y + mn.z) || !isfinite(mx.x + mx.y + mx.z))
             bad = 1;
@@ -1118,20 +1125,20 @@ __global__ void __launch_bounds__(256) k_sym_check(const float4* __restrict__ wi
     }
 }
 
-// EE candidates with every pair found once: the set query_template2 / fn_query_from_edges_v2 produce
-// ({(a, b): a < b, query box of a overlaps leaf box of b}).  The query of the leaf at sorted position i visits only
-// slots whose largest sorted position (`last`) exceeds i, so each pair of leaves is met from the lower position alone,
-// with a culling box a few ulps wider than the query box needs; at a leaf the reference's own test decides, in the
-// reference's direction: for q < e the query box of q against the leaf box of e, for e < q the query box of e against
-// the leaf box of q.  Pairs are written (smaller id, larger id) as the reference writes them.  Leaves of other queries
-// are pruned by position, not by id, so a traversal visits about half the nodes of k_query<true>.
-// PerEdge = false: every edge's first vertex has thickness 0 and the same d_hat r, so that e's query box is its leaf box
-// widened by r and q's leaf box is q's own.  PerEdge = true: per-vertex thickness and d_hat on the tree's own leaves
-// (k_sym_check); e's query box is formed from its vertices, and the culling box holds the largest d_hat.
+// EE candidates with every pair found once: the set query_template2 / fn_query_from_edges_v2 produce ({(a, b): a < b,
+// query box of a overlaps leaf box of b}).  The query of the leaf at sorted position i visits only slots whose largest
+// sorted position (`last`) exceeds i, so each pair of leaves is met from the lower position alone, with a culling box
+// a few ulps wider than the query box needs; at a leaf the reference's own test decides, in the reference's direction:
+// for q < e the query box of q against the leaf box of e, for e < q the query box of e against the leaf box of q.
+// Pairs are written (smaller id, larger id) as the reference writes them.  Leaves of other queries are pruned by
+// position, not by id, so a traversal visits about half the nodes of k_query<true>.
+// PerEdge = false: every edge's first vertex has thickness 0 and the same d_hat r, so that e's query box is its leaf
+// box widened by r and q's leaf box is q's own.  PerEdge = true: per-vertex thickness and d_hat on the tree's own
+// leaves (k_sym_check); e's query box is formed from its vertices, and the culling box holds the largest d_hat.
 // A warp walks the union of its 32 queries' paths -- they are neighbours in the tree's own order -- with one stack of
 // {node, the lanes it overlaps} in shared memory: a record is then one broadcast line for the warp instead of up to 32
-// scattered ones, no lane waits for another's longer walk, and the pairs leave in runs.  Each lane still counts its own
-// steps.
+// scattered ones, no lane waits for another's longer walk, and the pairs leave in runs.  Each lane still counts its
+// own steps.
 // Static and swept queries of two sheets of 448 x 448 vertices with a thickness: 12.9 ms as query_ref, 8.6 ms so; of
 // 212 x 212 vertices of thickness 0: 2.3 and 1.3 ms.
 template <bool PerEdge>
@@ -1217,11 +1224,13 @@ __global__ void __launch_bounds__(128) k_query_ee_sym(const float4* __restrict__
     }
 }
 
-// The same walk with one radius, one query per thread, for trees that leave most of the GPU's warps idle: a warp's union
-// of paths is longer than its longest path, which is what the time is there.
+// The same walk with one radius, one query per thread, for trees that leave most of the GPU's warps idle: a warp's
+// union of paths is longer than its longest path, which is what the time is there.
 __global__ void __launch_bounds__(128) k_query_ee_sym_lane(const float4* __restrict__ wide, const float4* __restrict__ wide4,
-                                                           const uint32_t* __restrict__ sgo, uint32_t n_leaves, const float4* __restrict__ x0,
-                                                           const float4* __restrict__ x1, const uint2* __restrict__ edges,
+                                                           const uint32_t* __restrict__ sgo, uint32_t n_leaves,
+                                                           const float4* __restrict__ x0,
+                                                           const float4* __restrict__ x1,
+                                                           const uint2* __restrict__ edges,
                                                            float uniform_r, uint2* __restrict__ pairs, uint32_t capacity,
                                                            uint32_t* d_count, uint32_t* capped, const Early early)
 {
@@ -1435,8 +1444,8 @@ extern "C" int lcs_bvh_destroy(lcs_bvh* h)
     void* ptrs[] = {h->centers, h->block_aabb, h->gaabb, h->m30, h->keys, h->keys_alt, h->vals, h->vals_alt,
                     h->hist, h->ms64, h->parent, h->children, h->slot, h->wide, h->wide4, h->even, h->range,
                     h->swap_diff, h->swap_cov, h->scan_tmp, h->n_plus_1, h->leaf_at, h->node_at,
-                    h->order_range, h->spans, h->span_count, h->seg_box, h->chunk_box, h->healthy, h->turns, h->top_lefts, h->early,
-                    h->sym_info};
+                    h->order_range, h->spans, h->span_count, h->seg_box, h->chunk_box, h->healthy, h->turns,
+                    h->top_lefts, h->early, h->sym_info};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete h;
@@ -1627,8 +1636,8 @@ static Early ask_early(const lcs_bvh* t, uint32_t call, const float* x0, const f
     uint32_t* flag = t->early + call % kSymSlots;
     if (t->ni > 0) {
         const auto ask = t->ni > kRefNodes ? k_may_end<EE, true> : k_may_end<EE, false>;
-        ask<<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, p0, p1, e2, n, dhat, thickness, uniform_r,
-                                             order, t->leaves_newer, t->ni, call, flag, info);
+        ask<<<grid_for(n, 256), 256, 0, s>>>(t->wide, t->slot, t->turns, t->top_lefts, p0, p1, e2, n, dhat, thickness,
+                                             uniform_r, order, t->leaves_newer, t->ni, call, flag, info);
         lcs_count_launch();
     }
     return Early{flag, call};
@@ -1689,14 +1698,15 @@ int lcs_bvh_query_ee_capped(const lcs_bvh* t, const float* x0, const float* x1, 
     const uint2* e2 = reinterpret_cast<const uint2*>(edges);
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t call = next_call(t);
-    // The tree's own edges in earnest numbers: once per pair, if the device finds the arguments fit for it.  Two sheets of
-    // 74,000, 268,000 and 1.2 million edges: 376, 966 and 4,525 us so, 350, 1,033 and 5,700 by k_query<true> alone.
+    // The tree's own edges in earnest numbers: once per pair, if the device finds the arguments fit for it.  Two
+    // sheets of 74,000, 268,000 and 1.2 million edges: 376, 966 and 4,525 us so, 350, 1,033 and 5,700 by k_query<true>
+    // alone.
     uint32_t* info = nullptr;
     if (n_edges == t->n && n_edges >= kSymEdges) {
         info = t->sym_info + kSymWords * (call % kSymSlots);
         LCS_CUDA_TRY(cudaMemsetAsync(info, 0, 4 * kSymWords, s));
-        k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat, thickness, t->turns,
-                                                             info);
+        k_sym_check<<<grid_for(n_edges, 256), 256, 0, s>>>(t->wide, t->sgo, t->slot, t->n, p0, p1, e2, d_hat,
+                                                           thickness, t->turns, info);
         lcs_count_launch();
     }
     const Early early = ask_early<true>(t, call, x0, x1, edges, n_edges, d_hat, thickness, 0.0f,

@@ -17,9 +17,9 @@ namespace {
 
 // The evaluators write 224 to 832 bytes per element, so they are bound by those stores.  One thread storing its own
 // element spreads every store instruction of a warp over 32 half-written sectors (bending of an 88,800-vertex cloth,
-// 221 MB: 212 us, 1.0 TB/s; the three evaluators and the energy: 368 us, now 88 us).  Here a warp's 32 elements are evaluated one per lane into shared memory (an odd
-// number of words per element: no bank conflicts) and the warp then writes their output as one run of consecutive
-// 16-byte words, each lane forming the word it stores.
+// 221 MB: 212 us, 1.0 TB/s; the three evaluators and the energy: 368 us, now 88 us).  Here a warp's 32 elements are
+// evaluated one per lane into shared memory (an odd number of words per element: no bank conflicts) and the warp then
+// writes their output as one run of consecutive 16-byte words, each lane forming the word it stores.
 constexpr int kEvalThreads = 128, kEvalWarps = kEvalThreads / 32;
 
 __global__ void __launch_bounds__(kEvalThreads) k_eval_springs(uint32_t n, const float4* __restrict__ x,
@@ -173,10 +173,11 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_bending(uint32_t n, const
 }
 
 // energy terms: [0] inertia (fn_calc_energy_inertia), [1] springs, [2] stretch faces, [3] bending
-// One atomic per block and term: with one per warp, about 8,300 additions to each of four addresses took most of the time
-// (46 us on 88,800 vertices).
-__global__ void __launch_bounds__(256) k_material_energy(lcs_cloth_elements m, const float4* __restrict__ x, const float4* __restrict__ xt,
-                                  float dt, float dirichlet, double* out)
+// One atomic per block and term: with one per warp, about 8,300 additions to each of four addresses took most of the
+// time (46 us on 88,800 vertices).
+__global__ void __launch_bounds__(256) k_material_energy(lcs_cloth_elements m, const float4* __restrict__ x,
+                                                         const float4* __restrict__ xt, float dt, float dirichlet,
+                                                         double* out)
 {
     const uint32_t n = max(max(m.n_verts, m.n_springs), max(m.n_stretch_faces, m.n_bending));
     const uint32_t stride = gridDim.x * blockDim.x;

@@ -422,11 +422,12 @@ __global__ void k_segments(const uint64_t* __restrict__ keys, const uint32_t* __
     }
 }
 
-// The (row, column, triplet) order of the contact triplets without a global radix sort (pairs without affine
-// bodies): the 12 directed vertex pairs of every contact pair are bucketed by row (a count, a scan and a
-// scatter with per-row cursors), and each entry finds its place in its row's bucket by counting the entries
-// that precede it in (column, triplet index) order -- the order the stable radix sort gives.  Most rows hold at
-// most a few hundred entries; a vertex that many others touch has thousands.  k_heads, k_segments and k_row_ptr then run on the result as after the sort.
+// The (row, column, triplet) order of the contact triplets without a global radix sort (pairs without affine bodies):
+// the 12 directed vertex pairs of every contact pair are bucketed by row (a count, a scan and a scatter with per-row
+// cursors), and each entry finds its place in its row's bucket by counting the entries that precede it in (column,
+// triplet index) order -- the order the stable radix sort gives.  Most rows hold at most a few hundred entries; a
+// vertex that many others touch has thousands.  k_heads, k_segments and k_row_ptr then run on the result as after the
+// sort.
 __global__ void k_row_count(const lcs_pair* __restrict__ pairs, const uint32_t* d_count, uint32_t cap,
                             uint32_t* __restrict__ rcnt)
 {
@@ -468,12 +469,12 @@ __global__ void k_row_scatter(const lcs_pair* __restrict__ pairs, const uint32_t
 
 // A warp takes `rows` rows (at most 31), one after the other: the row's entries as (column, triplet) words in shared
 // memory, each lane counting the words below its own, two at a time.  One thread per entry over 64-bit keys in global
-// memory was bound by the latency of its serial loads: 401,408 vertices with 476,000 pairs 982 us, 366 us so; 5,000 with
-// 4,348 pairs 34 and 16.
-// The entries of rows beyond kRankCap, if there are any, are then dealt out to all warps, 32 at a time, each of which counts
-// through the whole row in pieces of kRankCap words, so that the GPU shares a work that grows by the square of the length
-// (an assembly with a row of 15,000 entries 0.26 ms, of 30,000 0.54; by one warp 342 ms and 1.4 s, by a thread per entry 1.3
-// and 2.6 ms).
+// memory was bound by the latency of its serial loads: 401,408 vertices with 476,000 pairs 982 us, 366 us so; 5,000
+// with 4,348 pairs 34 and 16.
+// The entries of rows beyond kRankCap, if there are any, are then dealt out to all warps, 32 at a time, each of which
+// counts through the whole row in pieces of kRankCap words, so that the GPU shares a work that grows by the square of
+// the length (an assembly with a row of 15,000 entries 0.26 ms, of 30,000 0.54; by one warp 342 ms and 1.4 s, by a
+// thread per entry 1.3 and 2.6 ms).
 __device__ __forceinline__ uint32_t count_below(const unsigned long long* word, uint32_t len, unsigned long long mine)
 {
     uint32_t rank = 0;
@@ -686,7 +687,7 @@ int offdiag_bsr(lcs_assembler* a, const lcs_pair* pairs, const uint32_t* d_count
                                                                    a->keys_alt, a->vals_alt, any_long);
             lcs_count_launch();
         }
-        // few rows: a warp each, so that the longest ones do not follow one another; many: four each, most of them empty
+        // few rows: a warp each, so that the longest do not follow one another; many: four each, most of them empty
         const uint32_t rows = a->n_rows <= 32768 ? 1 : 4;
         // (two blocks per SM at least: the entries of long rows are dealt out to all)
         const uint32_t blocks = std::max((a->n_rows + kRankWarps * rows - 1) / (kRankWarps * rows), 2u * kNumSMs);

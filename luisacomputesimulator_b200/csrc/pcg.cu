@@ -330,7 +330,8 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
 }
 
 // The inverse of a diagonal block as three columns.
-__device__ __forceinline__ void invert_diag(const float4 c0, const float4 c1, const float4 c2, float4& m0, float4& m1, float4& m2)
+__device__ __forceinline__ void invert_diag(const float4 c0, const float4 c1, const float4 c2, float4& m0, float4& m1,
+                                            float4& m2)
 {
     const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, k = c2.z;
     const float A = e * k - f * h, B = f * g - d * k, C = d * h - e * g;
@@ -347,14 +348,14 @@ __device__ __forceinline__ float3 mul3(const float4 m0, const float4 m1, const f
                        __fmaf_rn(m2.z, v.z, __fmaf_rn(m1.z, v.y, m0.z * v.x)));
 }
 
-// The persistent solve of systems beyond k_pcg_small, whose passes over the vectors and the matrix (0.7 KB of HBM and 1.6 KB
-// of L2 traffic a row and iteration at 13 blocks a row) three grid barriers keep apart: 401,322 rows move 280 MB an iteration
-// from HBM at 3.5 TB/s and 660 MB from L2 at 8.4.  The step's x and r updates and the next preconditioner are one pass.
-// A matrix that does not fit L2 beside the vectors is read under evict_first, so that it does not push them out: 250,000
-// rows 3.71 ms, 4.39 without; 401,322 rows 5.96 and 6.24.  One that fits is read as it comes and stays: 88,800 rows 2.06 ms,
-// under evict_first 2.20.  The line is three quarters of L2: 148,000 rows (0.72 of it) take 2.56 and 2.57 ms, 160,000
-// (0.78) 3.00 and 3.19.  Copies of the blocks to shared memory (row_stage.cuh), which pay in k_pcg_batch's
-// smaller blocks, took 8.4 ms against 1,024 threads that read directly.
+// The persistent solve of systems beyond k_pcg_small, whose passes over the vectors and the matrix (0.7 KB of HBM and
+// 1.6 KB of L2 traffic a row and iteration at 13 blocks a row) three grid barriers keep apart: 401,322 rows move 280
+// MB an iteration from HBM at 3.5 TB/s and 660 MB from L2 at 8.4.  The step's x and r updates and the next
+// preconditioner are one pass.  A matrix that does not fit L2 beside the vectors is read under evict_first, so that it
+// does not push them out: 250,000 rows 3.71 ms, 4.39 without; 401,322 rows 5.96 and 6.24.  One that fits is read as it
+// comes and stays: 88,800 rows 2.06 ms, under evict_first 2.20.  The line is three quarters of L2: 148,000 rows (0.72
+// of it) take 2.56 and 2.57 ms, 160,000 (0.78) 3.00 and 3.19.  Copies of the blocks to shared memory (row_stage.cuh),
+// which pay in k_pcg_batch's smaller blocks, took 8.4 ms against 1,024 threads that read directly.
 constexpr uint64_t kRowBytes = 176;  // diag, minv and five vectors
 template <int G>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_pcg_fused(FusedArgs a)
@@ -506,12 +507,13 @@ struct SmallShared {
     int fail;  // 0 before the first exchange
 };
 
-// The sums of one or two values over the grid, the same in every warp of it, in one trip: a block's partial sums carry the
-// exchange's number (`step`, from 0; no word has step + 1 before) and are its arrival at the barrier too (release /
-// acquire).  False (in the block's every thread) once a wait has run out.
+// The sums of one or two values over the grid, the same in every warp of it, in one trip: a block's partial sums carry
+// the exchange's number (`step`, from 0; no word has step + 1 before) and are its arrival at the barrier too (release
+// / acquire).  False (in the block's every thread) once a wait has run out.
 template <int BT>
-__device__ __forceinline__ bool small_exchange(SmallShared<BT>& sh, TaggedSum* slots, unsigned step, double v0, double v1, int count,
-                                               double* out, lcs_pcg_stats* stats, unsigned limit = kBarrierSpinLimit)
+__device__ __forceinline__ bool small_exchange(SmallShared<BT>& sh, TaggedSum* slots, unsigned step, double v0,
+                                               double v1, int count, double* out, lcs_pcg_stats* stats,
+                                               unsigned limit = kBarrierSpinLimit)
 {
     const uint32_t t = threadIdx.x, lane = lane_id();
     const unsigned long long tag = step + 1ull;
@@ -559,8 +561,8 @@ __device__ __forceinline__ bool small_exchange(SmallShared<BT>& sh, TaggedSum* s
 }
 
 // Test hook (lcs_debug_pcg_exchange): two exchanges of the blocks' values, of which block `missing` takes no part.
-__global__ void __launch_bounds__(256) k_exchange_probe(const double* values, TaggedSum* slots, int missing, unsigned limit, double* out,
-                                                        lcs_pcg_stats* stats)
+__global__ void __launch_bounds__(256) k_exchange_probe(const double* values, TaggedSum* slots, int missing,
+                                                        unsigned limit, double* out, lcs_pcg_stats* stats)
 {
     __shared__ SmallShared<256> sh;
     if (threadIdx.x == 0) sh.fail = 0;
@@ -2144,8 +2146,10 @@ __global__ void __launch_bounds__(32 * W, !Staged ? 4 : W > 8 ? 1 : 2) k_pcg_bat
                         rv = a.b[i];
                         a.x[i] = make_float4(0, 0, 0, 0);
                         a.p[i] = make_float4(0, 0, 0, 0);
-                        const float4 c0 = a.diag[3 * (size_t)i], c1 = a.diag[3 * (size_t)i + 1], c2 = a.diag[3 * (size_t)i + 2];
-                        const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y, g = c0.z, h = c1.z, kk = c2.z;
+                        const float4* dg = a.diag + 3 * (size_t)i;
+                        const float4 c0 = dg[0], c1 = dg[1], c2 = dg[2];
+                        const float aa = c0.x, bb = c1.x, c = c2.x, d = c0.y, e = c1.y, f = c2.y;
+                        const float g = c0.z, h = c1.z, kk = c2.z;
                         const float A = e * kk - f * h, Bc = f * g - d * kk, Cc = d * h - e * g;
                         const float id = 1.0f / (aa * A + bb * Bc + c * Cc);
                         m0 = make_float4(A * id, Bc * id, Cc * id, 0.0f);
@@ -2251,10 +2255,10 @@ __global__ void __launch_bounds__(32 * W, !Staged ? 4 : W > 8 ? 1 : 2) k_pcg_bat
     if (st.failed && lane == 0) a.stats[s].status = LCS_ERR_TIMEOUT;
 }
 
-// Test hook of the staged copies (lcs_debug_pcg_copy_wait): one warp forms A x slice by slice as k_pcg_batch does.  With
-// `omit` the first copy's barrier also expects 16 bytes that nothing sends, so that the wait for it runs out.
-__global__ void __launch_bounds__(32) k_copy_wait_probe(Bsr A, uint32_t n, const float4* x, float4* y, int omit, uint32_t limit,
-                                                        lcs_pcg_stats* stats)
+// Test hook of the staged copies (lcs_debug_pcg_copy_wait): one warp forms A x slice by slice as k_pcg_batch does.
+// With `omit` the first copy's barrier also expects 16 bytes that nothing sends, so that the wait for it runs out.
+__global__ void __launch_bounds__(32) k_copy_wait_probe(Bsr A, uint32_t n, const float4* x, float4* y, int omit,
+                                                        uint32_t limit, lcs_pcg_stats* stats)
 {
     extern __shared__ __align__(128) unsigned char s_stage[];
     __shared__ __align__(8) uint64_t s_bar[2];
@@ -2381,7 +2385,8 @@ extern "C" int lcs_debug_pcg_exchange(const double* values, double* sums, int32_
     lcs_pcg_stats* st = reinterpret_cast<lcs_pcg_stats*>(mem + bytes);
     cudaError_t e = cudaMemsetAsync(mem, 0, bytes + sizeof(h), s);
     void* args[] = {&values, &slots, &missing_block, &spin_limit, &sums, &st};
-    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)k_exchange_probe, dim3(blocks), dim3(256), args, 0, s);
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel((const void*)k_exchange_probe, dim3(blocks), dim3(256), args, 0, s);
     if (e == cudaSuccess) lcs_count_launch();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -2392,8 +2397,8 @@ extern "C" int lcs_debug_pcg_exchange(const double* values, double* sums, int32_
     return h.status;
 }
 
-extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* y, int32_t omit_copy, uint32_t poll_limit,
-                                       lcs_stream stream)
+extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* y, int32_t omit_copy,
+                                       uint32_t poll_limit, lcs_stream stream)
 {
     if (!A || !A->row_ptr || !A->col || !A->val || A->n_rows == 0 || !x || !y)
         return lcs_fail(LCS_ERR_INVALID, "lcs_debug_pcg_copy_wait: bad argument");
@@ -2405,7 +2410,8 @@ extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* 
     LCS_CUDA_TRY(cudaMalloc(&st, sizeof(h)));
     cudaError_t e = cudaMemsetAsync(st, 0, sizeof(h), s);
     if (e == cudaSuccess) {
-        k_copy_wait_probe<<<1, 32, stage::kWarpBytes, s>>>(Bsr{A->row_ptr, A->col, A->val}, A->n_rows, reinterpret_cast<const float4*>(x),
+        const Bsr M{A->row_ptr, A->col, A->val};
+        k_copy_wait_probe<<<1, 32, stage::kWarpBytes, s>>>(M, A->n_rows, reinterpret_cast<const float4*>(x),
                                                            reinterpret_cast<float4*>(y), omit_copy, poll_limit, st);
         e = cudaGetLastError();
         lcs_count_launch();
@@ -2423,7 +2429,8 @@ extern "C" int lcs_debug_pcg_copy_wait(const lcs_bsr* A, const float* x, float* 
 static int fused_per_sm()
 {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused<kRowLanes>, kFusedThreads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused<kRowLanes>, kFusedThreads, 0) != cudaSuccess)
+        return 0;
     return per_sm > 0 ? 1 : 0;
 }
 
@@ -2838,8 +2845,8 @@ int lcs_pcg_solve_sell(lcs_pcg* P, const float* diag, const uint32_t* slice_ptr,
                       (cudaStream_t)stream, c_ptr, c_col, c_val, c_ok);
 }
 
-// The persistent solve on at most `grid` co-resident blocks (one per SM); a.part holds kSmallSumBytes per block.  Rows that
-// fit four lanes each in one block of 256 or 512 threads per SM take k_pcg_small.
+// The persistent solve on at most `grid` co-resident blocks (one per SM); a.part holds kSmallSumBytes per block.  Rows
+// that fit four lanes each in one block of 256 or 512 threads per SM take k_pcg_small.
 static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
 {
     // the partial sums' tags (small), the barrier arrival counter and the stats have to be set; the rest is written
@@ -2850,15 +2857,16 @@ static int launch_persistent(FusedArgs& a, int grid, cudaStream_t s)
     if (a.n <= 128 * cap) {
         const uint32_t bt = a.n <= 64 * cap ? 256 : 512, blocks = (a.n + bt / 4 - 1) / (bt / 4);
         LCS_CUDA_TRY(cudaMemsetAsync(a.part, 0, kSmallSumBytes * blocks, s));
-        LCS_CUDA_TRY(cudaLaunchCooperativeKernel(bt == 256 ? (const void*)k_pcg_small<256> : (const void*)k_pcg_small<512>,
-                                                 dim3(blocks), dim3(bt), args, 0, s));
+        const void* kernel = bt == 256 ? (const void*)k_pcg_small<256> : (const void*)k_pcg_small<512>;
+        LCS_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(bt), args, 0, s));
     } else {
         int dev = 0, l2 = 0;
         LCS_CUDA_TRY(cudaGetDevice(&dev));
         LCS_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
         a.l2_bytes = (uint64_t)l2;
         LCS_CUDA_TRY(cudaMemsetAsync(a.bar_count, 0, sizeof(unsigned), s));
-        LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(grid), dim3(kFusedThreads), args, 0, s));
+        LCS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_pcg_fused<kRowLanes>, dim3(grid), dim3(kFusedThreads),
+                                                 args, 0, s));
     }
     lcs_count_launch();
     return LCS_OK;
@@ -3106,13 +3114,14 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
     a.stats = stats_per_scene;
     a.scenes = nullptr;
     a.n_rows = P->n;
-    auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list, cudaStream_t st) -> cudaError_t {
-        // By the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a single slice, for which
-        // the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600 rows: 2.7 ms so, 3.7 ms
-        // staged).  Two or more are staged, by 16 warps (one CTA per SM) if the grid fits the GPU once or a CTA has
-        // work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to 4,000: 1.7 and 2.3), else
-        // by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).  Clusters of 16 stay at 8 warps,
-        // so that the SMs of one GPC always hold them.
+    auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list,
+                      cudaStream_t st) -> cudaError_t {
+        // By the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a single slice, for
+        // which the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600 rows: 2.7 ms so,
+        // 3.7 ms staged).  Two or more are staged, by 16 warps (one CTA per SM) if the grid fits the GPU once or a CTA
+        // has work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to 4,000: 1.7 and 2.3),
+        // else by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).  Clusters of 16 stay at 8
+        // warps, so that the SMs of one GPC always hold them.
         const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
         const bool staged = cta_chunks >= 2;
         const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= (uint32_t)kNumSMs);
@@ -3121,7 +3130,8 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         const uint32_t warps = wide ? 16 : 8, smem = staged ? warps * stage::kWarpBytes : 0;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
-        if (e == cudaSuccess && C == 16) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess && C == 16)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         BatchArgs b = a;
         b.scenes = scene_list;

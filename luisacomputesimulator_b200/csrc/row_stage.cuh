@@ -52,7 +52,8 @@ __device__ __forceinline__ void bar_expect_more(uint64_t* bar, uint32_t bytes)
 __device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(kPollNs) : "memory");
     return ok != 0;
 }
@@ -83,7 +84,8 @@ struct Warp {
     uint32_t limit = kWaitLimit;
     bool failed = false;  // a copy did not arrive within the limit
 
-    __device__ __forceinline__ void init(unsigned char* b, uint64_t* barriers, const Csr& a, const Csr& extra, uint32_t n_rows)
+    __device__ __forceinline__ void init(unsigned char* b, uint64_t* barriers, const Csr& a, const Csr& extra,
+                                         uint32_t n_rows)
     {
         buf = b;
         bar = barriers;
@@ -228,7 +230,8 @@ __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const
     for (int j = 0; j < 4; ++j) {
         float3 acc = make_float3(0.f, 0.f, 0.f);
         const uint32_t ge = __shfl_sync(0xFFFFFFFFu, cur.hi, 8 * j + 7);
-        const uint32_t rs = __shfl_sync(0xFFFFFFFFu, cur.lo, 8 * j + g), re = __shfl_sync(0xFFFFFFFFu, cur.hi, 8 * j + g);
+        const uint32_t rs = __shfl_sync(0xFFFFFFFFu, cur.lo, 8 * j + g);
+        const uint32_t re = __shfl_sync(0xFFFFFFFFu, cur.hi, 8 * j + g);
         uint32_t k = rs + lig;
         while (Staged && w.bulk && k0 < ge) {
             const uint32_t nb = min(kWin, ge - k0), k1 = k0 + nb;
@@ -242,7 +245,8 @@ __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const
             uint32_t* sc = reinterpret_cast<uint32_t*>(d + kValBytes) + (k0 & 3u);
             if (k1 + 4 > w.nnz) {  // the last words of the arrays, where a 16-byte copy would pass their end
                 const int have = (int)(Warp::copy_bytes(9ull * k0, 9 * nb, 9ull * w.nnz) / 4) - (int)((9u * k0) & 3u);
-                for (int c = max(have, 0) + (int)lane; c < (int)(9 * nb); c += 32) sv[c] = __ldg(&w.A.val[9ull * k0 + c]);
+                for (int c = max(have, 0) + (int)lane; c < (int)(9 * nb); c += 32)
+                    sv[c] = __ldg(&w.A.val[9ull * k0 + c]);
                 const int havec = (int)(Warp::copy_bytes(k0, nb, w.nnz) / 4) - (int)(k0 & 3u);
                 for (int c = max(havec, 0) + (int)lane; c < (int)nb; c += 32) sc[c] = __ldg(&w.A.col[k0 + c]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -270,7 +274,8 @@ __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const
             k0 = ge;
         }
         if (has_b) {
-            const uint32_t bs = __shfl_sync(0xFFFFFFFFu, cur.blo, 8 * j + g), be = __shfl_sync(0xFFFFFFFFu, cur.bhi, 8 * j + g);
+            const uint32_t bs = __shfl_sync(0xFFFFFFFFu, cur.blo, 8 * j + g);
+            const uint32_t be = __shfl_sync(0xFFFFFFFFu, cur.bhi, 8 * j + g);
             direct_blocks<4>(w.B, bs + lig, be, ld, acc);
             __syncwarp();
         }
