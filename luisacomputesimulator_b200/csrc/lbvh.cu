@@ -804,10 +804,11 @@ __device__ __forceinline__ bool exceeds(const float4* wide, uint32_t ni, const f
 {
     for (uint32_t small = 16384;; small >>= 3) {  // subtrees of so many inner nodes count whole
         uint2 stack[64];                          // node, first sorted position under it; a path has at most 62 levels
-        uint32_t left = ni;
+        uint32_t left = ni, popped = 0;
         int sp = 0;
         stack[sp++] = make_uint2(0u, 0u);
         while (sp > 0) {
+            if (++popped > kRefNodes) return true;
             const uint2 b = stack[--sp];
             float4 mn[2], mx[2];
 #pragma unroll
@@ -878,6 +879,7 @@ __global__ void __launch_bounds__(256) k_may_end(const float4* __restrict__ wide
         const uint32_t q = t < n_queries && order ? __ldg(&order[t]) : t;
         if (t < n_queries) query_box<EE>(x0, x1, edges, dhat, thickness, uniform_r, q, box);
         if (Count && deep) {
+            if (__any_sync(0xFFFFFFFFu, *reinterpret_cast<volatile uint32_t*>(flag) == call)) return;  // marked already
             float cull[6] = {box[0], box[1], box[2], box[3], box[4], box[5]};
             if (EE && (sym || !dhat) && t < n_queries) {  // what the once-per-pair walk culls with
                 const SymQuery Q = sym ? sym_query<true>(x0, x1, edges, 0.0f, dhat, thickness, from_ordered(info[1]),
