@@ -3116,14 +3116,18 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
     a.n_rows = P->n;
     auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list,
                       cudaStream_t st) -> cudaError_t {
-        // By the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a single slice, for
-        // which the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600 rows: 2.7 ms so,
-        // 3.7 ms staged).  Two or more are staged, by 16 warps (one CTA per SM) if the grid fits the GPU once or a CTA
-        // has work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to 4,000: 1.7 and 2.3),
-        // else by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).  Clusters of 16 stay at 8
-        // warps, so that the SMs of one GPC always hold them.
+        // Clusters of a given size, by the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a
+        // single slice, for which the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600
+        // rows: 2.7 ms so, 3.7 ms staged).  Two or more are staged, by 16 warps (one CTA per SM) if the grid fits the
+        // GPU once or a CTA has work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to
+        // 4,000: 1.7 and 2.3), else by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).
+        // Clusters of 16 stay at 8 warps, so that the SMs of one GPC always hold them.
+        // Clusters by scene (a list of them) cut the work into as many CTAs as the GPU wants, so that 1,024 threads per SM
+        // read directly.  Staged CTAs leave half of them to wait for the contact blocks, which grow while a tuned batch
+        // runs: a step of 272 drapes of 1,000 to 32,000 vertices in contact 385 ms so, 490 staged by 16 warps, 422 by 8;
+        // of 16 drapes of 100 x 100 31.9 and 34.4 ms.  (Few contacts: 272 systems of 1,000 to 4,000 rows 6.9 and 6.1.)
         const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
-        const bool staged = cta_chunks >= 2;
+        const bool staged = !scene_list && cta_chunks >= 2;
         const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= (uint32_t)kNumSMs);
         const void* kernel = wide ? (const void*)k_pcg_batch<16, true>
                                   : staged ? (const void*)k_pcg_batch<8, true> : (const void*)k_pcg_batch<8, false>;
