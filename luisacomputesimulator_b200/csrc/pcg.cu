@@ -3114,6 +3114,9 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
     a.stats = stats_per_scene;
     a.scenes = nullptr;
     a.n_rows = P->n;
+    uint64_t total_chunks = 0;
+    for (uint32_t sc = 0; sc < n_scenes; ++sc)
+        total_chunks += (host_row_offsets[sc + 1] - host_row_offsets[sc] + kChunk - 1) / kChunk;
     auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list,
                       cudaStream_t st) -> cudaError_t {
         // Clusters of a given size, by the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a
@@ -3122,12 +3125,16 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         // GPU once or a CTA has work for long (2,000 to 16,000 rows: 5.3 ms, with 8 warps 8.8; 8 scenes of 2,000 to
         // 4,000: 1.7 and 2.3), else by 8 (two CTAs per SM; 48 scenes of 4,000 rows: 3.2 ms, with 16 warps 3.5).
         // Clusters of 16 stay at 8 warps, so that the SMs of one GPC always hold them.
+        // Where the SMs' average share is well over the largest CTA's, all SMs are busy to the end, and 1,024 threads that
+        // read directly do more than the copies.  The line is 2 1/8 times: a step of 48 drapes of 120 x 120 in contact by
+        // clusters of 8 (2.18 times) 91 ms so, 137 staged, by clusters of 4 (1.1) 115 and 112; 272 systems of 1,000 to
+        // 32,000 rows with few contacts by clusters of 4 (2.10) 35.8 and 30.5, by 8 (4.1) 31.3 and 35.6.
         // Clusters by scene (a list of them) cut the work into as many CTAs as the GPU wants, so that 1,024 threads per SM
         // read directly.  Staged CTAs leave half of them to wait for the contact blocks, which grow while a tuned batch
         // runs: a step of 272 drapes of 1,000 to 32,000 vertices in contact 385 ms so, 490 staged by 16 warps, 422 by 8;
         // of 16 drapes of 100 x 100 31.9 and 34.4 ms.  (Few contacts: 272 systems of 1,000 to 4,000 rows 6.9 and 6.1.)
         const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
-        const bool staged = !scene_list && cta_chunks >= 2;
+        const bool staged = !scene_list && cta_chunks >= 2 && 8 * total_chunks <= 17ull * kNumSMs * cta_chunks;
         const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= (uint32_t)kNumSMs);
         const void* kernel = wide ? (const void*)k_pcg_batch<16, true>
                                   : staged ? (const void*)k_pcg_batch<8, true> : (const void*)k_pcg_batch<8, false>;

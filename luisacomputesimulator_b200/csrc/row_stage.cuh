@@ -214,8 +214,8 @@ __device__ __forceinline__ void group_sum(float3& v)
 // `next` is the warp's next slice: its first window is put in flight while this slice ends (and this slice's first
 // window may be in flight already).  B (contacts) is read directly: copies of its short, uneven runs made a batched
 // solve 6% slower with few contacts and 45% with many.  ld(col) reads one vector of x.
-// Staged = false reads A directly too (no shared memory, no barriers): for a warp's single slice the copies only add
-// their latency.
+// Staged = false reads A directly too (no shared memory, no barriers): for launches whose CTAs fill the GPU with threads,
+// and for a warp's single slice, where the copies only add their latency.
 template <bool Staged, class Load>
 __device__ __forceinline__ float3 slice_product(Warp& w, const Slice& cur, const Slice& next, const Load& ld)
 {
