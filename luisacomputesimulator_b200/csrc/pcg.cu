@@ -3117,7 +3117,7 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
     uint64_t total_chunks = 0;
     for (uint32_t sc = 0; sc < n_scenes; ++sc)
         total_chunks += (host_row_offsets[sc + 1] - host_row_offsets[sc] + kChunk - 1) / kChunk;
-    auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list,
+    auto launch = [&](int C, uint32_t clusters, uint32_t max_rows, const uint32_t* scene_list, uint32_t all_ctas,
                       cudaStream_t st) -> cudaError_t {
         // Clusters of a given size, by the chunks of 256 rows that a CTA gets of the largest scene: one leaves each warp a
         // single slice, for which the copies only add latency and smaller CTAs fill the SMs (256 scenes of 300 to 600
@@ -3129,12 +3129,16 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         // read directly do more than the copies.  The line is 2 1/8 times: a step of 48 drapes of 120 x 120 in contact by
         // clusters of 8 (2.18 times) 91 ms so, 137 staged, by clusters of 4 (1.1) 115 and 112; 272 systems of 1,000 to
         // 32,000 rows with few contacts by clusters of 4 (2.10) 35.8 and 30.5, by 8 (4.1) 31.3 and 35.6.
-        // Clusters by scene (a list of them) cut the work into as many CTAs as the GPU wants, so that 1,024 threads per SM
-        // read directly.  Staged CTAs leave half of them to wait for the contact blocks, which grow while a tuned batch
-        // runs: a step of 272 drapes of 1,000 to 32,000 vertices in contact 385 ms so, 490 staged by 16 warps, 422 by 8;
-        // of 16 drapes of 100 x 100 31.9 and 34.4 ms.  (Few contacts: 272 systems of 1,000 to 4,000 rows 6.9 and 6.1.)
+        // Clusters by scene (a list of them, all_ctas in all its launches) are staged if the GPU holds a CTA on each SM at
+        // most: 13 drapes of 58 x 58 vertices 10.3 ms a step, 11.9 read directly.  Beyond that the CTAs fill the GPU with
+        // 1,024 threads per SM that read directly.  Staged CTAs leave half of them to wait for the contact blocks, which
+        // grow while a batch, tuned on its first solve, runs: a step of 272 drapes of 1,000 to 32,000 vertices in contact
+        // 385 ms so, 490 staged by 16 warps, 422 by 8; of 16 drapes of 100 x 100 31.9 and 34.4 ms.  (Few contacts: 272
+        // systems of 1,000 to 4,000 rows 6.9 and 6.1.)
         const uint32_t cta_chunks = ((max_rows + kChunk - 1) / kChunk + C - 1) / C;
-        const bool staged = !scene_list && cta_chunks >= 2 && 8 * total_chunks <= 17ull * kNumSMs * cta_chunks;
+        const bool worth = scene_list ? all_ctas <= (uint32_t)kNumSMs && C < 16
+                                      : 8 * total_chunks <= 17ull * kNumSMs * cta_chunks;
+        const bool staged = worth && cta_chunks >= 2;
         const bool wide = staged && C < 16 && (cta_chunks >= 8 || clusters * C <= (uint32_t)kNumSMs);
         const void* kernel = wide ? (const void*)k_pcg_batch<16, true>
                                   : staged ? (const void*)k_pcg_batch<8, true> : (const void*)k_pcg_batch<8, false>;
@@ -3166,7 +3170,7 @@ extern "C" int lcs_pcg_solve_batch(lcs_pcg* P, uint32_t n_scenes, const uint32_t
         uint32_t max_rows = 0;
         for (uint32_t sc = 0; sc < n_scenes; ++sc)
             max_rows = std::max(max_rows, host_row_offsets[sc + 1] - host_row_offsets[sc]);
-        LCS_CUDA_TRY(launch(cluster, n_scenes, max_rows, nullptr, s0));
+        LCS_CUDA_TRY(launch(cluster, n_scenes, max_rows, nullptr, n_scenes * (uint32_t)cluster, s0));
         lcs_count_launch();
         return LCS_OK;
     }
@@ -3245,11 +3249,13 @@ static int solve_batch_auto(lcs_pcg* P, uint32_t n_scenes, const uint32_t* host_
         }
     }
     LCS_CUDA_TRY(cudaEventRecord(P->class_fork, s0));
+    uint32_t ctas = 0;
+    for (int k = 0; k < 5; ++k) ctas += (uint32_t)(start[k + 1] - start[k]) << k;
     for (int k = 0; k < 5; ++k) {
         const uint32_t m = (uint32_t)(start[k + 1] - start[k]);
         if (m == 0) continue;
         LCS_CUDA_TRY(cudaStreamWaitEvent(P->class_stream[k], P->class_fork, 0));
-        LCS_CUDA_TRY(launch(1 << k, m, rows_of(flat[start[k]]), P->class_scenes + start[k], P->class_stream[k]));
+        LCS_CUDA_TRY(launch(1 << k, m, rows_of(flat[start[k]]), P->class_scenes + start[k], ctas, P->class_stream[k]));
         lcs_count_launch();
         LCS_CUDA_TRY(cudaEventRecord(P->class_join[k], P->class_stream[k]));
         LCS_CUDA_TRY(cudaStreamWaitEvent(s0, P->class_join[k], 0));
