@@ -53,6 +53,7 @@ def _apply(D, rp, col, val, x):
     (150, 20, False),                                              # 40 blocks a row: beyond the ones held in registers
     (9472, 3, False), (9473, 3, False),                            # 64 and 128 rows per block on 148 SMs
     (18944, 3, False), (18945, 3, False), (30001, 9, False),       # the largest system of one row per four lanes; beyond
+    (20000, 60, False),                                            # 120 blocks a row
     (20000, 56, False), (20000, 64, False),                        # a matrix below and beyond three quarters of L2
 ])
 def test_persistent_solve_at_the_edges(n, reach, as_b, fp64):
